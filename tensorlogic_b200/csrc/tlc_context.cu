@@ -62,6 +62,9 @@ extern "C" int32_t tlc_init(int32_t ordinal, tlc_ctx **out) {
         cudaMemset(ctx->dev_status, 0, sizeof(tlc_dev_status)) != cudaSuccess ||
         cudaMalloc(&ctx->tickets, 16384 * sizeof(int)) != cudaSuccess ||
         cudaMemset(ctx->tickets, 0, 16384 * sizeof(int)) != cudaSuccess ||
+        cudaMalloc(&ctx->wt_partial, (size_t)ctx->sm_count * 256 * 128 * sizeof(float)) != cudaSuccess ||
+        cudaMalloc(&ctx->wt_flags, (size_t)ctx->sm_count * sizeof(int)) != cudaSuccess ||
+        cudaMemset(ctx->wt_flags, 0, (size_t)ctx->sm_count * sizeof(int)) != cudaSuccess ||
         cudaMallocHost(&ctx->host_status, sizeof(tlc_dev_status)) != cudaSuccess) {
         const char *msg = cudaGetErrorString(cudaGetLastError());
         if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -82,6 +85,7 @@ extern "C" int32_t tlc_init(int32_t ordinal, tlc_ctx **out) {
     else if (getenv("TL_PERF")) ctx->perf = true;  // the reference's own switch
     if (const char *e = getenv("TLC_COMM_LL")) ctx->comm_ll = atoi(e) != 0;
     if (const char *e = getenv("TLC_GEMM_SPLITK")) ctx->gemm_splitk = atoi(e);
+    if (const char *e = getenv("TLC_GEMM_WT_MAX_M")) ctx->gemm_wt_max_m = atoi(e);
     if (const char *e = getenv("TLC_GEMM_PG")) ctx->gemm_pg = atoi(e);
     if (const char *e = getenv("TLC_GEMM_TMA")) ctx->gemm_tma = atoi(e) != 0;
     if (const char *e = getenv("TLC_ATTN_WIDE")) ctx->attn_wide = atoi(e);
@@ -119,7 +123,16 @@ extern "C" int32_t tlc_set_option(tlc_ctx *ctx, const char *name, int64_t value)
     else if (n == "gemm_pg") {
         TLC_REQUIRE(value >= 0 && value <= 2, TLC_ERR_INVALID_OPERATION, "set_option: gemm_pg must be 0, 1 or 2");
         ctx->gemm_pg = (int)value;
-    } else if (n == "gemm_tma")
+    } else if (n == "gemm_wt_bn") {
+        TLC_REQUIRE(value >= 0 && value <= 256 && value % 16 == 0, TLC_ERR_INVALID_OPERATION,
+                    "set_option: gemm_wt_bn must be a multiple of 16 up to 256");
+        ctx->gemm_wt_bn = (int)value;
+    } else if (n == "gemm_wt_ks") {
+        TLC_REQUIRE(value >= 0 && value <= 9, TLC_ERR_INVALID_OPERATION, "set_option: gemm_wt_ks must be 0..9");
+        ctx->gemm_wt_ks = (int)value;
+    } else if (n == "gemm_wt_max_m")
+        ctx->gemm_wt_max_m = (int)value;
+    else if (n == "gemm_tma")
         ctx->gemm_tma = value != 0;
     else if (n == "pdl")
         ctx->use_pdl = value != 0;
@@ -225,6 +238,8 @@ extern "C" int32_t tlc_destroy(tlc_ctx *ctx) {
     if (ctx->scratch) cudaFree(ctx->scratch);
     cudaFree(ctx->dev_status);
     cudaFree(ctx->tickets);
+    cudaFree(ctx->wt_partial);
+    cudaFree(ctx->wt_flags);
     cudaFreeHost(ctx->host_status);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
@@ -269,6 +284,8 @@ int32_t tlc_status_after_sync(tlc_ctx *ctx) {
     if (ctx->host_status->code != 0) {
         int code = ctx->host_status->code, where = ctx->host_status->where;
         cudaMemsetAsync(ctx->dev_status, 0, sizeof(tlc_dev_status), ctx->stream);
+        if (code < TLC_DEV_INDEX)  // a kernel that gave up may have left a hand-over flag behind
+            cudaMemsetAsync(ctx->wt_flags, 0, (size_t)ctx->sm_count * sizeof(int), ctx->stream);
         cudaStreamSynchronize(ctx->stream);
         if (code == TLC_DEV_INDEX)
             return tlc_fail(TLC_ERR_INDEX, "Index out of bounds: a sequence position lies outside the KV cache "

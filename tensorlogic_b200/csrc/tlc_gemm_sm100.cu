@@ -2,16 +2,18 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
+#include <climits>
 #include <type_traits>
 
 #include "tlc_gemm_kernel.cuh"
+#include "tlc_gemm_wt.h"
 
 using namespace tlc_gemm;
 
-// Tensor map of the activations [M, K] (f16, rows K elements apart): boxes of 128 rows
-// x 64 columns, 128-byte swizzle, zero fill outside.  False when the driver entry point
-// is missing or refuses the shape; the cp.async loaders take over then.
-bool tlc_gemm::encode_x_map(CUtensorMap *map, const GemmParams &p) {
+// Tensor map of a row-major matrix [outer, inner], rows `pitch` bytes apart: boxes of box_outer rows x
+// box_inner elements, zero fill outside.  False when the driver entry point is missing or refuses the shape.
+bool tlc_gemm::encode_map(CUtensorMap *map, CUtensorMapDataType type, CUtensorMapSwizzle swizzle, const void *ptr,
+                          uint64_t inner, uint64_t outer, uint64_t pitch, uint32_t box_inner, uint32_t box_outer) {
     static PFN_cuTensorMapEncodeTiled_v12000 encode = [] {
         void *fn = nullptr;
         cudaDriverEntryPointQueryResult qres;
@@ -21,14 +23,26 @@ bool tlc_gemm::encode_x_map(CUtensorMap *map, const GemmParams &p) {
         cudaGetLastError();
         return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
     }();
-    if (!encode || ((uintptr_t)p.x & 15) != 0 || (p.k & 7) != 0) return false;
-    const cuuint64_t dims[2] = {(cuuint64_t)p.k, (cuuint64_t)p.m};
-    const cuuint64_t strides[1] = {(cuuint64_t)p.k * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)kBK, 128};
+    if (!encode || ((uintptr_t)ptr & 15) != 0 || (pitch & 15) != 0) return false;
+    const cuuint64_t dims[2] = {inner, outer};
+    const cuuint64_t strides[1] = {pitch};
+    const cuuint32_t box[2] = {box_inner, box_outer};
     const cuuint32_t estr[2] = {1, 1};
-    return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half *>(p.x), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+    return encode(map, type, 2, const_cast<void *>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+bool tlc_gemm::encode_f16_map(CUtensorMap *map, const void *ptr, uint64_t inner, uint64_t outer, uint64_t pitch,
+                              uint32_t box_inner, uint32_t box_outer) {
+    return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, CU_TENSOR_MAP_SWIZZLE_128B, ptr, inner, outer, pitch, box_inner,
+                      box_outer);
+}
+
+// Tensor map of the activations [M, K] for the 128-row tiles of this file; the cp.async loaders take
+// over when there is none.
+bool tlc_gemm::encode_x_map(CUtensorMap *map, const GemmParams &p) {
+    return encode_f16_map(map, p.x, (uint64_t)p.k, (uint64_t)p.m, (uint64_t)p.k * 2, kBK, 128);
 }
 
 namespace {
@@ -255,7 +269,7 @@ __global__ void __launch_bounds__(gemm_threads(NT, PG), 1)
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(accum_bar + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int n0 = blockIdx.x * (SW ? 128 : BN), m0 = blockIdx.y * 128 * MT;
     const int KT_all = (p.k + kBK - 1) / kBK;  // K is a multiple of 32: the last step may hold one block only
     // split K (two-group form only): this CTA's share of the K steps, never empty
@@ -301,23 +315,29 @@ __global__ void __launch_bounds__(gemm_threads(NT, PG), 1)
                                                     lane, (tid - 128) / BN, kt0);
     } else if (warp < 4 && p.a_tma) {
         // ------------------------------ A tile by TMA ------------------------------
-        // One thread issues, per K step, MT boxes of 128 rows x 64 columns with the 128-byte
+        // One warp issues, per K step, MT boxes of 128 rows x 64 columns with the 128-byte
         // swizzle of the tile; rows past M and columns past K read the zero fill.  The
         // inner coordinate is a multiple of 64 elements (128 bytes).
-        if (tid == 0) {
-            asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&x_map)) : "memory");
+        if (warp == 0) {
+            const uint32_t el = elect_one();
+            if (el) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&x_map)) : "memory");
+            int s = 0;
+            uint32_t ph = 1;
             for (int j = 0; j < KT; j++) {
-                const int s = j % kStages;
-                if (!mbar_wait(&empty[s], ((j / kStages) & 1u) ^ 1u, abort_flag, p.status, 12, p.wait_ns)) break;
+                if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], ph, abort_flag, p.status, 12, p.wait_ns))) break;
                 const uint32_t bar = smem_u32(&full[s]);
                 const uint32_t abase = smem_u32(tiles + (size_t)s * STAGE_BYTES);
-                mbar_arrive_expect_tx(&full[s], A_BYTES);
+                mbar_arrive_expect_tx_el(&full[s], A_BYTES, el);
 #pragma unroll
                 for (int i = 0; i < MT; i++)
-                    tma_load_2d(abase + i * (128 * 128), &x_map, (kt0 + j) * kBK, m0 + 128 * i, bar);
+                    tma_load_2d_el(abase + i * (128 * 128), &x_map, (kt0 + j) * kBK, m0 + 128 * i, bar, el);
+                if (++s == kStages) {
+                    s = 0;
+                    ph ^= 1u;
+                }
             }
         }
-        __syncwarp();  // the other lanes of warp 0 sleep here instead of polling beside the issuer
+        __syncwarp();
     } else if (warp < 4) {
         // ------------------------------ A loaders (cp.async) ------------------------------
         auto issue = [&](int j) {
@@ -352,26 +372,31 @@ __global__ void __launch_bounds__(gemm_threads(NT, PG), 1)
         }
     } else if (warp == MMA_WARP) {
         // ------------------------------ MMA issuer ------------------------------
+        const uint32_t el = elect_one();
+        const uint32_t a0 = (smem_u32(tiles) & 0x3FFFF) >> 4;
+        int s = 0;
+        uint32_t ph = 0, acc = 0;
         for (int kt = 0; kt < KT; kt++) {
-            const int s = kt % kStages;
-            const bool ready = __all_sync(0xffffffffu, mbar_wait(&full[s], (kt / kStages) & 1u, abort_flag, p.status, 14, p.wait_ns));
+            const bool ready = __all_sync(0xffffffffu, mbar_wait(&full[s], ph, abort_flag, p.status, 14, p.wait_ns));
             tc_fence_after();
-            if (lane == 0 && ready) {
-                const uint32_t a_addr = smem_u32(tiles + (size_t)s * STAGE_BYTES);
-                const uint32_t b_addr = a_addr + A_BYTES;
+            if (ready) {
+                const uint32_t a_addr = a0 + (uint32_t)s * (STAGE_BYTES >> 4), b_addr = a_addr + (A_BYTES >> 4);
 #pragma unroll
                 for (int k16 = 0; k16 < kBK / 16; k16++) {
-                    const uint64_t bdesc = make_desc(b_addr + k16 * 32);
 #pragma unroll
                     for (int i = 0; i < MT; i++)
-                        umma_f16(tmem_base + BN * i, make_desc(a_addr + i * (128 * 128) + k16 * 32), bdesc, IDESC,
-                                 (kt > 0 || k16 > 0) ? 1u : 0u);
+                        umma_f16(tmem_base + BN * i, desc_at(a_addr + i * ((128 * 128) >> 4) + k16 * 2),
+                                 desc_at(b_addr + k16 * 2), IDESC, acc, el);
+                    acc = 1;
                 }
             }
-            if (lane == 0) umma_commit(&empty[s]);  // arrives when the MMAs above have read the stage
-            __syncwarp();
+            umma_commit(&empty[s], el);  // arrives when the MMAs above have read the stage
+            if (++s == kStages) {
+                s = 0;
+                ph ^= 1u;
+            }
         }
-        if (lane == 0) umma_commit(accum_bar);
+        umma_commit(accum_bar, el);
         __syncwarp();
     }
 
@@ -381,12 +406,14 @@ __global__ void __launch_bounds__(gemm_threads(NT, PG), 1)
     // 256-row weight tile) take the 32-column pieces in turn.
     if (warp < MMA_WARP) {
         mbar_wait(accum_bar, 0, abort_flag, p.status, 13, p.wait_ns);
+        __syncwarp();  // the lanes leave a wait one by one; tcgen05.ld is for a whole warp
         tc_fence_after();
         const int wq = warp & 3;
         constexpr int OUT_COLS = SW ? 128 : BN;  // output columns of the CTA
         constexpr int PIECES = MT * OUT_COLS / 32;
 #pragma unroll 1
         for (int pc = warp >> 2; pc < PIECES; pc += MMA_WARP / 4) {
+            __syncwarp();
             const int i = pc / (OUT_COLS / 32), c0 = (pc % (OUT_COLS / 32)) * 32;
             const int row = m0 + 128 * i + 32 * wq + lane;
             bool row_ok = row < p.m;
@@ -604,7 +631,21 @@ int32_t tlc_launch_gemm(tlc_ctx *ctx, const tlc_gemv_args &a) {
     const size_t norm_bytes = a.norm_w ? align256((size_t)a.m * k * 2) : 0;
     int64_t ntot = 0;
     for (int i = 0; i < a.n_out; i++) ntot += a.outs[i].w->n_rows;
-    const int ksplit = gemm_choose_ksplit(ctx, a.m, k, gemm_tiles(a), ntot);
+    // Which form: the one with 128 activation rows on the M side of the MMA (this file) moves half the
+    // activation bytes per MMA, but only in 256 x 256 tiles, and pays off where these fill the waves of SMs:
+    // 8192 -> 28672 at 256 rows (112 tiles) 112 us against 134, 4096 -> 4096 at 2048 rows (128) 57 against
+    // 64; but 4096 -> 11008 at 1024 rows (172 tiles, 58 % of two waves) 124 us against 100.
+    // (An option that forces a detail of that form asks for the form.)
+    bool wt = a.m <= ctx->gemm_wt_max_m && ctx->gemm_tile == 0 && !ctx->gemm_pair && ctx->gemm_pg == 0 && ctx->gemm_tma &&
+              ctx->gemm_splitk == 1;
+    if (wt && ctx->gemm_wt_max_m == INT_MAX && a.m >= 192) {
+        int64_t tiles = 0;
+        for (int i = 0; i < a.n_out; i++) tiles = tiles > a.outs[i].w->n_rows ? tiles : a.outs[i].w->n_rows;
+        tiles = ((tiles + (swiglu ? 127 : 255)) / (swiglu ? 128 : 256)) * ((a.m + 255) / 256);
+        const int64_t slots = (tiles + ctx->sm_count - 1) / ctx->sm_count * ctx->sm_count;
+        wt = tiles < 100 || tiles * 10 < slots * 7;
+    }
+    const int ksplit = wt ? 1 : gemm_choose_ksplit(ctx, a.m, k, gemm_tiles(a), ntot);
     const size_t part_bytes = ksplit > 1 ? align256((size_t)ksplit * a.m * (size_t)ntot * sizeof(float)) : 0;
     if (norm_bytes + part_bytes > 0)
         if (int32_t rc = tlc_scratch_reserve(ctx, norm_bytes + part_bytes)) return rc;
@@ -617,6 +658,12 @@ int32_t tlc_launch_gemm(tlc_ctx *ctx, const tlc_gemv_args &a) {
         x = reinterpret_cast<const __half *>(scratch);
     }
     TLC_REQUIRE(((uintptr_t)x & 15) == 0, TLC_ERR_INVALID_OPERATION, "gemm: activations must be 16-byte aligned");
+    if (wt) {
+        tlc_gemv_args b = a;
+        b.x = x;
+        b.norm_w = nullptr;
+        return tlc_launch_gemm_wt(ctx, b);
+    }
     // The SiLU.mul pair is ONE launch: gate and up rows share the weight tile of a CTA.
     const int n_launch = swiglu ? 1 : a.n_out;
     for (int i = 0; i < n_launch; i++) {

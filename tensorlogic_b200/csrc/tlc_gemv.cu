@@ -30,6 +30,7 @@
 // shared memory, where they are kept pre-permuted in fragment order.
 #include <cuda_fp16.h>
 
+#include "tlc_gemm_wt.h"
 #include "tlc_gemv_kernel.cuh"
 #include "tlc_internal.h"
 #include "tlc_tile.cuh"
@@ -68,14 +69,13 @@ __global__ void linear_generic_kernel(const uint8_t *__restrict__ w, size_t pitc
 
 // ---------------------------------------------------------------------------
 // Dense f16 weights (F16 / F32 files, Q6_K after its load-time dequantization,
-// tied embeddings): one warp per output row, 16-byte loads of the row and of up
-// to 8 activation rows, f32 accumulation, optional bias / residual.  HBM-bound
-// on the 2 bytes per weight; K must be a multiple of 8 and rows 16-byte aligned.
+// tied embeddings), one activation row: one warp per output row, 16-byte loads of the row and of
+// the activations, f32 accumulation, optional bias / residual.  HBM-bound on the 2 bytes
+// per weight; K must be a multiple of 8 and rows 16-byte aligned.  (More rows: tlc_gemm_wt.cu.)
 // ---------------------------------------------------------------------------
-template <int MR>
-__global__ void __launch_bounds__(256) linear_f16_kernel(const uint8_t *__restrict__ w, size_t pitch, int n_rows,
-                                                         int k, const __half *__restrict__ x, int m,
-                                                         __half *__restrict__ y, const __half *__restrict__ bias,
+__global__ void __launch_bounds__(256) linear_f16_kernel(const uint8_t *__restrict__ w, size_t pitch, int n_rows, int k,
+                                                         const __half *__restrict__ x, __half *__restrict__ y,
+                                                         const __half *__restrict__ bias,
                                                          const __half *__restrict__ residual) {
     tlc_pdl_prologue();
     const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -83,43 +83,25 @@ __global__ void __launch_bounds__(256) linear_f16_kernel(const uint8_t *__restri
     if (row >= n_rows) return;
     const uint4 *wr = reinterpret_cast<const uint4 *>(w + (size_t)row * pitch);
     const int steps = k >> 3;  // 16-byte pieces per row
-    float acc[MR];
-#pragma unroll
-    for (int i = 0; i < MR; i++) acc[i] = 0.f;
+    float acc = 0.f;
 #pragma unroll 4
     for (int s = lane; s < steps; s += 32) {
-        const uint4 wv = __ldg(wr + s);
-        const __half2 *wh = reinterpret_cast<const __half2 *>(&wv);
-        float2 wf[4];
+        const uint4 wv = __ldg(wr + s), xv = *(reinterpret_cast<const uint4 *>(x) + s);
+        const __half2 *wh = reinterpret_cast<const __half2 *>(&wv), *xh = reinterpret_cast<const __half2 *>(&xv);
 #pragma unroll
-        for (int j = 0; j < 4; j++) wf[j] = __half22float2(wh[j]);
-#pragma unroll
-        for (int i = 0; i < MR; i++) {
-            if (i < m) {
-                const uint4 xv = *(reinterpret_cast<const uint4 *>(x + (size_t)i * k) + s);
-                const __half2 *xh = reinterpret_cast<const __half2 *>(&xv);
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const float2 xf = __half22float2(xh[j]);
-                    acc[i] = fmaf(wf[j].x, xf.x, acc[i]);
-                    acc[i] = fmaf(wf[j].y, xf.y, acc[i]);
-                }
-            }
+        for (int j = 0; j < 4; j++) {
+            const float2 wf = __half22float2(wh[j]), xf = __half22float2(xh[j]);
+            acc = fmaf(wf.x, xf.x, acc);
+            acc = fmaf(wf.y, xf.y, acc);
         }
     }
 #pragma unroll
-    for (int i = 0; i < MR; i++) {
-        if (i < m) {
-            float v = acc[i];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) {
-                __half h = __float2half_rn(v);
-                if (bias) h = __hadd(h, bias[row]);
-                if (residual) h = __hadd(h, residual[(size_t)i * n_rows + row]);
-                y[(size_t)i * n_rows + row] = h;
-            }
-        }
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) {
+        __half h = __float2half_rn(acc);
+        if (bias) h = __hadd(h, bias[row]);
+        if (residual) h = __hadd(h, residual[row]);
+        y[row] = h;
     }
 }
 
@@ -547,6 +529,9 @@ int32_t tlc_launch_gemv(tlc_ctx *ctx, const tlc_gemv_args &a) {
         const unsigned grid = (unsigned)((w0->n_rows * 32 + threads - 1) / threads);
         const __half *residual = a.epilogue == TLC_EPI_RESIDUAL ? static_cast<const __half *>(a.residual) : nullptr;
         const bool vec = k % 8 == 0 && w0->row_pitch % 16 == 0 && ((uintptr_t)x % 16) == 0 && ((uintptr_t)w0->data % 16) == 0;
+        if (a.m >= 2 && (vec || (!residual && !a.norm_w)))  // (a normalised x of odd width lies in the scratch the copies need)
+            return tlc_launch_gemm_f16(ctx, w0->data, w0->row_pitch, (int)w0->n_rows, (int)k, x, a.m, a.outs[0].y,
+                                       a.epilogue == TLC_EPI_STORE ? a.bias : nullptr, residual);
         if (!vec) {
             TLC_REQUIRE(!residual, TLC_ERR_INVALID_OPERATION, "residual epilogue needs 16-byte aligned f16 rows");
             linear_generic_kernel<<<grid, threads, 0, ctx->stream>>>(
@@ -555,19 +540,14 @@ int32_t tlc_launch_gemv(tlc_ctx *ctx, const tlc_gemv_args &a) {
             TLC_CHECK_LAUNCH(ctx);
             return TLC_OK;
         }
-        for (int m0 = 0; m0 < a.m; m0 += 8) {
-            const int mc = a.m - m0 < 8 ? a.m - m0 : 8;
-            cudaError_t le = tlc_launch_pdl(
-                ctx, mc <= 2 ? linear_f16_kernel<2> : linear_f16_kernel<8>, dim3(grid), dim3(threads), 0,
-                static_cast<const uint8_t *>(w0->data), w0->row_pitch, (int)w0->n_rows, (int)k, x + (size_t)m0 * k, mc,
-                static_cast<__half *>(a.outs[0].y) + (size_t)m0 * w0->n_rows, static_cast<const __half *>(a.bias),
-                residual ? residual + (size_t)m0 * w0->n_rows : nullptr);
-            if (le != cudaSuccess) {
-                cudaGetLastError();
-                return tlc_fail(TLC_ERR_CUDA, "f16 linear launch failed: %s", cudaGetErrorString(le));
-            }
-            TLC_CHECK_LAUNCH(ctx);
+        const cudaError_t le = tlc_launch_pdl(ctx, linear_f16_kernel, dim3(grid), dim3(threads), 0,
+                                              static_cast<const uint8_t *>(w0->data), w0->row_pitch, (int)w0->n_rows, (int)k, x,
+                                              static_cast<__half *>(a.outs[0].y), static_cast<const __half *>(a.bias), residual);
+        if (le != cudaSuccess) {
+            cudaGetLastError();
+            return tlc_fail(TLC_ERR_CUDA, "f16 linear launch failed: %s", cudaGetErrorString(le));
         }
+        TLC_CHECK_LAUNCH(ctx);
         return TLC_OK;
     }
 

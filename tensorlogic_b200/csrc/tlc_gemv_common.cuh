@@ -109,12 +109,17 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
 // returns instead of hanging.  The result is made warp-uniform by the callers.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag,
                                           tlc_dev_status *status, int where, uint64_t wait_ns) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const uint64_t limit = *abort_flag ? 20000ull : wait_ns;
-    const uint64_t t0 = tlc_globaltimer_ns();
-    do {
+    // The clock is looked at on every 32nd failed poll only: reading %globaltimer takes longer than
+    // a hand-over between warps.
+    uint64_t t0 = 0;
+    for (int spin = 1;; spin++) {
         if (mbar_try_wait(bar, parity)) return true;
-    } while (tlc_globaltimer_ns() - t0 < limit);
+        if ((spin & 31) == 0) {
+            const uint64_t now = tlc_globaltimer_ns();
+            if (t0 == 0) t0 = now;
+            if (now - t0 >= (*abort_flag ? 20000ull : wait_ns)) break;
+        }
+    }
     *abort_flag = 1;
     if (atomicCAS(&status->code, 0, 1) == 0) status->where = where;
     return false;

@@ -4,6 +4,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <climits>
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
@@ -50,6 +51,10 @@ struct tlc_ctx {
     // Reusable scratch for kernels that need global workspace (grows on demand).
     void *scratch = nullptr;
     size_t scratch_bytes = 0;
+    // tlc_gemm_wt.cu: the f32 sums of a tile's parts (one slot of 256 x 128 per SM) and their flags
+    // (zero between launches; cleared by the host after a wait that ran out).
+    float *wt_partial = nullptr;
+    int *wt_flags = nullptr;
     // Zero-initialised ticket counters for kernels whose last CTA merges
     // partial results; every user leaves them at zero again.
     int *tickets = nullptr;
@@ -76,6 +81,10 @@ struct tlc_ctx {
     bool gemm_pair = false;  // GEMM tiles of 256 x 256 on CTA pairs (tcgen05 cta_group::2) from 129 rows on; measured slower
     bool comm_ll = true;  // peer-memory all-reduces of up to 256 Ki values use flagged words instead of fences + flags
     int gemm_splitk = 1;  // GEMMs of up to 128 rows and few weight tiles share K over several CTAs per tile: 0 off, 1 where a cost model says it pays, 2 wherever possible
+    // The form with the weight rows on the M side of the MMA (tlc_gemm_wt.cu): activation rows per tile
+    // and CTAs per tile (9: the stream form), 0 = from the shape (tests force the others).
+    int gemm_wt_bn = 0, gemm_wt_ks = 0;
+    int gemm_wt_max_m = INT_MAX;  // activation rows up to which quantized linears take that form (INT_MAX: by shape)
     int gemm_pg = 0;  // producer groups of the GEMM: 0 = two where K is shared out over CTAs, else one; 1 / 2 = forced
     bool gemm_tma = true;  // activation tiles of the GEMM by TMA (false: cp.async loader warps)
     int gemm_tile = 0;  // 0: pick the GEMM tile from the shape; 11, 12, 22: force 128x128, 128x256, 256x256

@@ -6,6 +6,7 @@
 #include <cmath>
 #include <vector>
 
+#include "tlc_gemm_wt.h"
 #include "tlc_internal.h"
 
 namespace {
@@ -108,49 +109,6 @@ __global__ void rope_table_kernel(const __half *__restrict__ x, const __half *__
     const float x0 = __half2float(x[o]), x1 = __half2float(x[o + 1]);
     y[o] = __float2half_rn(__fsub_rn(__fmul_rn(x0, cs), __fmul_rn(x1, sn)));
     y[o + 1] = __float2half_rn(__fadd_rn(__fmul_rn(x0, sn), __fmul_rn(x1, cs)));
-}
-
-// Dense C[M, N] = A[M, K] . B[K, N], f16 in, f32 accumulate, one rounding to f16 (the matmul
-// builtin: Tensor::matmul, src/ops/matmul.rs:13-75; kernels matmul_f16 / matmul_tiled_f16,
-// shaders/unified.metal:33-478).  64 x 64 output tile per CTA of 256 threads, 4 x 4 outputs per
-// thread, K in steps of 16 through shared memory.  A general-purpose builtin, not a tuned path:
-// the model's linears never come here (they are quantized or go through tlc_linear).
-__global__ void __launch_bounds__(256) matmul_f16_kernel(const __half *__restrict__ a, const __half *__restrict__ b,
-                                                         __half *__restrict__ c, int m, int k, int n) {
-    __shared__ float as[16][64 + 1], bs[16][64 + 1];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int row0 = blockIdx.y * 64, col0 = blockIdx.x * 64;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < k; k0 += 16) {
-        for (int i = threadIdx.x; i < 64 * 16; i += 256) {
-            const int r = i >> 4, kk = i & 15;  // A tile: 64 rows x 16 k
-            as[kk][r] = row0 + r < m && k0 + kk < k ? __half2float(a[(size_t)(row0 + r) * k + k0 + kk]) : 0.f;
-            const int kb = i >> 6, cc = i & 63;  // B tile: 16 k x 64 columns
-            bs[kb][cc] = k0 + kb < k && col0 + cc < n ? __half2float(b[(size_t)(k0 + kb) * n + col0 + cc]) : 0.f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < 16; kk++) {
-            float av[4], bv[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                av[i] = as[kk][ty * 4 + i];
-                bv[i] = bs[kk][tx * 4 + i];
-            }
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int r = row0 + ty * 4 + i, cc = col0 + tx * 4 + j;
-            if (r < m && cc < n) c[(size_t)r * n + cc] = __float2half_rn(acc[i][j]);
-        }
 }
 
 // sigmoid: f32 math, RNE to f16 (Tensor::sigmoid_cpu, src/ops/activations.rs:252-266).
@@ -324,10 +282,8 @@ extern "C" int32_t tlc_matmul(tlc_ctx *ctx, const void *a_dev, const void *b_dev
     TLC_REQUIRE(m >= 0 && k >= 0 && k2 >= 0 && n >= 0, TLC_ERR_INVALID_DIMENSION, "matmul: bad shape");
     TLC_REQUIRE(k == k2, TLC_ERR_INVALID_OPERATION, "matmul shape mismatch: [%d, %d] @ [%d, %d]", m, k, k2, n);
     if (m == 0 || n == 0) return TLC_OK;
-    const dim3 grid((unsigned)((n + 63) / 64), (unsigned)((m + 63) / 64));
-    matmul_f16_kernel<<<grid, 256, 0, ctx->stream>>>(static_cast<const __half *>(a_dev), static_cast<const __half *>(b_dev),
-                                                     static_cast<__half *>(y_dev), m, k, n);
-    TLC_CHECK_LAUNCH(ctx);
+    if (k > 0) return tlc_launch_matmul_f16(ctx, a_dev, b_dev, y_dev, m, k, n);
+    TLC_CUDA(cudaMemsetAsync(y_dev, 0, (size_t)m * n * 2, ctx->stream));  // a sum of nothing
     return TLC_OK;
 }
 
