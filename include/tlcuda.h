@@ -96,7 +96,6 @@ TLC_API int32_t tlc_destroy(tlc_ctx *ctx);
  *   "pdl_mode"    when a GEMV lets the next kernel of the stream be scheduled: 1 = at once,
  *                 2 = after its last slab, 3 = after its own dependency wait, 4 (default) = 3 for
  *                 kernels that stream 40 MB of weights or more and 2 for shorter ones;
- *   "l2_hint"     the GEMV's weight copies carry the evict-first L2 hint (1, default) or none (0);
  *   "host_graph"  tlc_llama_decode_host runs as one graph launch with copy nodes (1, default)
  *                 or as copy + graph + copy (0);
  *   "host_poll"   with host_graph: the host watches the pinned result words (1, default)
@@ -117,11 +116,14 @@ TLC_API int32_t tlc_destroy(tlc_ctx *ctx);
  *   "gemm_pair"   from 129 activation rows on, the GEMM runs on CTA pairs (tcgen05 cta_group::2,
  *                 persistent, two accumulators in tensor memory) (1) or on single CTAs (0,
  *                 default: faster on a B200);
- *   "gemv_splitk" 2 to 16 activation rows whose fragments crowd the shared memory: K is cut into
- *                 windows, one pass over the weights (2, default: windows sized for one CTA per
- *                 SM; 1: for two CTAs per SM) or several passes (0);
- *   "gemv_f8"     one activation row of a Q4_0 weight on the FP8 tensor-core form (1) or the
- *                 f16 form (0, default: faster);
+ *   "gemm_wt_max_m" activation rows up to which quantized linears of 17 and more rows put the weight
+ *                 rows on the M side of the MMA (default: decided from the shape; the options above
+ *                 that force a detail of the other form ask for that form);
+ *   "gemm_wt_bn"  activation rows per tile of that form (a multiple of 16 up to 256; 0 = from the shape);
+ *   "gemm_wt_ks"  CTAs per tile of that form, 1..8, or 9 = tiles dealt out step by step (0 = from the shape);
+ *   "gemv_splitk" accepted and without effect: 2 to 16 rows always take one pass over the weights;
+ *   "gemv_f8"     accepted and without effect: one row always runs on the f16 form;
+ *   "l2_hint"     accepted and without effect: the weight copies always carry the evict-first L2 hint;
  *   "q6k_resident" Q6_K tensors stay quantized in HBM (1, default) or become f16 at upload (0);
  *   "attn_wide"   decode attention of one sequence with at most four KV heads over a long
  *                 context runs on clusters of sixteen key splits (1) or eight (0, default: no slower).

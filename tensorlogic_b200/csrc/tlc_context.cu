@@ -89,12 +89,9 @@ extern "C" int32_t tlc_init(int32_t ordinal, tlc_ctx **out) {
     if (const char *e = getenv("TLC_GEMM_PG")) ctx->gemm_pg = atoi(e);
     if (const char *e = getenv("TLC_GEMM_TMA")) ctx->gemm_tma = atoi(e) != 0;
     if (const char *e = getenv("TLC_ATTN_WIDE")) ctx->attn_wide = atoi(e);
-    if (const char *e = getenv("TLC_L2_HINT")) ctx->l2_hint = atoi(e);
     if (const char *e = getenv("TLC_HOST_GRAPH")) ctx->host_graph = atoi(e) != 0;
     if (const char *e = getenv("TLC_HOST_POLL")) ctx->host_poll = atoi(e) != 0;
     if (const char *e = getenv("TLC_STEP_KERNEL")) ctx->step_kernel = atoi(e) != 0;
-    if (const char *e = getenv("TLC_GEMV_F8")) ctx->gemv_f8 = atoi(e) != 0;
-    if (const char *e = getenv("TLC_GEMV_SPLITK")) ctx->gemv_splitk = atoi(e);
     if (const char *e = getenv("TLC_Q6K_RESIDENT")) ctx->q6k_resident = atoi(e) != 0;
     *out = ctx;
     return TLC_OK;
@@ -141,18 +138,14 @@ extern "C" int32_t tlc_set_option(tlc_ctx *ctx, const char *name, int64_t value)
         ctx->pdl_mode = (int)value;
     } else if (n == "attn_wide")
         ctx->attn_wide = (int)value;
-    else if (n == "l2_hint")
-        ctx->l2_hint = value != 0;
     else if (n == "host_graph")
         ctx->host_graph = value != 0;
     else if (n == "host_poll")
         ctx->host_poll = value != 0;
     else if (n == "step_kernel")
         ctx->step_kernel = value != 0;
-    else if (n == "gemv_f8")
-        ctx->gemv_f8 = value != 0;
-    else if (n == "gemv_splitk")
-        ctx->gemv_splitk = (int)value;
+    else if (n == "gemv_f8" || n == "gemv_splitk" || n == "l2_hint")
+        ;  // forms that no longer exist (see the header)
     else if (n == "q6k_resident")
         ctx->q6k_resident = value != 0;
     else

@@ -7,31 +7,34 @@
 // and of the separate rms_norm / rope / sigmoid / mul / add launches around
 // them in the TL scripts (debug/chat_demo_with_kvcache.tl:219-290).
 //
-// Design (the weight bytes are read from HBM exactly once):
-//   * persistent CTAs, up to two per SM, each walking 16-row slabs of the weight(s);
-//   * a producer warp streams the tiles of a slab into a shared memory ring,
-//     ONE bulk async copy of up to 18 KB per stage (a stage's 16 tiles are
-//     contiguous in HBM), completing on mbarriers -- no thread ever issues a
-//     narrow global load for weight data, and the ring keeps tens of KB per SM
-//     in flight independent of occupancy;
-//   * eight consumer warps read their fragment words with two conflict-free
-//     16-byte shared loads per tile and unpack nibbles / bytes in registers
-//     straight into f16 tensor-core fragments: a 4-bit (8-bit) integer n placed
-//     in the low mantissa bits of a binary16 is the subnormal n * 2^-24, so one
-//     AND per pair of weights yields an exact A fragment; the -8 (-128) offset is
-//     carried by the accumulator's initial value (-8 * sum of the 32
-//     activations of the block) and the block scale d multiplies the 16x8 block
-//     result in f32;  mma.sync m16n8k16 with f32 accumulation does the dot
-//     products for up to 8 activation rows at no extra cost;
-//   * the K range of a slab is split over the eight warps, reduced through
-//     shared memory (up to four slabs per reduction), and the epilogue (f16 rounding, bias / residual add,
-//     SiLU(gate)*up, interleaved RoPE) is applied before the single store.
-// The activation vector(s) are optionally RMS-normalised on the way into
-// shared memory, where they are kept pre-permuted in fragment order.
+// Common to both kernels (the weight bytes are read from HBM exactly once):
+//   * persistent CTAs, up to two per SM, each walking 16-row slabs of the weight(s); the tiles of a slab
+//     arrive through a shared memory ring in bulk async copies (a slab's tiles are contiguous in HBM),
+//     completing on mbarriers -- no thread ever issues a narrow global load for weight data, and the
+//     ring keeps tens of KB per SM in flight independent of occupancy;
+//   * consumer warps read their fragment words with two conflict-free 16-byte shared loads per tile and
+//     unpack nibbles / bytes in registers straight into f16 tensor-core fragments: a 4-bit (8-bit) integer n
+//     placed in the low mantissa bits of a binary16 is the subnormal n * 2^-24, so one AND per pair of
+//     weights yields an exact A fragment; the -8 (-128) offset is carried by the accumulator's initial value
+//     (-8 * sum of the 32 activations of the block) and the block scale d multiplies the 16x8 block
+//     result in f32;  mma.sync m16n8k16 with f32 accumulation does the dot products for up to 8
+//     activation rows at no extra cost (8 clocks per sub-core, as long as the unpacking of its block takes
+//     the integer pipe, which needs two clocks an operation);
+//   * the K range of a slab is split over the warps, reduced through shared memory (several slabs per
+//     reduction), and the epilogue (f16 rounding, bias / residual add, SiLU(gate)*up, interleaved RoPE)
+//     is applied before the single store.
+// One row (tlc_gemv_row1.cuh): the row, optionally RMS-normalised, lies in shared memory in fragment order.
+// 2 to 16 rows (tlc_gemv_kernel.cuh): that copy would be read 512 bytes a block and warp, by far more than the
+// weights, and crowd out the ring.  Each warp keeps its share of K of all rows in registers for the whole
+// launch instead, a K longer than a CTA's registers hold is shared out over a thread-block cluster,
+// and the RMSNorm is done once by a kernel of its own (frag_rows_kernel) and not by every CTA.  Measured on one
+// B200, before -> now: Q4_0 4096 x 4096, 8 rows 10.1 -> 7.1 us; norm + 7168 x 8192 at 8 / 16 rows 31.2 -> 18.0 /
+// 43.8 -> 24 us; norm + 2560 x 2048 at 5 / 16 rows 9.5 -> 6.4 / 19.3 -> 8.1 us; 28672 x 8192 at 8 rows 42.8 -> 35.9 us.
 #include <cuda_fp16.h>
 
 #include "tlc_gemm_wt.h"
 #include "tlc_gemv_kernel.cuh"
+#include "tlc_gemv_row1.cuh"
 #include "tlc_internal.h"
 #include "tlc_tile.cuh"
 
@@ -248,27 +251,36 @@ __global__ void __launch_bounds__(256) gemv_splitk_finish_kernel(const GemvParam
     }
 }
 
-template <int QT, int NT, int AS, bool M1, int CW, bool F8 = false>
-int32_t launch_mma_as(tlc_ctx *ctx, GemvParams &p, int grid, size_t smem) {
-    static bool configured[64] = {};
+// Launches a GEMV kernel (fn) in `threads`-wide CTAs with all the shared memory it asks for, PDL and, with
+// p.ksplit > 1, clusters; `configured` belongs to fn.
+int32_t launch_kernel(tlc_ctx *ctx, void (*fn)(GemvParams), bool (&configured)[64], const GemvParams &p, int grid, int threads,
+                      size_t smem) {
     if (!configured[ctx->device & 63]) {
-        TLC_CUDA(cudaFuncSetAttribute(gemv_mma_kernel<QT, NT, AS, M1, CW, F8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)ctx->prop.sharedMemPerBlockOptin));
-        TLC_CUDA(cudaFuncSetAttribute(gemv_mma_kernel<QT, NT, AS, M1, CW, F8>,
-                                      cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+        TLC_CUDA(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx->prop.sharedMemPerBlockOptin));
+        TLC_CUDA(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+        TLC_CUDA(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         configured[ctx->device & 63] = true;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((CW + 1) * 32);
+    cfg.blockDim = dim3((unsigned)threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    int na = 0;
+    if (ctx->use_pdl) {
+        attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[na++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (p.ksplit > 1) {
+        attr[na].id = cudaLaunchAttributeClusterDimension;
+        attr[na].val.clusterDim.x = (unsigned)p.ksplit;
+        attr[na].val.clusterDim.y = 1;
+        attr[na++].val.clusterDim.z = 1;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = ctx->use_pdl ? 1 : 0;
-    cudaError_t le = cudaLaunchKernelEx(&cfg, gemv_mma_kernel<QT, NT, AS, M1, CW, F8>, p);
+    cfg.numAttrs = na;
+    cudaError_t le = cudaLaunchKernelEx(&cfg, fn, p);
     if (le != cudaSuccess) {
         cudaGetLastError();
         return tlc_fail(TLC_ERR_CUDA, "gemv launch failed: %s", cudaGetErrorString(le));
@@ -276,73 +288,49 @@ int32_t launch_mma_as(tlc_ctx *ctx, GemvParams &p, int grid, size_t smem) {
     TLC_CHECK_LAUNCH(ctx);
     return TLC_OK;
 }
-
-template <int QT, int NT, int CW>
-int32_t launch_mma_cw(tlc_ctx *ctx, GemvParams &p, int grid, size_t smem, int as, bool f8) {
-    if constexpr (NT == 1 && QT == TLC_TYPE_Q4_0) {
-        if (p.m == 1 && f8) {  // one sequence, Q4_0: the FP8-limb form of the dot products
-            if (as == 1) return launch_mma_as<QT, 1, 1, true, CW, true>(ctx, p, grid, smem);
-            if (as == 2) return launch_mma_as<QT, 1, 2, true, CW, true>(ctx, p, grid, smem);
-            return launch_mma_as<QT, 1, 4, true, CW, true>(ctx, p, grid, smem);
-        }
-    }
-    if constexpr (NT == 1) {
-        if (p.m == 1) {  // the decode step of one sequence
-            if (as == 1) return launch_mma_as<QT, 1, 1, true, CW>(ctx, p, grid, smem);
-            if (as == 2) return launch_mma_as<QT, 1, 2, true, CW>(ctx, p, grid, smem);
-            return launch_mma_as<QT, 1, 4, true, CW>(ctx, p, grid, smem);
-        }
-    }
-    if (as == 1) return launch_mma_as<QT, NT, 1, false, CW>(ctx, p, grid, smem);
-    if (as == 2) return launch_mma_as<QT, NT, 2, false, CW>(ctx, p, grid, smem);
-    return launch_mma_as<QT, NT, 4, false, CW>(ctx, p, grid, smem);
+template <int QT, int NT, int TI, int CW>
+int32_t launch_rows(tlc_ctx *ctx, const GemvParams &p, int grid, size_t smem) {
+    static bool configured[64] = {};
+    return launch_kernel(ctx, gemv_mma_kernel<QT, NT, TI, CW>, configured, p, grid, CW * 32, smem);
+}
+template <int QT, int AS, int CW>
+int32_t launch_row1_as(tlc_ctx *ctx, const GemvParams &p, int grid, size_t smem) {
+    static bool configured[64] = {};
+    return launch_kernel(ctx, gemv_row1_kernel<QT, AS, CW>, configured, p, grid, (CW + 1) * 32, smem);
 }
 
-template <int QT, int NT>
-int32_t launch_mma(tlc_ctx *ctx, GemvParams &p) {
-    using T = QTraits<QT>;
-    constexpr size_t STAGE_BYTES = (size_t)kTilesPerStage * T::TILE_BYTES;
+// One activation row.
+template <int QT>
+int32_t launch_row1(tlc_ctx *ctx, GemvParams &p) {
+    constexpr size_t STAGE_BYTES = (size_t)kTilesPerStage * QTraits<QT>::TILE_BYTES;
+    p.ksplit = 1;
+    p.nblk_pad = p.ktiles * QTraits<QT>::TB;
+    p.nchunks = (p.ktiles + kTilesPerStage - 1) / kTilesPerStage;
     const size_t budget = (size_t)ctx->prop.sharedMemPerBlockOptin;
-    // One activation row of a Q4_0 weight runs on the FP8 form (option "gemv_f8"), as long as its
-    // limbs (128 bytes per block) leave room for the ring.
-    bool f8 = QT == TLC_TYPE_Q4_0 && NT == 1 && p.m == 1 && ctx->gemv_f8;
-    if (f8 && fixed_smem_bytes(p.nblk_pad, p.m, NT, p.subs, 8, true) + 3 * STAGE_BYTES > budget) f8 = false;
-    auto fixed_smem_bytes = [f8](int nblk_pad, int m, int nt, int as, int cw = 8) {
-        return tlc_gemv::fixed_smem_bytes(nblk_pad, m, nt, as, cw, f8);
-    };
-    const size_t fixed1 = fixed_smem_bytes(p.nblk_pad, p.m, NT, p.subs);
-    TLC_REQUIRE(fixed1 + 2 * STAGE_BYTES <= budget, TLC_ERR_INVALID_OPERATION,
-                "gemv: activations of %d x %d do not fit in shared memory", p.m, p.k);
+    TLC_REQUIRE(row1_fixed_smem(p.nblk_pad, p.subs) + 2 * STAGE_BYTES <= budget, TLC_ERR_INVALID_OPERATION,
+                "gemv: K = %d too large for the shared-memory staging", p.k);
     // Two CTAs per SM (16 consumer warps hide the shared-memory and MMA latency
     // of the unpack loop) whenever the activations leave room for at least
     // three ring stages in half of the SM's shared memory.
     const size_t half = (size_t)ctx->prop.sharedMemPerMultiprocessor / 2 - 1024;
-    const bool fits_half = fixed1 + 3 * STAGE_BYTES <= half;
     // (Measured on the TinyLlama decode step: keeping small launches at one CTA per
     // SM, to leave room for the next kernel's early CTAs, costs 8 % against
     // letting them spread over two CTAs per SM.)
-    const bool two = fits_half;
-    // One CTA per SM: sixteen consumer warps instead of eight, if the larger reduction
-    // buffers still leave three ring stages.
-    const int cw = !two && fixed_smem_bytes(p.nblk_pad, p.m, NT, p.subs, 16) + 3 * STAGE_BYTES <= budget ? 16 : 8;
+    const bool two = row1_fixed_smem(p.nblk_pad, p.subs) + 3 * STAGE_BYTES <= half;
+    // One CTA per SM: sixteen consumer warps instead of eight, if three ring stages remain.
+    const int cw = !two && row1_fixed_smem(p.nblk_pad, p.subs, 16) + 3 * STAGE_BYTES <= budget ? 16 : 8;
     const size_t cap = two ? half : budget;
     const int max_ctas = two ? 2 * ctx->sm_count : ctx->sm_count;
-    const int ks = p.ksplit > 1 ? p.ksplit : 1;
-    // Split K: the CTAs come in groups of ks (one per window); a group shares the slabs.
-    int grid = p.total_units * ks < max_ctas ? p.total_units * ks : max_ctas;
-    grid -= grid % ks;
-    if (grid < ks) grid = ks;
+    const int grid = p.total_units < max_ctas ? p.total_units : max_ctas;
     // Accumulator sets per reduction: enough units for about four ring stages
-    // between two cross-warp reductions, as far as this CTA has units and the
-    // shared memory (reduction buffers grow with the sets) allows.
-    const int units_per_cta = (p.total_units + grid / ks - 1) / (grid / ks);
+    // between two cross-warp reductions, as far as this CTA has units.
+    const int units_per_cta = (p.total_units + grid - 1) / grid;
     const int iters_per_unit = p.subs * p.nchunks;
     int ub = (4 + iters_per_unit - 1) / iters_per_unit;
     if (ub > units_per_cta) ub = units_per_cta;
     int as = p.subs;
-    while (as < ub * p.subs && as < (NT == 2 ? 2 : 4)) as *= 2;
-    while (as > p.subs && fixed_smem_bytes(p.nblk_pad, p.m, NT, as, cw) + 3 * STAGE_BYTES > cap) as /= 2;
-    const size_t smem_fixed = fixed_smem_bytes(p.nblk_pad, p.m, NT, as, cw);
+    while (as < ub * p.subs && as < 4) as *= 2;
+    const size_t smem_fixed = row1_fixed_smem(p.nblk_pad, as, cw);
     // No more stages than this CTA will ever fill.
     const long per_cta = (long)units_per_cta * p.subs * p.nchunks;
     int stages = (int)((cap - smem_fixed) / STAGE_BYTES);
@@ -355,13 +343,120 @@ int32_t launch_mma(tlc_ctx *ctx, GemvParams &p) {
     // 9.74 ms per token).  Shorter kernels keep the late trigger (TinyLlama decode: 2.2 % slower with
     // the early one from three stages on, 0.5 % slower with it everywhere).
     p.pdl_mode = ctx->pdl_mode == 4 ? (per_cta >= 8 ? 3 : 2) : ctx->pdl_mode;
-    p.l2_hint = ctx->l2_hint;
     p.contig = units_per_cta <= 4 ? 1 : 0;
     const size_t smem = smem_fixed + (size_t)stages * STAGE_BYTES;
-    return cw == 16 ? launch_mma_cw<QT, NT, 16>(ctx, p, grid, smem, as, f8) : launch_mma_cw<QT, NT, 8>(ctx, p, grid, smem, as, f8);
+    if (cw == 16)
+        return as == 1   ? launch_row1_as<QT, 1, 16>(ctx, p, grid, smem)
+               : as == 2 ? launch_row1_as<QT, 2, 16>(ctx, p, grid, smem)
+                         : launch_row1_as<QT, 4, 16>(ctx, p, grid, smem);
+    return as == 1   ? launch_row1_as<QT, 1, 8>(ctx, p, grid, smem)
+           : as == 2 ? launch_row1_as<QT, 2, 8>(ctx, p, grid, smem)
+                     : launch_row1_as<QT, 4, 8>(ctx, p, grid, smem);
 }
 
-size_t gemv_fixed_smem(int nblk_pad, int m, int nt) { return fixed_smem_bytes(nblk_pad, m, nt, 2); }
+// Clusters of ks sixteen-warp CTAs that the device holds at once (asked once, with all of the shared memory).
+int gemv_clusters(tlc_ctx *ctx, int ks) {
+    static int known[64][17];
+    int &n = known[ctx->device & 63][ks];
+    if (n == 0) {
+        auto fn = gemv_mma_kernel<TLC_TYPE_Q4_0, 1, 1, 16>;
+        cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx->prop.sharedMemPerBlockOptin);
+        cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)ks);
+        cfg.blockDim = dim3(16 * 32);
+        cfg.dynamicSmemBytes = ctx->prop.sharedMemPerBlockOptin - 2048;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)ks;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) != cudaSuccess || n < 1) {
+            cudaGetLastError();
+            n = -1;
+        }
+    }
+    return n;
+}
+
+// Tiles along K that one launch can hold the activations of, per row tile count.
+constexpr int kMaxCluster = 16;
+template <int QT> constexpr int max_window(int nt, int cw) { return cw * tiles_of<QT>(nt == 1 ? 3 : 2); }
+
+// 2 to 16 activation rows.
+template <int QT, int NT>
+int32_t launch_mma(tlc_ctx *ctx, GemvParams &p) {
+    constexpr int TILE = QTraits<QT>::TILE_BYTES, T1 = tiles_of<QT>(1);
+    const size_t budget = (size_t)ctx->prop.sharedMemPerBlockOptin;
+    const size_t half = (size_t)ctx->prop.sharedMemPerMultiprocessor / 2 - 1024;
+    // A warp keeps its share of the activations in registers (up to 12 blocks of K, 8 for two row
+    // tiles): eight warps and two CTAs per SM hold K = 3072, sixteen warps and one CTA 6144; a
+    // longer K is shared out over the CTAs of a cluster.
+    const int cw = p.ktiles <= max_window<QT>(NT, 8) ? 8 : 16;
+    int ks = cw == 8 ? 1 : (p.ktiles + max_window<QT>(NT, 16) - 1) / max_window<QT>(NT, 16);
+    // ... over enough of them that three stages of the ring fit
+    while (ks > 1 && ks < 8 && (size_t)((p.ktiles + ks - 1) / ks) * TILE > 52 * 1024) ks++;
+    TLC_REQUIRE(ks <= kMaxCluster, TLC_ERR_INVALID_OPERATION, "gemv: K = %d too large", p.k);
+    int max_ctas = cw == 8 ? 2 * ctx->sm_count : ctx->sm_count;
+    if (ks > 1) {
+        const int n = gemv_clusters(ctx, ks);
+        TLC_REQUIRE(n >= 1, TLC_ERR_INVALID_OPERATION, "gemv: K = %d needs a cluster of %d CTAs", p.k, ks);
+        max_ctas = n * ks;
+    }
+    p.ksplit = ks;
+    p.ktiles_win = (p.ktiles + ks - 1) / ks;
+    p.tiles_warp = (p.ktiles_win + cw - 1) / cw;
+    const int ti = (p.tiles_warp + T1 - 1) / T1;
+    p.stage_bytes = p.ktiles_win * TILE;
+    p.m_inv = 65536 / p.m + 1;
+    int grid = p.total_units * ks < max_ctas ? p.total_units * ks : max_ctas;
+    const int units_per_cta = (p.total_units + grid / ks - 1) / (grid / ks);
+    const size_t cap = cw == 8 ? half : budget;
+    // Slabs between two cross-warp reductions, and (clusters) between two exchanges.
+    int batch = NT == 1 ? 4 : 2;
+    while (batch > p.subs && batch > units_per_cta * p.subs) batch /= 2;
+    if (batch < p.subs) batch = p.subs;
+    GemvSmem lay;
+    for (;; batch /= 2) {
+        p.batch = batch;
+        p.round = 0;
+        p.n_rounds = 1;
+        if (ks > 1) {
+            int round = (NT == 1 ? 64 : 32) / batch * batch;
+            const int all = (units_per_cta * p.subs + batch - 1) / batch * batch;
+            p.round = round < all ? round : all;
+            p.n_rounds = (units_per_cta * p.subs + p.round - 1) / p.round;
+        }
+        lay = gemv_smem(cw, ti, NT, p.batch, p.round);
+        if ((size_t)lay.ring + 3 * (size_t)p.stage_bytes <= cap || batch <= p.subs) break;
+    }
+    // No more stages than this CTA will ever fill.
+    const int per_cta = units_per_cta * p.subs;
+    int stages = lay.ring < (int)cap ? (int)((cap - lay.ring) / p.stage_bytes) : 0;
+    TLC_REQUIRE(stages >= 1, TLC_ERR_INVALID_OPERATION, "gemv: K = %d does not fit in shared memory", p.k);
+    if (stages > 8) stages = 8;
+    if (stages > per_cta) stages = per_cta;
+    p.nstages = stages;
+    // Mode 4 decides per launch.  A kernel whose CTAs stream 150 KB or more (40 MB over the grid, about 6 us
+    // of HBM time) lets its successor in right after its own dependency wait: the successor is then resident
+    // with its ring filled when this grid ends (Llama-70B decode: 10.07 -> 9.74 ms per token).  Shorter kernels
+    // keep the late trigger (TinyLlama decode: 2.2 % slower with the early one from 54 KB on, 0.5 %
+    // slower with it everywhere).
+    p.pdl_mode = ctx->pdl_mode == 4 ? ((size_t)per_cta * p.stage_bytes >= 147456 ? 3 : 2) : ctx->pdl_mode;
+    p.contig = units_per_cta <= 4 ? 1 : 0;
+    const size_t smem = (size_t)lay.ring + (size_t)stages * p.stage_bytes;
+#define TLC_GEMV_CASE(TI) \
+    if (ti == TI) return cw == 8 ? launch_rows<QT, NT, TI, 8>(ctx, p, grid, smem) : launch_rows<QT, NT, TI, 16>(ctx, p, grid, smem);
+    TLC_GEMV_CASE(1)
+    TLC_GEMV_CASE(2)
+    if constexpr (NT == 1) {
+        TLC_GEMV_CASE(3)
+    }
+#undef TLC_GEMV_CASE
+    return tlc_fail(TLC_ERR_INVALID_OPERATION, "gemv: K = %d too large", p.k);
+}
 
 }  // namespace
 
@@ -388,69 +483,8 @@ int32_t tlc_selftest_mbarrier_wait(tlc_ctx *ctx) {
     return TLC_OK;
 }
 
-// Largest number of activation rows one launch can take for this K.
-static int gemv_max_m(tlc_ctx *ctx, int type, int k) {
-    const int nblk_pad = (int)tlc_tile::k_tiles(type, k) * tlc_tile::tile_blocks(type);
-    const size_t budget = (size_t)ctx->prop.sharedMemPerBlockOptin;
-    const size_t stage = (size_t)kTilesPerStage * tlc_tile::tile_bytes(type);
-    for (int m = 16; m >= 1; m--) {
-        int nt = m > 8 ? 2 : 1;
-        if (gemv_fixed_smem(nblk_pad, m, nt) + 3 * stage <= budget) return m;
-    }
-    return 0;
-}
-
-// Split K for several activation rows.  The rows sit in shared memory in fragment order, 64 bytes
-// per block and row: 8 rows of K = 8192 already take half an SM's shared memory, 16 rows of
-// K = 28672 eight times an SM's.  Instead of passing over the weights once per group of rows that
-// fits, the K range is cut into windows: every CTA keeps only its window of the rows, the windows'
-// f32 partial sums meet in gemv_splitk_finish_kernel.  The weights are read once.
-// Returns the number of windows (1: no split) for m rows, of which max_m fit in one unsplit launch.
-//  - A launch that runs two CTAs per SM without a split is left alone.
-//  - More than four rows that fit one launch at one CTA per SM stay unsplit (sixteen consumer
-//    warps; 8 rows of K = 8192: 44 us against 50 us split).
-//  - Otherwise the windows are sized for one CTA per SM with sixteen consumer warps (option
-//    gemv_splitk = 2, the default: 16 rows of K = 8192 take 76 us, against 120 us with windows
-//    for two CTAs per SM and 87 us in two passes), else, or first with gemv_splitk = 1, for two
-//    CTAs per SM; a window holds at least eight tiles.
-static int gemv_choose_ksplit(tlc_ctx *ctx, int type, int64_t ktiles, int m, int n_sub, int max_m, int mode) {
-    const int tb = tlc_tile::tile_blocks(type);
-    const size_t stage = (size_t)kTilesPerStage * tlc_tile::tile_bytes(type);
-    const size_t half = (size_t)ctx->prop.sharedMemPerMultiprocessor / 2 - 1024;
-    const size_t budget = (size_t)ctx->prop.sharedMemPerBlockOptin;
-    const int nt = m > 8 ? 2 : 1;
-    auto fits = [&](int64_t win, bool two) {
-        return fixed_smem_bytes((int)win * tb, m, nt, n_sub, two ? 8 : 16) + 3 * stage <= (two ? half : budget);
-    };
-    if (fits(ktiles, true)) return 1;
-    const bool multi_pass = m > max_m;
-    if (!multi_pass && m > 4) return 1;
-    static const int cand[] = {2, 3, 4, 6, 8, 12, 16, 24, 32};
-    for (int round = 0; round < 2; round++) {
-        const bool two = (round == 0) != (mode == 2);
-        if (!two && !multi_pass) continue;  // one CTA per SM is what the unsplit launch already does
-        for (int ks : cand) {
-            const int64_t win = (ktiles + ks - 1) / ks;
-            if (win < 8) break;
-            if (fits(win, two)) return ks;
-        }
-    }
-    return 1;
-}
-
-// Bytes of context scratch a fused linear over m rows of width k with n_total outputs may need
-// (the split-K partial sums); callers that capture graphs reserve it up front.
-size_t tlc_gemv_scratch_bytes(tlc_ctx *ctx, int type, int64_t k, int m, int64_t n_total) {
-    if ((type != TLC_TYPE_Q4_0 && type != TLC_TYPE_Q8_0) || m < 2 || m > 16) return 0;
-    const int max_m = gemv_max_m(ctx, type, (int)k);
-    int ks = 1;
-    for (int mode = 1; mode <= 2; mode++)  // whatever the option says at launch time
-        for (int n_sub = 1; n_sub <= 2; n_sub++) {
-            const int c = gemv_choose_ksplit(ctx, type, tlc_tile::k_tiles(type, k), m, n_sub, max_m, mode);
-            ks = c > ks ? c : ks;
-        }
-    return ks > 1 ? (size_t)ks * m * (size_t)n_total * sizeof(float) : 0;
-}
+// Scratch the RMSNorm of 2..16 rows of width k takes (their fragment order).
+size_t tlc_gemv_scratch_bytes(int64_t k) { return frag_total_bytes(k / 32, 2); }
 
 int32_t tlc_gemv_splitk_finish(tlc_ctx *ctx, const tlc_gemv_args &a, int ksplit, float *partial) {
     GemvParams p{};
@@ -599,18 +633,9 @@ int32_t tlc_launch_gemv(tlc_ctx *ctx, const tlc_gemv_args &a) {
 
     if (tlc_gemm_eligible(ctx, a)) return tlc_launch_gemm(ctx, a);
 
-    int max_m = gemv_max_m(ctx, type, (int)k);
-    TLC_REQUIRE(max_m >= 1, TLC_ERR_INVALID_OPERATION, "gemv: K = %lld too large for the shared-memory staging",
-                (long long)k);
-    // Up to 16 rows whose fragments do not leave two CTAs per SM room: one pass with K cut into windows.
-    int ksplit = 1;
-    if (a.m >= 2 && a.m <= 16 && ctx->gemv_splitk) {
-        ksplit = gemv_choose_ksplit(ctx, type, w0->k_tiles, a.m, a.epilogue == TLC_EPI_SWIGLU ? 2 : 1, max_m,
-                                    ctx->gemv_splitk);
-        if (ksplit > 1) max_m = a.m;
-    }
-    // Otherwise activation rows beyond what one launch can hold are processed in
-    // further passes over the weights.
+    // (rows beyond sixteen come here only when an option keeps them from the GEMM)
+    const int64_t nt2_tiles = kMaxCluster * (type == TLC_TYPE_Q4_0 ? max_window<TLC_TYPE_Q4_0>(2, 16) : max_window<TLC_TYPE_Q8_0>(2, 16));
+    const int max_m = w0->k_tiles <= nt2_tiles ? 16 : 8;
     for (int m0 = 0; m0 < a.m; m0 += max_m) {
         const int mc = a.m - m0 < max_m ? a.m - m0 : max_m;
         GemvParams p{};
@@ -639,8 +664,6 @@ int32_t tlc_launch_gemv(tlc_ctx *ctx, const tlc_gemv_args &a) {
         p.k = (int)k;
         p.nblk = (int)(k / 32);
         p.ktiles = (int)w0->k_tiles;
-        p.nblk_pad = p.ktiles * tlc_tile::tile_blocks(type);
-        p.nchunks = (p.ktiles + kTilesPerStage - 1) / kTilesPerStage;
         p.m = mc;
         p.x = static_cast<const __half *>(a.x) + (size_t)m0 * k;
         p.norm_w = static_cast<const __half *>(a.norm_w);
@@ -654,38 +677,32 @@ int32_t tlc_launch_gemv(tlc_ctx *ctx, const tlc_gemv_args &a) {
         p.max_pos = a.max_pos;
         p.status = ctx->dev_status;
         p.wait_ns = ctx->wait_ns;
-        if (ksplit > 1) {
-            p.ksplit = ksplit;
-            p.ktiles_full = p.ktiles;
-            p.ktiles_win = (p.ktiles + ksplit - 1) / ksplit;
-            p.ntot = 0;
-            for (int i = 0; i < a.n_out; i++) p.ntot += p.t[i].n;
-            // what the launcher sizes shared memory, stages and batches by: one window
-            p.ktiles = p.ktiles_win;
-            p.nblk_pad = p.ktiles_win * tlc_tile::tile_blocks(type);
-            p.nblk = p.nblk_pad;
-            p.nchunks = (p.ktiles_win + kTilesPerStage - 1) / kTilesPerStage;
-            const size_t need = (size_t)ksplit * mc * (size_t)p.ntot * sizeof(float);
-            if (int32_t rc = tlc_scratch_reserve(ctx, need)) return rc;
-            p.partial = static_cast<float *>(ctx->scratch);
-        }
         const int nt = mc > 8 ? 2 : 1;
+        const bool q4 = type == TLC_TYPE_Q4_0;
+        if (mc > 1 && a.norm_w) {
+            const int64_t nblk = k / 32;
+            if (int32_t rc = tlc_scratch_reserve(ctx, frag_total_bytes(nblk, nt))) return rc;
+            uint4 *frag = static_cast<uint4 *>(ctx->scratch);
+            float *start = reinterpret_cast<float *>(static_cast<uint8_t *>(ctx->scratch) + frag_bytes(nblk, nt));
+            const cudaError_t le = tlc_launch_pdl(ctx, q4 ? frag_rows_kernel<TLC_TYPE_Q4_0> : frag_rows_kernel<TLC_TYPE_Q8_0>, dim3(8 * nt),
+                                                  dim3(512), 0, p.x, p.norm_w, mc, (int)k, a.eps, frag, start, nt);
+            if (le != cudaSuccess) {
+                cudaGetLastError();
+                return tlc_fail(TLC_ERR_CUDA, "gemv: RMSNorm launch failed: %s", cudaGetErrorString(le));
+            }
+            TLC_CHECK_LAUNCH(ctx);
+            p.frag = frag;
+            p.start = start;
+            p.norm_w = nullptr;
+        }
         int32_t rc;
-        if (type == TLC_TYPE_Q4_0)
+        if (mc == 1)
+            rc = q4 ? launch_row1<TLC_TYPE_Q4_0>(ctx, p) : launch_row1<TLC_TYPE_Q8_0>(ctx, p);
+        else if (q4)
             rc = nt == 1 ? launch_mma<TLC_TYPE_Q4_0, 1>(ctx, p) : launch_mma<TLC_TYPE_Q4_0, 2>(ctx, p);
         else
             rc = nt == 1 ? launch_mma<TLC_TYPE_Q8_0, 1>(ctx, p) : launch_mma<TLC_TYPE_Q8_0, 2>(ctx, p);
         if (rc) return rc;
-        if (ksplit > 1) {
-            const int nout = p.subs == 2 ? p.t[0].n : p.ntot;
-            const size_t total = (size_t)mc * nout;
-            cudaError_t le = tlc_launch_pdl(ctx, gemv_splitk_finish_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, p);
-            if (le != cudaSuccess) {
-                cudaGetLastError();
-                return tlc_fail(TLC_ERR_CUDA, "split-K finish launch failed: %s", cudaGetErrorString(le));
-            }
-            TLC_CHECK_LAUNCH(ctx);
-        }
     }
     return TLC_OK;
 }

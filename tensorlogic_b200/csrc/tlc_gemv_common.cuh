@@ -5,6 +5,8 @@
 
 #include <cuda_fp16.h>
 
+#include <climits>
+
 #include "tlc_internal.h"
 
 namespace tlc_gemv {
@@ -15,7 +17,6 @@ constexpr int kRows = 16;  // rows of W per slab (the M of m16n8k16)
 // one reduction over twice the warps).  Launches whose activations leave room for
 // one CTA only (several rows of a long K) take the sixteen-warp form.
 constexpr int kMaxStages = 12;
-constexpr int kHeaderBytes = 1536;  // mbarriers, abort flag, sum-of-squares partials
 
 // Weights arrive in the tiled layout of tlc_tile.cuh: a ring stage is 16
 // consecutive tiles of one 16-row slab (Q4_0: 64 blocks, Q8_0: 32 blocks of K).
@@ -51,12 +52,15 @@ struct GemvParams {
     int subs;      // slabs per unit (2 for the gate/up pair)
     int k;
     int nblk;      // k / 32
-    int nblk_pad;  // rounded up to whole tiles
+    int nblk_pad;  // one row: rounded up to whole tiles
     int ktiles;    // tiles per slab
-    int nchunks;   // ring stages per slab
+    int nchunks;   // one row: ring stages per slab
     int m;
     const __half *x;
-    const __half *norm_w;
+    const uint4 *frag;   // 2..16 rows: the activations in fragment order (then x is not read), and
+    const float *start;  //   the accumulator start values of their blocks
+    int m_inv;           // 65536 / m + 1
+    const __half *norm_w;  // one row
     float eps;
     int epilogue;
     const __half *bias;
@@ -66,16 +70,17 @@ struct GemvParams {
     const int *positions;
     int max_pos;   // > 0: positions of outputs addressed by position are brought into [0, max_pos) (the one-pass
                    // kernel; the attention kernel reports them) or dropped with status TLC_DEV_INDEX (split-K finish)
-    int nstages;
+    int nstages, stage_bytes;
     int contig;    // 1: each CTA takes a contiguous range of units, 0: units blockIdx.x, + gridDim.x, ...
-    int l2_hint;   // 1: weight copies carry the evict-first L2 hint
     int pdl_mode;  // 1: let the next kernel be scheduled at once, 2: only when this CTA's last slab is done, 3: after this CTA's own dependency wait
     tlc_dev_status *status;
     uint64_t wait_ns;  // how long a wait may last before the kernel gives up
-    // Split K (ksplit > 1): the K range is cut into ksplit windows of ktiles_win tiles (nblk_pad is
-    // then a window's padded block count); CTA b takes window b % ksplit and writes its f32 share of
-    // every output to partial[window][activation row][ntot outputs] instead of running the epilogue.
-    int ksplit, ktiles_win, ktiles_full, ntot;
+    // The K range: ksplit CTAs of a cluster, windows of ktiles_win tiles; each warp holds tiles_warp of them.
+    int ksplit, ktiles_win, tiles_warp;
+    int batch;  // slabs per cross-warp reduction
+    int round, n_rounds;  // cluster: slabs (of one CTA) per exchange, exchanges of a launch
+    // tlc_gemv_splitk_finish: f32 shares [ksplit][m][ntot] of a split-K GEMM
+    int ntot;
     float *partial;
 };
 
@@ -186,15 +191,6 @@ __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], 
         : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c[0]), "f"(c[1]), "f"(c[2]),
           "f"(c[3]));
-}
-
-// FP8 (e4m3) tensor-core step: 16 rows x 32 k of A, 32 k x 8 columns of B, f32 accumulate in place.
-__device__ __forceinline__ void mma16832_e4m3(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k32.row.col.f32.e4m3.e4m3.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-        "{%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
 // Integer fragments of one block for rows g (w0*) and g+8 (w1*).

@@ -72,7 +72,6 @@ struct tlc_ctx {
     // key splits (a non-portable cluster size) instead of eight.  Off: measured no faster (one
     // rank's share of the 70B-shape decode at TP8, 2048 keys: 3.79 ms per step against 3.73 ms).
     int attn_wide = 0;
-    int l2_hint = 1;         // GEMV weight copies marked evict-first in the L2 (measured: +3 % on the decode step)
     bool host_graph = true;  // decode_host: ids up, the step, results down as ONE graph launch
     bool host_poll = true;   // ... and the host watches the pinned result words instead of a stream sync
     // How long a device-side wait (mbarrier, peer flag) may last before the kernel gives up,
@@ -88,13 +87,6 @@ struct tlc_ctx {
     int gemm_pg = 0;  // producer groups of the GEMM: 0 = two where K is shared out over CTAs, else one; 1 / 2 = forced
     bool gemm_tma = true;  // activation tiles of the GEMM by TMA (false: cp.async loader warps)
     int gemm_tile = 0;  // 0: pick the GEMM tile from the shape; 11, 12, 22: force 128x128, 128x256, 256x256
-    // Option "gemv_f8" / TLC_GEMV_F8=1: one activation row against a Q4_0 weight takes the FP8-limb
-    // form of the fused GEMV (tlc_gemv_kernel.cuh).  Off by default: fewer instructions per block,
-    // but measured slower on a B200 (35.3 vs 30.5 us on a 132 MB weight, 7.1 vs 5.5 us on 6.5 MB).
-    bool gemv_f8 = false;
-    // Option "gemv_splitk" / TLC_GEMV_SPLITK=0: 2..16 activation rows whose fragments crowd the
-    // shared memory take further passes over the weights instead of one pass with K cut into windows.
-    int gemv_splitk = 2;  // 0: off; 1: windows sized for two CTAs per SM first; 2: for one CTA per SM first (measured faster)
     // Option "q6k_resident" / TLC_Q6K_RESIDENT=0: Q6_K tensors are expanded to f16 at upload (what
     // the reference's loader keeps) instead of staying quantized in HBM.
     bool q6k_resident = true;
@@ -268,8 +260,8 @@ int32_t tlc_launch_gemm(tlc_ctx *ctx, const tlc_gemv_args &a);
 size_t tlc_gemm_scratch_bytes(const tlc_ctx *ctx, int m, int64_t k, int64_t n_total);
 // Adds the ksplit f32 shares in partial[ksplit][m][sum of N] and applies the epilogue of `a` (tlc_gemv.cu).
 int32_t tlc_gemv_splitk_finish(tlc_ctx *ctx, const tlc_gemv_args &a, int ksplit, float *partial);
-// Scratch the fused GEMV may need for m rows (split-K partial sums; 0 when it does not split).
-size_t tlc_gemv_scratch_bytes(tlc_ctx *ctx, int type, int64_t k, int m, int64_t n_total);
+// Scratch the RMSNorm in front of a GEMV of 2..16 rows of width k takes.
+size_t tlc_gemv_scratch_bytes(int64_t k);
 
 struct tlc_kvcache;
 int32_t tlc_launch_attention(tlc_ctx *ctx, tlc_kvcache *cache, int layer, const void *q_dev, void *out_dev,

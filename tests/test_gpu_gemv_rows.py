@@ -1,0 +1,48 @@
+"""GPU parity of the fused GEMV for 2 to 16 activation rows (csrc/tlc_gemv_kernel.cuh) where its split of K changes:
+eight and sixteen warps, one to three windows a warp, clusters, and rows and columns that fill nothing."""
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+TIGHT = 1e-3
+
+
+@pytest.mark.parametrize("qtype", [2, 8])
+@pytest.mark.parametrize("n,k", [(16, 32), (17, 1056), (40, 3072), (33, 3104), (50, 4128), (48, 6176), (100, 12320)])
+@pytest.mark.parametrize("m", [2, 8, 9, 16])
+def test_rows_and_windows(dev, ref, qtype, n, k, m):
+    from tensorlogic_b200 import synth
+    from tensorlogic_b200.api import QTensor, linear
+    raw = synth.blocks(qtype, 6, synth.tensor_id(f"gr{n}x{k}"), n, k)
+    x = synth.activations(6, f"gx{m}x{k}", (m, k))
+    got = linear(dev.tensor(x), QTensor.from_blocks(dev, qtype, n, k, raw)).numpy()
+    assert rel_l2(got, ref.linear_q(qtype, raw, n, k, x)) < TIGHT
+
+
+@pytest.mark.parametrize("qtype", [2, 8])
+@pytest.mark.parametrize("k", [2048, 8256])
+@pytest.mark.parametrize("m", [3, 16])
+def test_fused_epilogues(dev, qtype, k, m):
+    """Norm + projections with RoPE, the SiLU.mul pair over more slabs than one round, the residual, against the
+    operations one by one."""
+    from tensorlogic_b200 import synth
+    from tensorlogic_b200.api import (QTensor, add, linear, linear_residual, norm_linear_multi, rms_norm, rope, swiglu,
+                                      swiglu_gate_up)
+    def q(name, rows):
+        return QTensor.synthetic(dev, qtype, rows, k, 8, synth.tensor_id(name), scale_log2=-1 if qtype == 2 else -5)
+    x, nw = dev.tensor(synth.activations(8, f"ex{k}", (m, k))), dev.tensor(synth.norm_weight(8, f"en{k}", k))
+    h = rms_norm(x, nw, 1e-5)
+    ws = [q("eq", 192), q("ek", 64), q("ev", 64)]
+    outs = norm_linear_multi(x, ws, nw, 1e-5, rope_heads=[3, 1, 0], position_offset=11)
+    for y, w, heads in zip(outs, ws, (3, 1, 0)):
+        want = linear(h, w)
+        if heads:
+            want = rope(want.reshape((m, heads, 64)), 11)
+        assert rel_l2(y.numpy().ravel(), want.numpy().ravel()) < TIGHT
+    g, u = q("eg", 1000), q("eu", 1000)
+    assert rel_l2(swiglu_gate_up(x, g, u, nw, 1e-5).numpy(), swiglu(linear(h, g), linear(h, u)).numpy()) < 2e-3
+    r = dev.tensor(synth.activations(8, "er", (m, 1000)))
+    assert rel_l2(linear_residual(h, g, r).numpy(), add(linear(h, g), r).numpy()) < TIGHT
