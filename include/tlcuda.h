@@ -177,6 +177,9 @@ typedef struct tlc_pool_stats {
  * classes 2 KiB..16 MiB, exact size above (buffer_pool.rs:78-101).  Memory is
  * not zeroed on reuse (buffer_pool.rs:222-230). */
 TLC_API int32_t tlc_alloc(tlc_ctx *ctx, size_t bytes, tlc_buf **out);
+/* The same with both results in one call: out[0] = the tlc_buf, out[1] = its device pointer (hosts
+ * for which a foreign call costs more than the allocation). */
+TLC_API int32_t tlc_alloc_ptr(tlc_ctx *ctx, size_t bytes, void **out);
 /* BufferPool::try_return_buffer (buffer_pool.rs:426-499).  Stream-ordered:
  * safe to call while kernels using the buffer are still queued. */
 TLC_API int32_t tlc_free(tlc_buf *buf);

@@ -69,6 +69,7 @@ PROTOTYPES = {
     "tlc_launch_count": (u64, [vp]),
     "tlc_perf_report": (i32, [vp, C.c_char_p, sz, i32, P(sz)]),
     "tlc_alloc": (i32, [vp, sz, P(vp)]),
+    "tlc_alloc_ptr": (i32, [vp, sz, vp]),
     "tlc_free": (i32, [vp]),
     "tlc_buf_ptr": (vp, [vp]),
     "tlc_buf_size": (sz, [vp]),

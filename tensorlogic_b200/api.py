@@ -18,6 +18,7 @@ runs through the C ABI of include/tlcuda.h; nothing here computes on the host.
 from __future__ import annotations
 
 import ctypes as C
+import math
 from typing import Optional, Sequence
 
 import numpy as np
@@ -38,6 +39,8 @@ class Device:
         check(self.lib.tlc_init(ordinal, C.byref(h)))
         self.handle = h
         self.ordinal = ordinal
+        self._slot = (C.c_void_p * 2)()  # tlc_alloc_ptr's results: the handles are used by one thread at a time
+        self._slot_at = C.addressof(self._slot)
 
     def set_option(self, name: str, value: int) -> None:
         """Runtime switch by name (tlc_set_option): "gemm_min_m", "pdl", "pdl_mode"."""
@@ -104,7 +107,7 @@ class Device:
 
     # -- tensors ---------------------------------------------------------
     def empty(self, shape: Sequence[int]) -> "Tensor":
-        return Tensor(self, tuple(int(s) for s in shape))
+        return Tensor(self, tuple(map(int, shape)))
 
     def tensor(self, array) -> "Tensor":
         """Upload a host array as an f16 tensor (Tensor::from_vec_gpu)."""
@@ -120,13 +123,23 @@ class Tensor:
     """f16 tensor on the device (Tensor<f16> with a pooled MetalBuffer upstream)."""
 
     def __init__(self, dev: Device, shape: tuple):
-        self.dev = dev
-        self.shape = tuple(shape)
-        self.size = int(np.prod(self.shape)) if len(self.shape) else 1
-        h = C.c_void_p()
-        check(dev.lib.tlc_alloc(dev.handle, max(self.size, 1) * 2, C.byref(h)))
-        self._buf = h
-        self.ptr = dev.lib.tlc_buf_ptr(h)
+        shape = tuple(shape)
+        self._take(dev, shape, math.prod(shape))
+
+    def _take(self, dev: Device, shape: tuple, size: int) -> None:
+        self.dev, self.shape, self.size = dev, shape, size
+        self._buf = None
+        rc = dev.lib.tlc_alloc_ptr(dev.handle, size * 2 if size else 2, dev._slot_at)
+        if rc:
+            check(rc)
+        self._buf, self.ptr = dev._slot
+
+    @classmethod
+    def _new(cls, dev: Device, shape: tuple, size: int) -> "Tensor":
+        """What the builtins return: shape and size are known to be right."""
+        t = cls.__new__(cls)
+        t._take(dev, shape, size)
+        return t
 
     def __del__(self):
         try:
@@ -148,8 +161,8 @@ class Tensor:
         return out
 
     def reshape(self, shape: Sequence[int]) -> "Tensor":
-        shape = tuple(int(s) for s in shape)
-        if int(np.prod(shape)) != self.size:
+        shape = tuple(map(int, shape))
+        if math.prod(shape) != self.size:
             raise TensorError(_lib.ERR_SHAPE_MISMATCH, f"expected {self.size} elements, got shape {shape}")
         v = Tensor.__new__(Tensor)
         v.dev, v.shape, v.size, v.ptr = self.dev, shape, self.size, self.ptr
@@ -237,8 +250,10 @@ def linear(x: Tensor, weight: QTensor, bias: Optional[Tensor] = None) -> Tensor:
     if bias is not None and not isinstance(bias, Tensor):
         raise TypeError("linear() bias must be f16 tensor")
     m, k = _rows_cols(x)
-    y = x.dev.empty((m, weight.shape[0]))
-    check(x.dev.lib.tlc_linear(x.dev.handle, weight.handle, x.ptr, m, k, y.ptr, bias.ptr if bias is not None else None))
+    y = Tensor._new(x.dev, (m, weight.shape[0]), m * weight.shape[0])
+    rc = x.dev.lib.tlc_linear(x.dev.handle, weight.handle, x.ptr, m, k, y.ptr, bias.ptr if bias is not None else None)
+    if rc:
+        check(rc)
     return y
 
 
@@ -246,8 +261,10 @@ def rms_norm(x: Tensor, weight: Tensor, eps: float = 1e-6) -> Tensor:
     d = weight.size
     if x.shape[-1] != d:
         raise TensorError(_lib.ERR_SHAPE_MISMATCH, f"rms_norm: last dim {x.shape[-1]} != weight {d}")
-    y = x.dev.empty(x.shape)
-    check(x.dev.lib.tlc_rms_norm(x.dev.handle, x.ptr, weight.ptr, y.ptr, x.size // d, d, eps))
+    y = Tensor._new(x.dev, x.shape, x.size)
+    rc = x.dev.lib.tlc_rms_norm(x.dev.handle, x.ptr, weight.ptr, y.ptr, x.size // d, d, eps)
+    if rc:
+        check(rc)
     return y
 
 
@@ -257,7 +274,7 @@ def rope(x: Tensor, position_offset: int = 0, positions: Optional[np.ndarray] = 
         raise TensorError(_lib.ERR_INVALID_OPERATION, "RoPE requires at least 3D tensor [seq, heads, head_dim]")
     heads, d = x.shape[-2], x.shape[-1]
     seq = x.size // (heads * d)
-    y = x.dev.empty(x.shape)
+    y = Tensor._new(x.dev, x.shape, x.size)
     pos_t = None
     pos_ptr = None
     if positions is not None:
@@ -266,7 +283,9 @@ def rope(x: Tensor, position_offset: int = 0, positions: Optional[np.ndarray] = 
             raise TensorError(_lib.ERR_SHAPE_MISMATCH, f"rope: {pos.size} positions for {seq} rows")
         pos_t = _upload_i32(x.dev, pos)
         pos_ptr = pos_t.ptr
-    check(x.dev.lib.tlc_rope(x.dev.handle, x.ptr, y.ptr, seq, heads, d, position_offset, base, pos_ptr))
+    rc = x.dev.lib.tlc_rope(x.dev.handle, x.ptr, y.ptr, seq, heads, d, position_offset, base, pos_ptr)
+    if rc:
+        check(rc)
     return y
 
 
@@ -289,9 +308,11 @@ def rope_table(x: Tensor, cos: Tensor, sin: Tensor) -> Tensor:
     if cos.shape != sin.shape or cos.shape[1] not in (d, d // 2):
         raise TensorError(_lib.ERR_INVALID_OPERATION,
                           f"cos/sin last dim must be head_dim = {d}, got cos: {cos.shape[1]}, sin: {sin.shape[1]}")
-    y = x.dev.empty(x.shape)
-    check(x.dev.lib.tlc_rope_table(x.dev.handle, x.ptr, cos.ptr, sin.ptr, y.ptr, seq, heads, d, cos.shape[0],
-                                   cos.shape[1]))
+    y = Tensor._new(x.dev, x.shape, x.size)
+    rc = x.dev.lib.tlc_rope_table(x.dev.handle, x.ptr, cos.ptr, sin.ptr, y.ptr, seq, heads, d, cos.shape[0],
+                                   cos.shape[1])
+    if rc:
+        check(rc)
     return y
 
 
@@ -301,20 +322,24 @@ def matmul(a: Tensor, b: Tensor) -> Tensor:
     if a.ndim != 2 or b.ndim != 2:
         raise TensorError(_lib.ERR_INVALID_OPERATION, "matmul requires 2D tensors")
     y = a.dev.empty((a.shape[0], b.shape[1]))
-    check(a.dev.lib.tlc_matmul(a.dev.handle, a.ptr, b.ptr, y.ptr, a.shape[0], a.shape[1], b.shape[0], b.shape[1]))
+    rc = a.dev.lib.tlc_matmul(a.dev.handle, a.ptr, b.ptr, y.ptr, a.shape[0], a.shape[1], b.shape[0], b.shape[1])
+    if rc:
+        check(rc)
     return y
 
 
 def sigmoid(x: Tensor) -> Tensor:
-    y = x.dev.empty(x.shape)
-    check(x.dev.lib.tlc_sigmoid(x.dev.handle, x.ptr, y.ptr, x.size))
+    y = Tensor._new(x.dev, x.shape, x.size)
+    rc = x.dev.lib.tlc_sigmoid(x.dev.handle, x.ptr, y.ptr, x.size)
+    if rc:
+        check(rc)
     return y
 
 
 def _binary(fn_name: str, a: Tensor, b: Tensor) -> Tensor:
     if a.shape != b.shape:
         raise TensorError(_lib.ERR_SHAPE_MISMATCH, f"expected {list(a.shape)}, got {list(b.shape)}")
-    y = a.dev.empty(a.shape)
+    y = Tensor._new(a.dev, a.shape, a.size)
     check(getattr(a.dev.lib, fn_name)(a.dev.handle, a.ptr, b.ptr, y.ptr, a.size))
     return y
 
@@ -340,8 +365,10 @@ def swiglu(gate: Tensor, up: Tensor) -> Tensor:
 def softmax(x: Tensor, dim: int = -1) -> Tensor:
     del dim  # the reference builtin always normalises the last axis
     last = x.shape[-1]
-    y = x.dev.empty(x.shape)
-    check(x.dev.lib.tlc_softmax(x.dev.handle, x.ptr, y.ptr, x.size // last, last))
+    y = Tensor._new(x.dev, x.shape, x.size)
+    rc = x.dev.lib.tlc_softmax(x.dev.handle, x.ptr, y.ptr, x.size // last, last)
+    if rc:
+        check(rc)
     return y
 
 
@@ -372,8 +399,10 @@ def embedding(table: Tensor, ids) -> Tensor:
     ids = np.ascontiguousarray(np.atleast_1d(ids), dtype=np.int32)
     vocab, d = table.shape
     y = table.dev.empty((ids.size, d))
-    check(table.dev.lib.tlc_embedding(table.dev.handle, table.ptr, vocab, d, ids.ctypes.data_as(C.POINTER(C.c_int32)),
-                                      ids.size, y.ptr))
+    rc = table.dev.lib.tlc_embedding(table.dev.handle, table.ptr, vocab, d, ids.ctypes.data_as(C.POINTER(C.c_int32)),
+                                      ids.size, y.ptr)
+    if rc:
+        check(rc)
     return y
 
 
@@ -472,8 +501,8 @@ class KVCache:
         if q.size % (n_heads * D * batch):
             raise TensorError(_lib.ERR_SHAPE_MISMATCH, f"attention: q has {q.size} elements")
         nq = q.size // (n_heads * D * batch)
-        out = self.dev.empty(q.shape)
-        scale = float(1.0 / np.sqrt(D)) if scale is None else scale
+        out = Tensor._new(self.dev, q.shape, q.size)
+        scale = 1.0 / math.sqrt(D) if scale is None else scale
         pos_t, max_keys = None, q_pos0 + nq
         if positions is not None:
             pos = np.ascontiguousarray(positions, dtype=np.int32)
@@ -486,6 +515,6 @@ class KVCache:
 
 def linear_residual(x: Tensor, weight: QTensor, residual: Tensor) -> Tensor:
     m, _ = _rows_cols(x)
-    y = x.dev.empty((m, weight.shape[0]))
+    y = Tensor._new(x.dev, (m, weight.shape[0]), m * weight.shape[0])
     check(x.dev.lib.tlc_linear_residual(x.dev.handle, weight.handle, x.ptr, m, residual.ptr, y.ptr))
     return y

@@ -642,9 +642,10 @@ static constexpr size_t attention_smem_limit(int D) {
     return (size_t)4 * kTileKeys * (D + 8) * sizeof(__half) + 128 + (size_t)16 * 16 * (D + 2) * sizeof(float);
 }
 
-__global__ void kv_append_kernel(const __half *__restrict__ k, const __half *__restrict__ v,
-                                 __half *__restrict__ kc, __half *__restrict__ vc, int m, int row_elems,
-                                 int tmax, int pos_offset, const int *__restrict__ positions, int batched) {
+template <typename V>
+__global__ void kv_append_kernel(const V *__restrict__ k, const V *__restrict__ v, V *__restrict__ kc, V *__restrict__ vc, int m,
+                                 int row_elems, int tmax, int pos_offset, const int *__restrict__ positions, int batched) {
+    tlc_pdl_after_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)m * row_elems) return;
     const int r = (int)(i / row_elems), c = (int)(i % row_elems);
@@ -937,11 +938,21 @@ extern "C" int32_t tlc_kvcache_append(tlc_ctx *ctx, tlc_kvcache *cache, int32_t 
                     "Index out of bounds: index %d, size %d", pos_offset + m, cache->max_seq);
     if (m <= 0) return TLC_OK;
     const int row_elems = cache->n_kv_heads * cache->head_dim;
-    const size_t total = (size_t)m * row_elems;
-    kv_append_kernel<<<(unsigned)((total + 255) / 256), 256, 0, ctx->stream>>>(
-        static_cast<const __half *>(k_dev), static_cast<const __half *>(v_dev),
-        cache->k + (size_t)layer * cache->layer_stride, cache->v + (size_t)layer * cache->layer_stride, m, row_elems,
-        cache->max_seq, pos_offset, positions_dev, batched ? 1 : 0);
+    __half *kc = cache->k + (size_t)layer * cache->layer_stride, *vc = cache->v + (size_t)layer * cache->layer_stride;
+    const bool vec = (((uintptr_t)k_dev | (uintptr_t)v_dev) & 15) == 0;  // a cache row is a multiple of eight values
+    const int per = vec ? row_elems / 8 : row_elems;
+    const dim3 grid((unsigned)(((size_t)m * per + 255) / 256)), block(256);
+    const cudaError_t le =
+        vec ? tlc_launch_pdl(ctx, kv_append_kernel<uint4>, grid, block, 0, static_cast<const uint4 *>(k_dev),
+                             static_cast<const uint4 *>(v_dev), reinterpret_cast<uint4 *>(kc), reinterpret_cast<uint4 *>(vc), m, per,
+                             cache->max_seq, pos_offset, positions_dev, batched ? 1 : 0)
+            : tlc_launch_pdl(ctx, kv_append_kernel<__half>, grid, block, 0, static_cast<const __half *>(k_dev),
+                             static_cast<const __half *>(v_dev), kc, vc, m, per, cache->max_seq, pos_offset, positions_dev,
+                             batched ? 1 : 0);
+    if (le != cudaSuccess) {
+        cudaGetLastError();
+        return tlc_fail(TLC_ERR_CUDA, "kvcache_append launch failed: %s", cudaGetErrorString(le));
+    }
     TLC_CHECK_LAUNCH(ctx);
     return TLC_OK;
 }

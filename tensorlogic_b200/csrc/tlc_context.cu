@@ -330,7 +330,6 @@ extern "C" int32_t tlc_alloc(tlc_ctx *ctx, size_t bytes, tlc_buf **out) {
     if (it != ctx->pool.idle.end() && !it->second.empty()) {
         p = it->second.back();
         it->second.pop_back();
-        if (it->second.empty()) ctx->pool.idle.erase(it);
         ctx->pool.stats.reuse_count++;
     } else {
         cudaError_t e = cudaMalloc(&p, cls);
@@ -371,6 +370,16 @@ extern "C" int32_t tlc_free(tlc_buf *buf) {
         if (vec.empty()) ctx->pool.idle.erase(buf->class_bytes);
     }
     delete buf;
+    return TLC_OK;
+}
+
+// The same in one call: out[0] the buffer, out[1] its device pointer.
+extern "C" int32_t tlc_alloc_ptr(tlc_ctx *ctx, size_t bytes, void **out) {
+    TLC_REQUIRE(out != nullptr, TLC_ERR_INVALID_OPERATION, "tlc_alloc_ptr: null out pointer");
+    tlc_buf *b = nullptr;
+    if (int32_t rc = tlc_alloc(ctx, bytes, &b)) return rc;
+    out[0] = b;
+    out[1] = b->ptr;
     return TLC_OK;
 }
 

@@ -201,6 +201,12 @@ __device__ __forceinline__ uint64_t tlc_globaltimer_ns() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
+// Device side of the above for the short kernels: wait for the predecessor's results, then let the successor be
+// scheduled (never two grids ahead).  No-ops for a kernel launched the plain way.
+__device__ __forceinline__ void tlc_pdl_after_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 // Device side of the above: let the successor be scheduled, then wait for the
 // predecessor's results.  Both are no-ops for a kernel launched the plain way.
 __device__ __forceinline__ void tlc_pdl_prologue() {

@@ -15,6 +15,7 @@ namespace {
 // (src/ops/normalization.rs:199-248): one CTA per row.
 __global__ void rms_norm_kernel(const __half *__restrict__ x, const __half *__restrict__ w,
                                 __half *__restrict__ y, int d, float eps) {
+    tlc_pdl_after_wait();
     __shared__ float warp_sums[32];
     __shared__ float inv_s;
     const __half *xr = x + (size_t)blockIdx.x * d;
@@ -72,6 +73,7 @@ __global__ void rms_norm_kernel(const __half *__restrict__ x, const __half *__re
 // rope_f16 (shaders/unified.metal:2355-2417): one thread per pair.
 __global__ void rope_kernel(const __half *__restrict__ x, __half *__restrict__ y, int seq, int heads, int d,
                             int pos_offset, float base, const int *__restrict__ positions) {
+    tlc_pdl_after_wait();
     const int half_d = d >> 1;
     const size_t total = (size_t)seq * heads * half_d;
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -97,6 +99,7 @@ __global__ void rope_kernel(const __half *__restrict__ x, __half *__restrict__ y
 __global__ void rope_table_kernel(const __half *__restrict__ x, const __half *__restrict__ cos_t,
                                   const __half *__restrict__ sin_t, __half *__restrict__ y, int seq, int heads, int d,
                                   int pitch) {
+    tlc_pdl_after_wait();
     const int half_d = d >> 1;
     const size_t total = (size_t)seq * heads * half_d;
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -112,34 +115,42 @@ __global__ void rope_table_kernel(const __half *__restrict__ x, const __half *__
 }
 
 // sigmoid: f32 math, RNE to f16 (Tensor::sigmoid_cpu, src/ops/activations.rs:252-266).
-__global__ void sigmoid_kernel(const __half *__restrict__ x, __half *__restrict__ y, size_t n) {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) y[i] = __float2half_rn(1.0f / (1.0f + expf(-__half2float(x[i]))));
+// One operation per element; eight elements a thread (16-byte accesses) where alignment allows.
+struct OpSigmoid {
+    static __device__ __forceinline__ __half run(__half x, __half) { return __float2half_rn(1.0f / (1.0f + expf(-__half2float(x)))); }
+};
+struct OpMul {
+    static __device__ __forceinline__ __half run(__half a, __half b) { return __hmul(a, b); }
+};
+struct OpAdd {
+    static __device__ __forceinline__ __half run(__half a, __half b) { return __hadd(a, b); }
+};
+struct OpSwiglu {  // silu(g) * u with the three f16 roundings of sigmoid, mul, mul
+    static __device__ __forceinline__ __half run(__half g, __half u) { return __hmul(__hmul(g, OpSigmoid::run(g, g)), u); }
+};
+template <class OP, bool TWO>
+__global__ void __launch_bounds__(256) elementwise_kernel(const __half *__restrict__ a, const __half *__restrict__ b,
+                                                          __half *__restrict__ y, size_t n, int vec) {
+    tlc_pdl_after_wait();
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (!vec) {
+        if (i < n) y[i] = OP::run(a[i], TWO ? b[i] : a[i]);
+        return;
+    }
+    if (i * 8 >= n) return;
+    const uint4 av = reinterpret_cast<const uint4 *>(a)[i], bv = TWO ? reinterpret_cast<const uint4 *>(b)[i] : av;
+    const __half *ah = reinterpret_cast<const __half *>(&av), *bh = reinterpret_cast<const __half *>(&bv);
+    __align__(16) __half o[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) o[j] = OP::run(ah[j], bh[j]);
+    reinterpret_cast<uint4 *>(y)[i] = *reinterpret_cast<const uint4 *>(o);
 }
-__global__ void mul_kernel(const __half *__restrict__ a, const __half *__restrict__ b, __half *__restrict__ y,
-                           size_t n) {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) y[i] = __hmul(a[i], b[i]);
-}
-__global__ void add_kernel(const __half *__restrict__ a, const __half *__restrict__ b, __half *__restrict__ y,
-                           size_t n) {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) y[i] = __hadd(a[i], b[i]);
-}
-__global__ void swiglu_kernel(const __half *__restrict__ g, const __half *__restrict__ u,
-                              __half *__restrict__ y, size_t n) {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const __half gv = g[i];
-    const __half s = __float2half_rn(1.0f / (1.0f + expf(-__half2float(gv))));
-    y[i] = __hmul(__hmul(gv, s), u[i]);
-}
-
 // softmax over the last dim, one warp per row; arithmetic of
 // softmax_simple_f16 (shaders/unified.metal:2150-2200): finite-only f32 max and
 // sum, exponentials rounded to f16 before the divide, uniform row when the sum
 // degenerates.
 __global__ void softmax_kernel(const __half *__restrict__ x, __half *__restrict__ y, int rows, int last) {
+    tlc_pdl_after_wait();
     const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (row >= rows) return;
@@ -175,6 +186,7 @@ __global__ void softmax_kernel(const __half *__restrict__ x, __half *__restrict_
 // embedding_lookup_f16 (shaders/unified.metal:658-675): 16-byte vector gather.
 __global__ void embedding_kernel(const __half *__restrict__ table, const int *__restrict__ ids, int d,
                                  int m, __half *__restrict__ y) {
+    tlc_pdl_after_wait();
     const int vec_per_row = d >> 3;
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)m * vec_per_row) return;
@@ -184,26 +196,23 @@ __global__ void embedding_kernel(const __half *__restrict__ table, const int *__
 }
 __global__ void embedding_scalar_kernel(const __half *__restrict__ table, const int *__restrict__ ids, int d,
                                         int m, __half *__restrict__ y) {
+    tlc_pdl_after_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)m * d) return;
     const int r = (int)(i / d), c = (int)(i % d);
     y[i] = table[(size_t)ids[r] * d + c];
 }
 
-// Eight elements per thread (16-byte accesses) for the large element-wise passes of a prefill.
-__global__ void swiglu_vec8_kernel(const uint4 *__restrict__ g, const uint4 *__restrict__ u, uint4 *__restrict__ y,
-                                   size_t n8) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n8) return;
-    const uint4 gv = g[i], uv = u[i];
-    const __half *gh = reinterpret_cast<const __half *>(&gv), *uh = reinterpret_cast<const __half *>(&uv);
-    __align__(16) __half o[8];
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-        const __half s = __float2half_rn(1.0f / (1.0f + expf(-__half2float(gh[j]))));
-        o[j] = __hmul(__hmul(gh[j], s), uh[j]);
+// Launch on the context's stream with programmatic dependent launch.
+template <typename... KArgs, typename... Args>
+int32_t launch_op(tlc_ctx *ctx, void (*kernel)(KArgs...), unsigned grid, unsigned block, Args &&...args) {
+    const cudaError_t le = tlc_launch_pdl(ctx, kernel, dim3(grid), dim3(block), 0, args...);
+    if (le != cudaSuccess) {
+        cudaGetLastError();
+        return tlc_fail(TLC_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(le));
     }
-    y[i] = *reinterpret_cast<const uint4 *>(o);
+    TLC_CHECK_LAUNCH(ctx);
+    return TLC_OK;
 }
 
 inline unsigned blocks_for(size_t n, int threads) { return (unsigned)((n + threads - 1) / threads); }
@@ -217,11 +226,9 @@ extern "C" int32_t tlc_rms_norm(tlc_ctx *ctx, const void *x_dev, const void *w_d
     TLC_REQUIRE(x_dev && w_dev && y_dev, TLC_ERR_INVALID_OPERATION, "rms_norm: null pointer");
     TLC_REQUIRE(rows >= 0 && d > 0, TLC_ERR_INVALID_DIMENSION, "rms_norm: bad shape [%d, %d]", rows, d);
     if (rows == 0) return TLC_OK;
-    rms_norm_kernel<<<rows, 256, 0, ctx->stream>>>(static_cast<const __half *>(x_dev),
+    return launch_op(ctx, rms_norm_kernel, rows, 256, static_cast<const __half *>(x_dev),
                                                    static_cast<const __half *>(w_dev),
                                                    static_cast<__half *>(y_dev), d, eps);
-    TLC_CHECK_LAUNCH(ctx);
-    return TLC_OK;
 }
 
 extern "C" int32_t tlc_rope(tlc_ctx *ctx, const void *x_dev, void *y_dev, int32_t seq, int32_t heads,
@@ -234,11 +241,9 @@ extern "C" int32_t tlc_rope(tlc_ctx *ctx, const void *x_dev, void *y_dev, int32_
     TLC_REQUIRE(seq >= 0 && heads > 0, TLC_ERR_INVALID_DIMENSION, "rope: bad shape [%d, %d, %d]", seq, heads, d);
     if (seq == 0) return TLC_OK;
     const size_t total = (size_t)seq * heads * (d / 2);
-    rope_kernel<<<blocks_for(total, 256), 256, 0, ctx->stream>>>(
+    return launch_op(ctx, rope_kernel, blocks_for(total, 256), 256, 
         static_cast<const __half *>(x_dev), static_cast<__half *>(y_dev), seq, heads, d, pos_offset, (float)base,
         positions_dev);
-    TLC_CHECK_LAUNCH(ctx);
-    return TLC_OK;
 }
 
 // rope(x, cos, sin): the arm of the rope builtin that takes precomputed tables
@@ -265,11 +270,9 @@ extern "C" int32_t tlc_rope_table(tlc_ctx *ctx, const void *x_dev, const void *c
                 "cos/sin first dim must be >= seq_len = %d, got cos: %d, sin: %d", seq, table_rows, table_rows);
     if (seq == 0) return TLC_OK;
     const size_t total = (size_t)seq * heads * (d / 2);
-    rope_table_kernel<<<blocks_for(total, 256), 256, 0, ctx->stream>>>(
+    return launch_op(ctx, rope_table_kernel, blocks_for(total, 256), 256, 
         static_cast<const __half *>(x_dev), static_cast<const __half *>(cos_dev), static_cast<const __half *>(sin_dev),
         static_cast<__half *>(y_dev), seq, heads, d, pitch);
-    TLC_CHECK_LAUNCH(ctx);
-    return TLC_OK;
 }
 
 // matmul(a, b): a [m, k] . b [k2, n] -> y [m, n], all f16 on the device.  Shape rule and message
@@ -287,46 +290,27 @@ extern "C" int32_t tlc_matmul(tlc_ctx *ctx, const void *a_dev, const void *b_dev
     return TLC_OK;
 }
 
-#define TLC_ELEMENTWISE_1(name, kernel)                                                                  \
-    extern "C" int32_t name(tlc_ctx *ctx, const void *x_dev, void *y_dev, size_t n) {                    \
-        if (int32_t rc = tlc_enter(ctx)) return rc;                                                      \
-        TLC_REQUIRE(x_dev && y_dev, TLC_ERR_INVALID_OPERATION, #name ": null pointer");                  \
-        if (n == 0) return TLC_OK;                                                                       \
-        tlc_perf_scope perf(ctx, "%s(n=%zu)", #name + 4, n);                                             \
-        kernel<<<blocks_for(n, 256), 256, 0, ctx->stream>>>(static_cast<const __half *>(x_dev),          \
-                                                            static_cast<__half *>(y_dev), n);            \
-        TLC_CHECK_LAUNCH(ctx);                                                                           \
-        return TLC_OK;                                                                                   \
-    }
-#define TLC_ELEMENTWISE_2(name, kernel)                                                                  \
-    extern "C" int32_t name(tlc_ctx *ctx, const void *a_dev, const void *b_dev, void *y_dev, size_t n) { \
-        if (int32_t rc = tlc_enter(ctx)) return rc;                                                      \
-        TLC_REQUIRE(a_dev && b_dev && y_dev, TLC_ERR_INVALID_OPERATION, #name ": null pointer");         \
-        if (n == 0) return TLC_OK;                                                                       \
-        tlc_perf_scope perf(ctx, "%s(n=%zu)", #name + 4, n);                                             \
-        kernel<<<blocks_for(n, 256), 256, 0, ctx->stream>>>(static_cast<const __half *>(a_dev),          \
-                                                            static_cast<const __half *>(b_dev),          \
-                                                            static_cast<__half *>(y_dev), n);            \
-        TLC_CHECK_LAUNCH(ctx);                                                                           \
-        return TLC_OK;                                                                                   \
-    }
-
-TLC_ELEMENTWISE_1(tlc_sigmoid, sigmoid_kernel)
-TLC_ELEMENTWISE_2(tlc_mul, mul_kernel)
-TLC_ELEMENTWISE_2(tlc_add, add_kernel)
-extern "C" int32_t tlc_swiglu(tlc_ctx *ctx, const void *a_dev, const void *b_dev, void *y_dev, size_t n) {
+template <class OP, bool TWO>
+static int32_t elementwise(tlc_ctx *ctx, const char *name, const void *a, const void *b, void *y, size_t n) {
     if (int32_t rc = tlc_enter(ctx)) return rc;
-    tlc_perf_scope perf(ctx, "swiglu(n=%zu)", n);
-    TLC_REQUIRE(a_dev && b_dev && y_dev, TLC_ERR_INVALID_OPERATION, "tlc_swiglu: null pointer");
+    TLC_REQUIRE(a && (b || !TWO) && y, TLC_ERR_INVALID_OPERATION, "tlc_%s: null pointer", name);
     if (n == 0) return TLC_OK;
-    if (n % 8 == 0 && (((uintptr_t)a_dev | (uintptr_t)b_dev | (uintptr_t)y_dev) & 15) == 0)
-        swiglu_vec8_kernel<<<blocks_for(n / 8, 256), 256, 0, ctx->stream>>>(
-            static_cast<const uint4 *>(a_dev), static_cast<const uint4 *>(b_dev), static_cast<uint4 *>(y_dev), n / 8);
-    else
-        swiglu_kernel<<<blocks_for(n, 256), 256, 0, ctx->stream>>>(
-            static_cast<const __half *>(a_dev), static_cast<const __half *>(b_dev), static_cast<__half *>(y_dev), n);
-    TLC_CHECK_LAUNCH(ctx);
-    return TLC_OK;
+    tlc_perf_scope perf(ctx, "%s(n=%zu)", name, n);
+    const int vec = n % 8 == 0 && (((uintptr_t)a | (uintptr_t)(TWO ? b : nullptr) | (uintptr_t)y) & 15) == 0 ? 1 : 0;
+    return launch_op(ctx, elementwise_kernel<OP, TWO>, blocks_for(vec ? n / 8 : n, 256), 256, static_cast<const __half *>(a),
+                     static_cast<const __half *>(b), static_cast<__half *>(y), n, vec);
+}
+extern "C" int32_t tlc_sigmoid(tlc_ctx *ctx, const void *x_dev, void *y_dev, size_t n) {
+    return elementwise<OpSigmoid, false>(ctx, "sigmoid", x_dev, nullptr, y_dev, n);
+}
+extern "C" int32_t tlc_mul(tlc_ctx *ctx, const void *a_dev, const void *b_dev, void *y_dev, size_t n) {
+    return elementwise<OpMul, true>(ctx, "mul", a_dev, b_dev, y_dev, n);
+}
+extern "C" int32_t tlc_add(tlc_ctx *ctx, const void *a_dev, const void *b_dev, void *y_dev, size_t n) {
+    return elementwise<OpAdd, true>(ctx, "add", a_dev, b_dev, y_dev, n);
+}
+extern "C" int32_t tlc_swiglu(tlc_ctx *ctx, const void *a_dev, const void *b_dev, void *y_dev, size_t n) {
+    return elementwise<OpSwiglu, true>(ctx, "swiglu", a_dev, b_dev, y_dev, n);
 }
 
 extern "C" int32_t tlc_softmax(tlc_ctx *ctx, const void *x_dev, void *y_dev, int32_t rows, int32_t last_dim) {
@@ -335,10 +319,8 @@ extern "C" int32_t tlc_softmax(tlc_ctx *ctx, const void *x_dev, void *y_dev, int
     TLC_REQUIRE(x_dev && y_dev, TLC_ERR_INVALID_OPERATION, "softmax: null pointer");
     TLC_REQUIRE(rows >= 0 && last_dim > 0, TLC_ERR_INVALID_DIMENSION, "softmax: bad shape [%d, %d]", rows, last_dim);
     if (rows == 0) return TLC_OK;
-    softmax_kernel<<<blocks_for((size_t)rows * 32, 256), 256, 0, ctx->stream>>>(
+    return launch_op(ctx, softmax_kernel, blocks_for((size_t)rows * 32, 256), 256, 
         static_cast<const __half *>(x_dev), static_cast<__half *>(y_dev), rows, last_dim);
-    TLC_CHECK_LAUNCH(ctx);
-    return TLC_OK;
 }
 
 extern "C" int32_t tlc_embedding(tlc_ctx *ctx, const void *table_dev, int32_t vocab, int32_t d,
@@ -361,19 +343,17 @@ extern "C" int32_t tlc_embedding(tlc_ctx *ctx, const void *table_dev, int32_t vo
         return tlc_fail(TLC_ERR_CUDA, "embedding: id upload failed: %s", cudaGetErrorString(e));
     }
     const bool vec = d % 8 == 0 && ((uintptr_t)table_dev % 16 == 0) && ((uintptr_t)y_dev % 16 == 0);
+    int32_t rc;
     if (vec)
-        embedding_kernel<<<blocks_for((size_t)m * (d / 8), 256), 256, 0, ctx->stream>>>(
+        rc = launch_op(ctx, embedding_kernel, blocks_for((size_t)m * (d / 8), 256), 256, 
             static_cast<const __half *>(table_dev), static_cast<const int *>(ids->ptr), d, m,
             static_cast<__half *>(y_dev));
     else
-        embedding_scalar_kernel<<<blocks_for((size_t)m * d, 256), 256, 0, ctx->stream>>>(
+        rc = launch_op(ctx, embedding_scalar_kernel, blocks_for((size_t)m * d, 256), 256, 
             static_cast<const __half *>(table_dev), static_cast<const int *>(ids->ptr), d, m,
             static_cast<__half *>(y_dev));
-    ctx->launches++;
-    e = cudaGetLastError();
     tlc_free(ids);  // stream-ordered: the gather above is already queued
-    if (e != cudaSuccess) return tlc_fail(TLC_ERR_CUDA, "embedding launch failed: %s", cudaGetErrorString(e));
-    return TLC_OK;
+    return rc;
 }
 
 // ---- linear family -----------------------------------------------------------
