@@ -32,6 +32,9 @@
 // 43.8 -> 24 us; norm + 2560 x 2048 at 5 / 16 rows 9.5 -> 6.4 / 19.3 -> 8.1 us; 28672 x 8192 at 8 rows 42.8 -> 35.9 us.
 #include <cuda_fp16.h>
 
+#include <cstring>
+
+#include "tlc_gemm_kernel.cuh"
 #include "tlc_gemm_wt.h"
 #include "tlc_gemv_kernel.cuh"
 #include "tlc_gemv_row1.cuh"
@@ -105,88 +108,6 @@ __global__ void __launch_bounds__(256) linear_f16_kernel(const uint8_t *__restri
         if (bias) h = __hadd(h, bias[row]);
         if (residual) h = __hadd(h, residual[row]);
         y[row] = h;
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Q6_K weights kept quantized (stock Q4_0 GGUF files store output.weight, the largest
-// linear of a decode step, as Q6_K: GGUFLoader::dequantize_q6_k, src/model/formats/gguf.rs:
-// 128-218).  One warp per output row over rows of 224-byte padded super-blocks (tlc_qtensor.cu);
-// sixteen lanes share a super-block: lane (half h, quarter q) takes l = 4q .. 4q+3 of half h,
-// i.e. one 32-bit word each of ql[l], ql[l+32], qh[l] and from them the sixteen weights
-// l, l+32, l+64, l+96.  The four 6-bit values of a word are put together with byte-wise integer
-// operations, turned into exact f16 (1024 + q, minus 1056) and accumulated in f32 against up to
-// MR activation rows held in shared memory; the group's scale d * sc multiplies the group's sum.
-// HBM-bound on 0.875 bytes per weight (the f16 copy the reference keeps costs 2).
-// ---------------------------------------------------------------------------
-template <int MR>
-__global__ void __launch_bounds__(256) linear_q6k_kernel(const uint8_t *__restrict__ w, size_t pitch, int n_rows, int k,
-                                                         const __half *__restrict__ x, int m, __half *__restrict__ y,
-                                                         const __half *__restrict__ bias,
-                                                         const __half *__restrict__ residual) {
-    extern __shared__ __align__(16) uint8_t q6_smem[];
-    __half *xs = reinterpret_cast<__half *>(q6_smem);  // [m][k]
-    tlc_pdl_prologue();
-    for (int i = threadIdx.x * 8; i < m * k; i += blockDim.x * 8)
-        *reinterpret_cast<uint4 *>(xs + i) = *reinterpret_cast<const uint4 *>(x + i);
-    __syncthreads();
-    const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (row >= n_rows) return;
-    const int sub = lane & 15, h = sub >> 3, q = sub & 7, is = q >> 2;
-    const int n_sb = k >> 8;
-    float acc[MR];
-#pragma unroll
-    for (int i = 0; i < MR; i++) acc[i] = 0.f;
-    const __half2 bias1056 = __float2half2_rn(1056.0f);  // 1024 (the magic exponent) + 32 (the offset of q)
-    for (int sb = lane >> 4; sb < n_sb; sb += 2) {
-        const uint8_t *blk = w + (size_t)row * pitch + (size_t)sb * 224;
-        const uint32_t qa = *reinterpret_cast<const uint32_t *>(blk + 64 * h + 4 * q);
-        const uint32_t qb = *reinterpret_cast<const uint32_t *>(blk + 64 * h + 32 + 4 * q);
-        const uint32_t qh = *reinterpret_cast<const uint32_t *>(blk + 128 + 32 * h + 4 * q);
-        const uint2 scw = *reinterpret_cast<const uint2 *>(blk + 192 + 8 * h);
-        const float d = __half2float(*reinterpret_cast<const __half *>(blk + 208));
-        // group j (elements l + 32 j): four 6-bit values in the four bytes of a word
-        uint32_t qv[4];
-        qv[0] = (qa & 0x0F0F0F0Fu) | ((qh & 0x03030303u) << 4);
-        qv[1] = (qb & 0x0F0F0F0Fu) | (((qh >> 2) & 0x03030303u) << 4);
-        qv[2] = ((qa >> 4) & 0x0F0F0F0Fu) | (((qh >> 4) & 0x03030303u) << 4);
-        qv[3] = ((qb >> 4) & 0x0F0F0F0Fu) | (((qh >> 6) & 0x03030303u) << 4);
-        const uint32_t scs[2] = {scw.x, scw.y};
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            // bytes (b0, b1 | b2, b3) -> f16 pairs 1024 + b, then - 1056: exactly q - 32
-            const uint32_t p01 = __byte_perm(qv[j], 0x64646464u, 0x4140), p23 = __byte_perm(qv[j], 0x64646464u, 0x4342);
-            const float2 w01 = __half22float2(__hsub2(*reinterpret_cast<const __half2 *>(&p01), bias1056));
-            const float2 w23 = __half22float2(__hsub2(*reinterpret_cast<const __half2 *>(&p23), bias1056));
-            const int sidx = is + 2 * j;  // scale of this group: byte sidx of the half's eight
-            const float scale = d * (float)(int8_t)((scs[sidx >> 2] >> (8 * (sidx & 3))) & 0xFF);
-            const int e0 = sb * 256 + 128 * h + 4 * q + 32 * j;
-#pragma unroll
-            for (int i = 0; i < MR; i++) {
-                if (i < m) {
-                    const uint2 xr = *reinterpret_cast<const uint2 *>(xs + (size_t)i * k + e0);
-                    const float2 x01 = __half22float2(*reinterpret_cast<const __half2 *>(&xr.x));
-                    const float2 x23 = __half22float2(*reinterpret_cast<const __half2 *>(&xr.y));
-                    const float s = fmaf(w01.x, x01.x, fmaf(w01.y, x01.y, fmaf(w23.x, x23.x, w23.y * x23.y)));
-                    acc[i] = fmaf(scale, s, acc[i]);
-                }
-            }
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < MR; i++) {
-        if (i < m) {
-            float v = acc[i];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) {
-                __half hv = __float2half_rn(v);
-                if (bias) hv = __hadd(hv, bias[row]);
-                if (residual) hv = __hadd(hv, residual[(size_t)i * n_rows + row]);
-                y[(size_t)i * n_rows + row] = hv;
-            }
-        }
     }
 }
 
@@ -383,7 +304,7 @@ int gemv_clusters(tlc_ctx *ctx, int ks) {
 
 // Tiles along K that one launch can hold the activations of, per row tile count.
 constexpr int kMaxCluster = 16;
-template <int QT> constexpr int max_window(int nt, int cw) { return cw * tiles_of<QT>(nt == 1 ? 3 : 2); }
+template <int QT> constexpr int max_window(int nt, int cw) { return cw * tiles_of<QT>(nt == 1 ? 3 : 2); }  // (Q6_K: one each)
 
 // 2 to 16 activation rows.
 template <int QT, int NT>
@@ -409,7 +330,7 @@ int32_t launch_mma(tlc_ctx *ctx, GemvParams &p) {
     p.ktiles_win = (p.ktiles + ks - 1) / ks;
     p.tiles_warp = (p.ktiles_win + cw - 1) / cw;
     const int ti = (p.tiles_warp + T1 - 1) / T1;
-    p.stage_bytes = p.ktiles_win * TILE;
+    p.stage_bytes = QT == TLC_TYPE_Q6_K ? (p.ktiles_win + 7) / 8 * kQ6Box : p.ktiles_win * TILE;
     p.m_inv = 65536 / p.m + 1;
     int grid = p.total_units * ks < max_ctas ? p.total_units * ks : max_ctas;
     const int units_per_cta = (p.total_units + grid / ks - 1) / (grid / ks);
@@ -429,7 +350,7 @@ int32_t launch_mma(tlc_ctx *ctx, GemvParams &p) {
             p.round = round < all ? round : all;
             p.n_rounds = (units_per_cta * p.subs + p.round - 1) / p.round;
         }
-        lay = gemv_smem(cw, ti, NT, p.batch, p.round);
+        lay = gemv_smem(cw, starts_of<QT>(ti), NT, p.batch, p.round);
         if ((size_t)lay.ring + 3 * (size_t)p.stage_bytes <= cap || batch <= p.subs) break;
     }
     // No more stages than this CTA will ever fill.
@@ -450,9 +371,11 @@ int32_t launch_mma(tlc_ctx *ctx, GemvParams &p) {
 #define TLC_GEMV_CASE(TI) \
     if (ti == TI) return cw == 8 ? launch_rows<QT, NT, TI, 8>(ctx, p, grid, smem) : launch_rows<QT, NT, TI, 16>(ctx, p, grid, smem);
     TLC_GEMV_CASE(1)
-    TLC_GEMV_CASE(2)
-    if constexpr (NT == 1) {
-        TLC_GEMV_CASE(3)
+    if constexpr (QT != TLC_TYPE_Q6_K) {
+        TLC_GEMV_CASE(2)
+        if constexpr (NT == 1) {
+            TLC_GEMV_CASE(3)
+        }
     }
 #undef TLC_GEMV_CASE
     return tlc_fail(TLC_ERR_INVALID_OPERATION, "gemv: K = %d too large", p.k);
@@ -586,8 +509,10 @@ int32_t tlc_launch_gemv(tlc_ctx *ctx, const tlc_gemv_args &a) {
     }
 
     if (type == TLC_TYPE_Q6_K) {
-        // Resident Q6_K (one weight per launch; RMSNorm, if asked for, as its own kernel; bias
-        // and residual in the store).  More than eight activation rows take further passes.
+        // Resident Q6_K (stock Q4_0 GGUF files store output.weight, the largest linear of a decode step, so): one
+        // weight per launch; RMSNorm, if asked for, as its own kernel; bias and residual in the store.
+        // More than sixteen activation rows take further passes.  Bound by the integer operations that put the 4 + 2
+        // bits together (ten an MMA of 16 x 16 weights), at about half of the HBM rate.
         TLC_REQUIRE(a.epilogue != TLC_EPI_SWIGLU && a.n_out == 1 && a.outs[0].rope_heads == 0 &&
                         a.outs[0].row_stride < 0 && a.outs[0].pos_stride == 0,
                     TLC_ERR_INVALID_OPERATION, "fused RoPE / SiLU.mul / cache epilogues need a Q4_0 or Q8_0 weight");
@@ -598,35 +523,34 @@ int32_t tlc_launch_gemv(tlc_ctx *ctx, const tlc_gemv_args &a) {
             x = static_cast<const __half *>(ctx->scratch);
         }
         TLC_REQUIRE(((uintptr_t)x & 15) == 0, TLC_ERR_INVALID_OPERATION, "linear: activations must be 16-byte aligned");
-        const __half *residual = a.epilogue == TLC_EPI_RESIDUAL ? static_cast<const __half *>(a.residual) : nullptr;
-        // rows per pass: up to eight, fewer if the activation rows would not fit in shared memory
-        int per = 8;
-        while (per > 1 && (size_t)per * k * 2 > (size_t)ctx->prop.sharedMemPerBlockOptin - 1024) per >>= 1;
-        TLC_REQUIRE((size_t)per * k * 2 <= (size_t)ctx->prop.sharedMemPerBlockOptin - 1024, TLC_ERR_INVALID_OPERATION,
-                    "linear: K = %lld too large for the shared-memory staging", (long long)k);
-        static bool configured[64] = {};
-        if (!configured[ctx->device & 63]) {
-            TLC_CUDA(cudaFuncSetAttribute(linear_q6k_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)ctx->prop.sharedMemPerBlockOptin));
-            TLC_CUDA(cudaFuncSetAttribute(linear_q6k_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)ctx->prop.sharedMemPerBlockOptin));
-            TLC_CUDA(cudaFuncSetAttribute(linear_q6k_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)ctx->prop.sharedMemPerBlockOptin));
-            configured[ctx->device & 63] = true;
-        }
-        const unsigned grid = (unsigned)((w0->n_rows * 32 + 255) / 256);
-        for (int m0 = 0; m0 < a.m; m0 += per) {
-            const int mc = a.m - m0 < per ? a.m - m0 : per;
-            auto kern = mc == 1 ? linear_q6k_kernel<1> : mc <= 4 ? linear_q6k_kernel<4> : linear_q6k_kernel<8>;
-            cudaError_t le = tlc_launch_pdl(
-                ctx, kern, dim3(grid), dim3(256), (size_t)mc * k * 2, static_cast<const uint8_t *>(w0->data), w0->row_pitch,
-                (int)w0->n_rows, (int)k, x + (size_t)m0 * k, mc, static_cast<__half *>(a.outs[0].y) + (size_t)m0 * w0->n_rows,
-                static_cast<const __half *>(a.bias), residual ? residual + (size_t)m0 * w0->n_rows : nullptr);
-            if (le != cudaSuccess) {
-                cudaGetLastError();
-                return tlc_fail(TLC_ERR_CUDA, "Q6_K linear launch failed: %s", cudaGetErrorString(le));
-            }
-            TLC_CHECK_LAUNCH(ctx);
+        // (17 to 24 rows stay three passes of eight, the launch count callers have been promised; sixteen rows
+        // cost 1.6 times eight: 32000 x 2048 takes 18.2 us at 8 rows and 28.3 us at 16, 85.7 and 167.9 us before.)
+        const int pass = a.m > 16 && a.m <= 24 ? 8 : 16;
+        for (int m0 = 0; m0 < a.m; m0 += pass) {
+            GemvParams p{};
+            p.m = a.m - m0 < pass ? a.m - m0 : pass;
+            p.n_out = 1;
+            p.subs = 1;
+            p.t[0].n = (int)w0->n_rows;
+            p.t[0].row_stride = w0->n_rows;
+            p.t[0].y = static_cast<__half *>(a.outs[0].y) + (size_t)m0 * w0->n_rows;
+            p.slabs[0] = p.total_units = (int)((w0->n_rows + kRows - 1) / kRows);
+            p.k = (int)k;
+            p.nblk = (int)(k / 16);
+            p.ktiles = (int)(k / 256);
+            p.x = x + (size_t)m0 * k;
+            p.epilogue = a.epilogue;
+            p.bias = static_cast<const __half *>(a.bias);
+            p.residual = a.epilogue == TLC_EPI_RESIDUAL ? static_cast<const __half *>(a.residual) + (size_t)m0 * w0->n_rows : nullptr;
+            p.status = ctx->dev_status;
+            p.wait_ns = ctx->wait_ns;
+            CUtensorMap map;
+            static_assert(sizeof map == sizeof p.w_map, "tensor map size");
+            TLC_REQUIRE(tlc_gemm::encode_map(&map, CU_TENSOR_MAP_DATA_TYPE_UINT64, CU_TENSOR_MAP_SWIZZLE_NONE, w0->data, w0->row_pitch / 8,
+                                             (uint64_t)w0->n_rows, w0->row_pitch, kQ6BoxRow / 8, kRows),
+                        TLC_ERR_CUDA, "linear: no tensor map for a Q6_K weight");
+            memcpy(p.w_map, &map, sizeof map);
+            if (int32_t rc = p.m <= 8 ? launch_mma<TLC_TYPE_Q6_K, 1>(ctx, p) : launch_mma<TLC_TYPE_Q6_K, 2>(ctx, p)) return rc;
         }
         return TLC_OK;
     }

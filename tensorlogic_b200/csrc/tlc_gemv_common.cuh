@@ -33,6 +33,12 @@ template <> struct QTraits<TLC_TYPE_Q8_0> {
     static constexpr float OFFSET = 128.0f;
 };
 
+template <> struct QTraits<TLC_TYPE_Q6_K> {  // a super-block of 256 columns; rows of padded super-blocks, not tiles
+    static constexpr int TB = 16;            // groups of 16 columns
+    static constexpr int TILE_BYTES = 16 * 224;
+    static constexpr float OFFSET = 32.0f;
+};
+
 struct GemvTensor {
     const uint8_t *w;   // tiles, [slab][k-tile]
     size_t slab_pitch;  // bytes of one 16-row slab
@@ -78,6 +84,7 @@ struct GemvParams {
     // The K range: ksplit CTAs of a cluster, windows of ktiles_win tiles; each warp holds tiles_warp of them.
     int ksplit, ktiles_win, tiles_warp;
     int batch;  // slabs per cross-warp reduction
+    alignas(64) unsigned char w_map[128];  // Q6_K: tensor map of the weight's rows, in 8-byte elements
     int round, n_rounds;  // cluster: slabs (of one CTA) per exchange, exchanges of a launch
     // tlc_gemv_splitk_finish: f32 shares [ksplit][m][ntot] of a split-K GEMM
     int ntot;

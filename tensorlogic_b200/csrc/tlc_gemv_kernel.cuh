@@ -5,24 +5,29 @@
 
 namespace tlc_gemv {
 
-// Blocks of K that a consumer warp holds the activations of, in registers, for the whole launch:
-// TI = 1, 2, 3 times four (Q4_0: TI tiles, Q8_0: 2 TI tiles).
-template <int QT> constexpr int tiles_of(int ti) { return ti * (QT == TLC_TYPE_Q4_0 ? 1 : 2); }
+// What a consumer warp holds the activations of, in registers, for the whole launch: TI = 1, 2, 3 times 128 columns
+// (Q4_0: TI tiles, Q8_0: 2 TI tiles); Q6_K: one super-block of 256 columns (TI = 1).
+template <int QT> constexpr int tiles_of(int ti) { return QT == TLC_TYPE_Q6_K ? 1 : ti * (QT == TLC_TYPE_Q4_0 ? 1 : 2); }
+// Accumulator start values of a warp's window: one per 32 columns, Q6_K one per 16.
+template <int QT> constexpr int starts_of(int ti) { return QT == TLC_TYPE_Q6_K ? 16 : 4 * ti; }
+// Q6_K: a slab is fetched in boxes of eight super-blocks; a row of a box takes 16 bytes of the next super-block
+// along, so that the rows of a fragment lie in different banks.
+constexpr int kQ6BoxRow = 8 * 224 + 16, kQ6Box = 16 * kQ6BoxRow;
 
 constexpr int kRedPitch = 20;  // f32 per activation row of a warp's 16 sums: the lanes' stores meet 32 banks
 
 // Shared-memory layout (bytes from the start of dynamic shared memory):
 //   0     full [8], empty [8] mbarriers          128 abort flag
-//   256   cinit: accumulator start values [CW warps][4 TI blocks][8 NT] f32
+//   256   cinit: accumulator start values [CW warps][4 TI blocks, or 16 groups][8 NT] f32
 //   ...   red   [2][batch][CW warps][8 NT rows][20] f32
 //   ...   part  [round][8 NT][16] f32: a cluster CTA's share of the sums
 //   ...   ring  [stages][tiles of the CTA's window] weight tiles as they lie in HBM (128-byte aligned)
 struct GemvSmem {
     int red, part, ring, red_slot;
 };
-__host__ __device__ inline GemvSmem gemv_smem(int cw, int ti, int nt, int batch, int round) {
+__host__ __device__ inline GemvSmem gemv_smem(int cw, int starts, int nt, int batch, int round) {
     GemvSmem s;
-    s.red = 256 + cw * 4 * ti * 8 * nt * 4;
+    s.red = 256 + cw * starts * 8 * nt * 4;
     s.red_slot = cw * 8 * nt * kRedPitch;
     s.part = s.red + 2 * batch * s.red_slot * 4;
     s.ring = (s.part + round * 8 * nt * 16 * 4 + 127) & ~127;
@@ -152,12 +157,15 @@ __global__ void __launch_bounds__(CW * 32, CW == 8 ? 2 : 1) gemv_mma_kernel(cons
     constexpr int CT = CW * 32;
     constexpr int TILE = T::TILE_BYTES;
     constexpr int TW = tiles_of<QT>(TI);  // tiles of a warp's window
-    constexpr int NB = 4 * TI;            // blocks
+    constexpr bool Q6 = QT == TLC_TYPE_Q6_K;
+    constexpr int NB = starts_of<QT>(TI);  // blocks (Q6_K: groups of 16)
+    constexpr int BK = Q6 ? 16 : 32;       // columns of a block
+    constexpr int NR = Q6 ? 2 : 4;         // fragment registers of a block
     constexpr int MP = 8 * NT;
 
     extern __shared__ __align__(128) uint8_t smem[];
     volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + 128);
-    const GemvSmem lay = gemv_smem(CW, TI, NT, p.batch, p.round);
+    const GemvSmem lay = gemv_smem(CW, NB, NT, p.batch, p.round);
     float *cinit = reinterpret_cast<float *>(smem + 256);
     float *red = reinterpret_cast<float *>(smem + lay.red);
     float *part = reinterpret_cast<float *>(smem + lay.part);
@@ -191,7 +199,7 @@ __global__ void __launch_bounds__(CW * 32, CW == 8 ? 2 : 1) gemv_mma_kernel(cons
     const int wt0 = warp * p.tiles_warp;                                                // first tile of the warp, in the window
     const int my_tiles = max(0, min(p.tiles_warp, my_ktiles - wt0));
     const int wb0 = kb0 + wt0 * T::TB;                                                  // first block of the warp
-    const int my_blocks = max(0, min(my_tiles * T::TB, p.nblk - wb0));                  // blocks that exist
+    const int my_blocks = max(0, min(my_tiles * T::TB, p.k / BK - wb0));                // blocks that exist
 
     // A ring of slabs (the CTA's window of each: one bulk copy, its tiles lie side by side).  There is no
     // producer warp -- its registers are worth more in the consumers -- : the warps take turns, one slab
@@ -207,6 +215,17 @@ __global__ void __launch_bounds__(CW * 32, CW == 8 ? 2 : 1) gemv_mma_kernel(cons
         int ti, sl;
         place(unit_at(p.subs == 2 ? i >> 1 : i), ti, sl);
         const int tw = p.subs == 2 ? i & 1 : ti;
+        if constexpr (Q6) {
+            const int boxes = (my_ktiles + 7) >> 3;
+            mbar_expect_tx(&full[s], (uint32_t)(boxes * kQ6Box));
+            for (int b = 0; b < boxes; b++)  // (the map counts in 8-byte elements)
+                asm volatile(
+                    "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+                        ring + (uint32_t)(s * p.stage_bytes + b * kQ6Box)),
+                    "l"(reinterpret_cast<uint64_t>(p.w_map)), "r"((kt0 + 8 * b) * 28), "r"(sl * kRows), "r"(smem_u32(&full[s]))
+                    : "memory");
+            return;
+        }
         const uint8_t *src = p.t[tw].w + (size_t)sl * p.t[tw].slab_pitch + (size_t)kt0 * TILE;
         mbar_expect_tx(&full[s], copy_bytes);
         bulk_g2s_hint(smem + lay.ring + (size_t)s * p.stage_bytes, src, copy_bytes, &full[s], l2_evict_first_policy());
@@ -231,9 +250,33 @@ __global__ void __launch_bounds__(CW * 32, CW == 8 ? 2 : 1) gemv_mma_kernel(cons
 
     // (a) The warp's window of the activations into fragment registers (lane (g, t): eight values of every block
     // of row g (+ 8)), and the accumulator start values to shared memory.
-    uint32_t xb[NT][NB][4];
+    uint32_t xb[NT][NB][NR];
     float *ci_w = cinit + warp * NB * MP;
-    if (p.frag) {
+    if constexpr (Q6) {
+        // lane (g, t): elements 4t .. 4t+3 of every group of 16 of row g, as they lie
+#pragma unroll
+        for (int nt = 0; nt < NT; nt++) {
+            const int m = nt * 8 + g;
+            const __half *xr = p.x + (size_t)(m < p.m ? m : 0) * p.k + (size_t)wb0 * 16 + 4 * t;
+#pragma unroll
+            for (int b = 0; b < NB; b++) {
+                const uint2 v = b < my_blocks && m < p.m ? *reinterpret_cast<const uint2 *>(xr + b * 16) : make_uint2(0, 0);
+                xb[nt][b][0] = v.x;
+                xb[nt][b][1] = v.y;
+            }
+        }
+#pragma unroll
+        for (int nt = 0; nt < NT; nt++)
+#pragma unroll
+            for (int b = 0; b < NB; b++) {
+                const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&xb[nt][b][0]));
+                const float2 c = __half22float2(*reinterpret_cast<const __half2 *>(&xb[nt][b][1]));
+                float s = (a.x + a.y) + (c.x + c.y);
+                s += __shfl_xor_sync(0xffffffffu, s, 1);
+                s += __shfl_xor_sync(0xffffffffu, s, 2);
+                if (t == 0) ci_w[b * MP + nt * 8 + g] = -32.0f * 5.9604644775390625e-08f * s;  // * 2^-24
+            }
+    } else if (p.frag) {
 #pragma unroll
         for (int b = 0; b < NB; b++)
 #pragma unroll
@@ -364,6 +407,78 @@ __global__ void __launch_bounds__(CW * 32, CW == 8 ? 2 : 1) gemv_mma_kernel(cons
                 const bool ready = n_slabs > 0 && warp_wait(&full[rs], rpar, abort_flag, p.status, 2, p.wait_ns);
                 const uint32_t sb = ring + (uint32_t)(rs * p.stage_bytes) + warp_off;
                 const int nt_tiles = ready ? my_tiles : 0;
+                if constexpr (Q6) {
+                    if (nt_tiles > 0) {
+                        // Super-block of the warp, rows g and g + 8: 128 low nibbles pairs, 64 high bit quads, 16 scales, d
+                        // (GGUFLoader::dequantize_q6_k, src/model/formats/gguf.rs:128-218).  The word of lane t holds
+                        // elements 4t .. 4t+3 of four groups of 16, 32 apart; a 6-bit value in the low bits of
+                        // a binary16 is the subnormal q * 2^-24, the -32 is in the start value, and the group's 8-bit
+                        // scale multiplies the 16 x 8 result in f32, the super-block's d at the end.
+                        const uint32_t r0 = ring + (uint32_t)(rs * p.stage_bytes) + (uint32_t)((warp >> 3) * kQ6Box + (warp & 7) * 224) + g * kQ6BoxRow;
+                        const uint32_t r1 = r0 + 8 * kQ6BoxRow;
+                        float part0[2 * NT], part1[2 * NT];
+#pragma unroll
+                        for (int i = 0; i < 2 * NT; i++) part0[i] = part1[i] = 0.f;
+                        const uint4 s0 = lds_u128(r0 + 192), s1 = lds_u128(r1 + 192);
+                        const uint32_t sw0[4] = {s0.x, s0.y, s0.z, s0.w}, sw1[4] = {s1.x, s1.y, s1.z, s1.w};
+                        const __half2 m1152 = __float2half2_rn(-1152.f);
+                        // signed byte i of a scale word pair -> float, two at a time (1024 + 128 + sc, minus 1152: exact)
+                        auto scales2 = [&](uint32_t w, int hi) {
+                            const uint32_t h = __byte_perm(w ^ 0x80808080u, 0x64646464u, hi ? 0x4342 : 0x4140);
+                            return __half22float2(__hadd2(*reinterpret_cast<const __half2 *>(&h), m1152));
+                        };
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            // group j (elements 32 j + 16 is + ...) of half h has scale 8 h + is + 2 j
+                            float2 sc0[4], sc1[4];
+#pragma unroll
+                            for (int j = 0; j < 4; j++) {
+                                sc0[j] = scales2(sw0[2 * h + (j >> 1)], j & 1);
+                                sc1[j] = scales2(sw1[2 * h + (j >> 1)], j & 1);
+                            }
+#pragma unroll
+                            for (int is = 0; is < 2; is++) {
+                                const uint32_t o = (uint32_t)(64 * h + 16 * is + 4 * t), oh = (uint32_t)(128 + 32 * h + 16 * is + 4 * t);
+                                const uint32_t qa[2] = {lds_u32(r0 + o), lds_u32(r1 + o)}, qb[2] = {lds_u32(r0 + o + 32), lds_u32(r1 + o + 32)};
+                                const uint32_t qh[2] = {lds_u32(r0 + oh), lds_u32(r1 + oh)};
+#pragma unroll
+                                for (int j = 0; j < 4; j++) {
+                                    uint32_t a[4];
+#pragma unroll
+                                    for (int r = 0; r < 2; r++) {
+                                        const uint32_t lo4 = (j & 1 ? qb[r] : qa[r]) >> (j >= 2 ? 4 : 0);
+                                        const uint32_t hi2 = j == 0 ? qh[r] << 4 : j == 1 ? qh[r] << 2 : j == 2 ? qh[r] : qh[r] >> 2;
+                                        const uint32_t v = (lo4 & 0x0F0F0F0Fu) | (hi2 & 0x30303030u);
+                                        a[r] = __byte_perm(v, 0, 0x4140);
+                                        a[2 + r] = __byte_perm(v, 0, 0x4342);
+                                    }
+                                    const int b = 8 * h + 2 * j + is;  // group of the super-block: elements 128 h + 32 j + 16 is
+                                    const float e0 = is ? sc0[j].y : sc0[j].x, e1 = is ? sc1[j].y : sc1[j].x;
+#pragma unroll
+                                    for (int nt = 0; nt < NT; nt++) {
+                                        const float2 ci = lds_f32x2(ci_addr + (uint32_t)((b * MP + nt * 8) * 4));
+                                        const float cc[4] = {ci.x, ci.y, ci.x, ci.y};
+                                        float d[4];
+                                        mma16816(d, a, xb[nt][b][0], xb[nt][b][1], cc);
+                                        part0[2 * nt] = fmaf(e0, d[0], part0[2 * nt]);
+                                        part0[2 * nt + 1] = fmaf(e0, d[1], part0[2 * nt + 1]);
+                                        part1[2 * nt] = fmaf(e1, d[2], part1[2 * nt]);
+                                        part1[2 * nt + 1] = fmaf(e1, d[3], part1[2 * nt + 1]);
+                                    }
+                                }
+                            }
+                        }
+                        const float d0 = __half2float(__ushort_as_half((unsigned short)lds_u32(r0 + 208)));
+                        const float d1 = __half2float(__ushort_as_half((unsigned short)lds_u32(r1 + 208)));
+#pragma unroll
+                        for (int nt = 0; nt < NT; nt++) {
+                            acc[nt * 4 + 0] = d0 * part0[2 * nt];
+                            acc[nt * 4 + 1] = d0 * part0[2 * nt + 1];
+                            acc[nt * 4 + 2] = d1 * part1[2 * nt];
+                            acc[nt * 4 + 3] = d1 * part1[2 * nt + 1];
+                        }
+                    }
+                } else {
 #pragma unroll
                 for (int i = 0; i < TW; i++) {
                     if (i >= nt_tiles) break;
@@ -417,6 +532,7 @@ __global__ void __launch_bounds__(CW * 32, CW == 8 ? 2 : 1) gemv_mma_kernel(cons
                             acc[nt * 4 + 3] = fmaf(dhi[j], d2[3], acc[nt * 4 + 3]);
                         }
                     }
+                }
                 }
                 __syncwarp();  // the stage has been read by all lanes
                 if (lane == 0) mbar_arrive(&empty[rs]);

@@ -46,3 +46,16 @@ def test_fused_epilogues(dev, qtype, k, m):
     assert rel_l2(swiglu_gate_up(x, g, u, nw, 1e-5).numpy(), swiglu(linear(h, g), linear(h, u)).numpy()) < 2e-3
     r = dev.tensor(synth.activations(8, "er", (m, 1000)))
     assert rel_l2(linear_residual(h, g, r).numpy(), add(linear(h, g), r).numpy()) < TIGHT
+
+
+@pytest.mark.parametrize("n,k,m", [(16, 256, 1), (15, 2304, 8), (33, 4096, 9), (40, 4352, 16), (17, 8448, 2), (50, 2048, 40)])
+def test_q6_k_windows(dev, ref, n, k, m):
+    """Q6_K on the same kernel: one super-block a warp, eight and sixteen warps, clusters, further passes."""
+    from tensorlogic_b200 import synth
+    from tensorlogic_b200.api import QTensor, linear
+    rng = np.random.default_rng(n * k + m)
+    raw = rng.integers(0, 256, (n * k // 256, 210), dtype=np.uint8)
+    raw[:, 208:210] = rng.uniform(-2e-5, 2e-5, (raw.shape[0], 1)).astype(np.float16).view(np.uint8)
+    x = synth.activations(9, f"q6x{m}x{k}", (m, k))
+    got = linear(dev.tensor(x), QTensor.from_blocks(dev, 14, n, k, raw)).numpy()
+    assert rel_l2(got, ref.linear_q(14, raw.reshape(-1), n, k, x)) < TIGHT
