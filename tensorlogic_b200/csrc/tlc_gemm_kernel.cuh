@@ -184,6 +184,15 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(el)
         : "memory");
 }
+// (A in tensor memory: two f16 of a row per column)
+__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
+                                            uint32_t accumulate, uint32_t el) {
+    asm volatile(
+        "{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(tmem_d),
+        "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(el)
+        : "memory");
+}
 __device__ __forceinline__ void umma_commit(uint64_t *bar, uint32_t el) {
     asm volatile(
         "{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n"
@@ -334,6 +343,8 @@ __device__ __forceinline__ void epilogue_piece_swiglu(const GemmParams &p, const
 
 // Tensor map of activations for the TMA-fed A tile (defined in tlc_gemm_sm100.cu).
 bool encode_x_map(CUtensorMap *map, const GemmParams &p);
+bool encode_map_nd(CUtensorMap *map, CUtensorMapDataType type, CUtensorMapSwizzle swizzle, const void *ptr, int rank,
+                   const uint64_t *dims, const uint64_t *pitches, const uint32_t *box);
 bool encode_map(CUtensorMap *map, CUtensorMapDataType type, CUtensorMapSwizzle swizzle, const void *ptr, uint64_t inner,
                 uint64_t outer, uint64_t pitch, uint32_t box_inner, uint32_t box_outer);
 // f16, boxes of 64 columns under the 128-byte swizzle

@@ -12,8 +12,10 @@ using namespace tlc_gemm;
 
 // Tensor map of a row-major matrix [outer, inner], rows `pitch` bytes apart: boxes of box_outer rows x
 // box_inner elements, zero fill outside.  False when the driver entry point is missing or refuses the shape.
-bool tlc_gemm::encode_map(CUtensorMap *map, CUtensorMapDataType type, CUtensorMapSwizzle swizzle, const void *ptr,
-                          uint64_t inner, uint64_t outer, uint64_t pitch, uint32_t box_inner, uint32_t box_outer) {
+// Extents and box from the contiguous dimension outwards; `pitches`: bytes from one element to the next of
+// each dimension but that one.
+bool tlc_gemm::encode_map_nd(CUtensorMap *map, CUtensorMapDataType type, CUtensorMapSwizzle swizzle, const void *ptr,
+                             int rank, const uint64_t *dims, const uint64_t *pitches, const uint32_t *box) {
     static PFN_cuTensorMapEncodeTiled_v12000 encode = [] {
         void *fn = nullptr;
         cudaDriverEntryPointQueryResult qres;
@@ -23,14 +25,28 @@ bool tlc_gemm::encode_map(CUtensorMap *map, CUtensorMapDataType type, CUtensorMa
         cudaGetLastError();
         return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
     }();
-    if (!encode || ((uintptr_t)ptr & 15) != 0 || (pitch & 15) != 0) return false;
-    const cuuint64_t dims[2] = {inner, outer};
-    const cuuint64_t strides[1] = {pitch};
-    const cuuint32_t box[2] = {box_inner, box_outer};
-    const cuuint32_t estr[2] = {1, 1};
-    return encode(map, type, 2, const_cast<void *>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+    if (!encode || ((uintptr_t)ptr & 15) != 0) return false;
+    cuuint64_t d[5], st[4];
+    cuuint32_t bx[5], es[5];
+    for (int i = 0; i < rank; i++) {
+        d[i] = dims[i];
+        bx[i] = box[i];
+        es[i] = 1;
+        if (i + 1 < rank) {
+            if ((pitches[i] & 15) != 0) return false;
+            st[i] = pitches[i];
+        }
+    }
+    return encode(map, type, (cuuint32_t)rank, const_cast<void *>(ptr), d, st, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+bool tlc_gemm::encode_map(CUtensorMap *map, CUtensorMapDataType type, CUtensorMapSwizzle swizzle, const void *ptr,
+                          uint64_t inner, uint64_t outer, uint64_t pitch, uint32_t box_inner, uint32_t box_outer) {
+    const uint64_t dims[2] = {inner, outer};
+    const uint32_t box[2] = {box_inner, box_outer};
+    return encode_map_nd(map, type, swizzle, ptr, 2, dims, &pitch, box);
 }
 
 bool tlc_gemm::encode_f16_map(CUtensorMap *map, const void *ptr, uint64_t inner, uint64_t outer, uint64_t pitch,

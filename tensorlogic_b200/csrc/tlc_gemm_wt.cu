@@ -103,14 +103,6 @@ constexpr int kATile = 128 * 64 * 2;  // f16 weights: one K step of the A operan
 // unpacked quantized weights hold rows of eight slabs, 16 apart; 20 apart they meet 32 banks.
 __device__ __forceinline__ int fpos(int n) { return n + ((n >> 4) << 2); }
 
-__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
-                                            uint32_t accumulate, uint32_t el) {
-    asm volatile(
-        "{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n"
-        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(tmem_d),
-        "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(el)
-        : "memory");
-}
 // 16 consecutive tensor-memory columns of this thread's lane.
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
     asm volatile(

@@ -161,3 +161,34 @@ def test_attention_errors(dev):
         cache.attention(0, dev.tensor(np.zeros((1, 4, 64), np.float16)), 4, q_pos0=16)
     with pytest.raises(TensorError):
         KVCache(dev, 1, 2, 60)
+
+
+@pytest.mark.parametrize("H,Hkv,D", [(16, 1, 64), (4, 4, 128), (16, 2, 128)])
+@pytest.mark.parametrize("B,I,pos0", [(1, 2, 62), (1, 63, 1), (1, 64, 64), (1, 129, 0), (3, 33, 31), (2, 128, 65)])
+@pytest.mark.parametrize("rise", [0.0, 6.0])
+def test_prefill_attention_tile_edges(dev, ref, H, Hkv, D, B, I, pos0, rise):
+    """Query and key counts around the tiles of the prefill kernel, several sequences in one launch (a tile's last
+    rows belong to the next one), and scores that grow along the context, so that the reference of the exponentials
+    moves in every tile; and the same from an address TMA cannot read."""
+    import ctypes as C
+    from tensorlogic_b200._lib import check
+    from tensorlogic_b200.api import KVCache
+    T, cap, row, scale = pos0 + I, pos0 + I + 5, Hkv * D, 1.0 / np.sqrt(D)
+    cache = KVCache(dev, 1, Hkv, D, max_seq=cap, max_batch=B)
+    kptr, vptr = C.c_void_p(), C.c_void_p()
+    check(dev.lib.tlc_kvcache_layer_ptrs(cache.handle, 0, C.byref(kptr), C.byref(vptr)))
+    seqs = [_qkv(I + 3 * b, I, T, H, Hkv, D) for b in range(B)]
+    for b, (q, k, v) in enumerate(seqs):
+        k *= np.linspace(0.3, 0.3 + rise, T, dtype=np.float16)[:, None, None]
+        check(dev.lib.tlc_upload(dev.handle, kptr.value + b * cap * row * 2, k.ctypes.data, T * row * 2))
+        check(dev.lib.tlc_upload(dev.handle, vptr.value + b * cap * row * 2, v.ctypes.data, T * row * 2))
+    dev.synchronize()
+    n = B * I * H * D
+    q = dev.tensor(np.concatenate([np.zeros(2, np.float16)] + [s[0].ravel() for s in seqs]))
+    q0 = dev.tensor(np.concatenate([s[0].ravel() for s in seqs]))
+    out = dev.tensor(np.zeros(n, np.float16))
+    for ptr in (q0.ptr, q.ptr + 4):
+        check(dev.lib.tlc_attention(dev.handle, cache.handle, 0, ptr, out.ptr, B, I, H, pos0, None, 0, scale))
+        got = out.numpy().reshape(B, I, H, D)
+        for b, (qb, k, v) in enumerate(seqs):
+            assert rel_l2(got[b], ref.attention(qb, k, v, scale, q_pos0=pos0)) < TIGHT, (ptr, b)
