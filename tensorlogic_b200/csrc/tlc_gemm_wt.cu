@@ -47,6 +47,7 @@ constexpr int kChunk = 32;                     // activation rows per round of t
 constexpr int kMaxRaw = 12, kMaxX = 8, kMaxA = 7;
 constexpr int kHeader = 1024;
 constexpr int kStagePitch = 160;  // f32 per activation row of the epilogue staging (see fpos)
+constexpr int kSumPitch = 144;    // ... of a CTA's sums for the cluster: two rows apart meet all banks (see sum8)
 
 struct WtOut {
     const uint8_t *w;
@@ -70,6 +71,7 @@ struct WtParams {
     long long total_steps;
     int grid;
     int ks;             // cluster form: CTAs per tile; 0: stream form
+    int own_gather;     // cluster form: the sums' place is not in the rings
     int m, bn, tm;      // activation rows, of a tile, tiles of them
     int raw_stages, x_stages, a_stages, acc_stages;
     int tmem_cols, a_col0, a_col_a;  // columns of an accumulator; first column of the A stages
@@ -267,33 +269,22 @@ __device__ __forceinline__ void load8(const float *at, float (&v)[8]) {
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
     v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
-// The same from the CTAs of the cluster (shared-memory address `at` in each), added in rank order; four
-// ranks in flight at once, since one remote load takes most of a microsecond.
-__device__ __forceinline__ void sum8(uint32_t at, int ks, float (&v)[8]) {
+// The cluster's sums of eight consecutive weight rows from n on, added in rank order.  They lie in tensor-memory
+// lane order (`at`: this activation row's from rank 0, `part`: f32 from one rank's to the next one's), where
+// the lanes of quantized weights hold the rows of a slab in pairs 16 apart.
+template <bool DQ>
+__device__ __forceinline__ void sum8(const float *at, int part, int ks, int n, float (&v)[8]) {
 #pragma unroll
     for (int e = 0; e < 8; e++) v[e] = 0.f;
-    for (int r0 = 0; r0 < ks; r0 += 4) {
-        float4 a[4], b[4];
+    const float *src = at + (DQ ? ((n & 15) >> 1) * 16 + (n >> 4) * 2 : n);
+#pragma unroll 2
+    for (int r = 0; r < ks; r++, src += part)
 #pragma unroll
-        for (int r = 0; r < 4; r++) {
-            a[r] = b[r] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (r0 + r < ks) {
-                uint32_t ra;
-                asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(at), "r"(r0 + r));
-                asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];"
-                             : "=f"(a[r].x), "=f"(a[r].y), "=f"(a[r].z), "=f"(a[r].w)
-                             : "r"(ra));
-                asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];"
-                             : "=f"(b[r].x), "=f"(b[r].y), "=f"(b[r].z), "=f"(b[r].w)
-                             : "r"(ra + 16));
-            }
+        for (int e = 0; e < 8; e += 2) {
+            const float2 t = *reinterpret_cast<const float2 *>(src + (DQ ? 8 * e : e));
+            v[e] += t.x;
+            v[e + 1] += t.y;
         }
-#pragma unroll
-        for (int r = 0; r < 4; r++) {
-            v[0] += a[r].x; v[1] += a[r].y; v[2] += a[r].z; v[3] += a[r].w;
-            v[4] += b[r].x; v[5] += b[r].y; v[6] += b[r].z; v[7] += b[r].w;
-        }
-    }
 }
 
 // A piece of a CTA's work: K steps [k0, k0 + n) of a tile.  A CTA owns the steps [lo, hi) of all
@@ -333,8 +324,8 @@ __global__ void __launch_bounds__(threads_of<SRC>(), 1)
     const int x_bytes = p.bn * KSTEP * 2;
     const int x_stage = x_bytes + (DQ ? 0 : kATile);  // f16 weights: the A tile lies behind the x tile
     uint8_t *raw = rings + (size_t)p.x_stages * x_stage;
-    // (cluster form: a whole tile, over the rings when they are done)
-    float *staging = reinterpret_cast<float *>(CLUSTER ? rings : raw + (size_t)p.raw_stages * RAW);
+    // stream form: staging of the epilogue; cluster form: the sums of this CTA's activation rows, from every rank
+    float *staging = reinterpret_cast<float *>(CLUSTER && !p.own_gather ? rings : raw + (size_t)p.raw_stages * RAW);
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const bool pair = p.w2 != nullptr;
@@ -381,6 +372,8 @@ __global__ void __launch_bounds__(threads_of<SRC>(), 1)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    // (the peers may write to this CTA's shared memory from here on)
+    if (CLUSTER && p.own_gather) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
     // tile -> (output, tile of that output's rows, tile of activation rows)
     auto locate = [&](int tile, int &oi, int &tn, int &m0) {
@@ -603,17 +596,7 @@ __global__ void __launch_bounds__(threads_of<SRC>(), 1)
             __syncwarp();
             tc_fence_after();
             const uint32_t taddr = tmem + ((uint32_t)(32 * q) << 16) + rc.s * p.a_col0;
-            if (CLUSTER) {  // the one tile of this CTA; everything copied or stored to the rings has been read
-                for (int c0 = 0; c0 < p.bn; c0 += 16) {
-                    uint32_t r[16];
-                    tmem_ld16(taddr + c0, r);
-                    float *dst = staging + (size_t)c0 * kStagePitch + fpos(n_local);
-#pragma unroll
-                    for (int e = 0; e < 16; e++) dst[e * kStagePitch] = __uint_as_float(r[e]);
-                }
-                tc_fence_before();
-                break;
-            }
+            if (CLUSTER) break;  // the one tile of this CTA
             if (sg.k0 + sg.n < p.steps) {
                 // The tile's last steps are with the next CTAs: leave the sums for the one that has the very last.
                 float *dst = p.partial + (size_t)g * slot + 32 * q + lane;
@@ -692,31 +675,55 @@ __global__ void __launch_bounds__(threads_of<SRC>(), 1)
         }
     }
     if (CLUSTER) {
-        // The CTAs of the cluster take the activation rows in turn and add the shares of all of them; every
-        // warp helps.  (A second barrier: the peers may still be reading this CTA's staging.)
+        // The CTAs of the cluster take the activation rows in turn.  Each stores its sums where their owner adds them
+        // up: stores need no answer, where loads from the peers took a microsecond and a barrier to let them leave
+        // (2048 x 2048, 32 rows: 8.3 -> 7.7 us; 4096 x 4096, 64 rows:
+        // 12.3 -> 10.7).  Without a place of their own the sums go over the rings, which the peers have to be done
+        // with first.
         asm volatile("griddepcontrol.wait;" ::: "memory");
         __syncwarp();
-        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        if (!p.own_gather) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         const int tile = g / p.ks;
         int oi, tn, m0;
         locate(tile, oi, tn, m0);
         const WtOut &out = p.out[oi];
         const int rows = min(p.bn, p.m - m0), groups = pair ? 8 : 16, n_base = tn * (pair ? 64 : 128);
-        const int mine = (rows - rank + p.ks - 1) / p.ks;
-        for (int item = tid; item < mine * groups; item += threads_of<SRC>()) {
-            const int c = (pair ? item >> 3 : item >> 4) * p.ks + rank, g8 = (pair ? item & 7 : item & 15) * 8;
-            const int n = n_base + g8;
-            if (n >= out.n) continue;
-            float v[8], u[8];
-            const uint32_t at = smem_u32(staging + (size_t)c * kStagePitch);
-            sum8(at + 4 * fpos(g8), p.ks, v);
-            if (pair) sum8(at + 4 * fpos(64 + g8), p.ks, u);
-            store_item(p, out, pair, v, u, m0 + c, n);
+        const int part = (p.bn + p.ks - 1) / p.ks * kSumPitch;
+        if (warp >= 4 && warp < 8) {
+            const int q = warp & 3;
+            uint32_t at = smem_u32(staging + rank * part + 32 * q + lane);
+            int owner = 0;
+            for (int c0 = 0; c0 < rows; c0 += 16) {
+                uint32_t r[16];
+                tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + c0, r);
+#pragma unroll
+                for (int e = 0; e < 16; e++) {
+                    uint32_t ra;
+                    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(at), "r"(owner));
+                    if (c0 + e < rows) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(ra), "r"(r[e]) : "memory");
+                    if (++owner == p.ks) {
+                        owner = 0;
+                        at += kSumPitch * 4;
+                    }
+                }
+                __syncwarp();
+            }
+            tc_fence_before();
         }
         __syncwarp();
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        const int mine = (rows - rank + p.ks - 1) / p.ks;
+        for (int item = tid; item < mine * groups; item += threads_of<SRC>()) {
+            const int i = pair ? item >> 3 : item >> 4, g8 = (pair ? item & 7 : item & 15) * 8;
+            const int n = n_base + g8;
+            if (n >= out.n) continue;
+            float v[8], u[8];
+            sum8<DQ>(staging + i * kSumPitch, part, p.ks, g8, v);
+            if (pair) sum8<DQ>(staging + i * kSumPitch, part, p.ks, 64 + g8, u);
+            store_item(p, out, pair, v, u, m0 + i * p.ks + rank, n);
+        }
     }
     __syncthreads();
     if (warp == 2) {
@@ -852,7 +859,10 @@ int32_t launch(tlc_ctx *ctx, WtParams &p, int tiles_n, const Plan &plan, const C
     p.partial = ctx->wt_partial;
     p.flags = ctx->wt_flags;
     const size_t x_stage = (size_t)p.bn * S::KSTEP * 2 + (S::DQ ? 0 : kATile), RAW = raw_stage_bytes<SRC>();
-    const size_t stage = (size_t)kChunk * kStagePitch * sizeof(float), budget = (size_t)224 * 1024 - kHeader - 1024 - stage;
+    // The cluster's sums get a place of their own while it costs the rings little (up to 64 activation rows).
+    const size_t sums = p.ks ? (size_t)p.ks * ((p.bn + p.ks - 1) / p.ks) * kSumPitch * sizeof(float) : 0;
+    p.own_gather = p.ks && sums <= 40 * 1024;
+    const size_t stage = p.own_gather ? sums : p.ks ? 0 : (size_t)kChunk * kStagePitch * sizeof(float), budget = (size_t)224 * 1024 - kHeader - 1024 - stage;
     int xs = (int)((S::DQ ? budget / 2 : budget) / x_stage);
     xs = xs < 2 ? 2 : xs > kMaxX ? kMaxX : xs;
     // A raw stage always returns to the same unpacking group (the ring is a multiple of the groups): a
@@ -876,12 +886,8 @@ int32_t launch(tlc_ctx *ctx, WtParams &p, int tiles_n, const Plan &plan, const C
     p.tmem_cols = 32;
     while (p.tmem_cols < cols) p.tmem_cols *= 2;
     size_t smem = xs * x_stage + rs * RAW;
-    if (p.ks) {
-        const size_t whole = (size_t)p.bn * kStagePitch * sizeof(float);
-        smem = smem > whole ? smem : whole;
-    } else {
-        smem += stage;
-    }
+    smem += stage;
+    if (p.ks && !p.own_gather && smem < sums) smem = sums;
     smem += kHeader + 1024;
     if (int32_t rc = configure<SRC>(ctx)) return rc;
     cudaLaunchConfig_t cfg = {};
