@@ -58,7 +58,6 @@ struct AttnParams {
     float *part_o;   // [rows][nsplit][D]
     int *counters;   // [B][q_tiles][Hkv], zero between launches
     int push_offset; // cluster mode: byte offset of the merge area in dynamic shared memory
-    int push_splits; // cluster mode: splits the merge area of rank 0 is laid out for (8 or 16)
     int cluster;     // 1: the nsplit CTAs of a tile form a thread-block cluster and merge through
                      // distributed shared memory instead of global scratch
     int pos_settled; // 1: the launcher vouches that positions[] was final before this kernel could start
@@ -351,36 +350,37 @@ __global__ void __launch_bounds__(kAttnThreads) attention_kernel(const AttnParam
         // rank 0 merges from its own memory; the peers are free to leave at once ----
         namespace cg = cooperative_groups;
         cg::cluster_group cl = cg::this_cluster();
-        // [nsplit][16] max, [nsplit][16] sum, [nsplit][16][D] O, behind the K/V tiles
+        // [nsplit][G] max, [nsplit][G] sum, [nsplit][G][D] O, behind the K/V tiles (one query: G of the 16 rows count)
         float *push = reinterpret_cast<float *>(smem_raw + p.push_offset);
         float *r0 = cl.map_shared_rank(push, 0);
-        const int PS = p.push_splits;
-        float *pm = r0, *pl = r0 + PS * 16, *po = r0 + 2 * PS * 16;
+        const int l_at = p.nsplit * G, o_at = (2 * p.nsplit * G + 3) & ~3;
+        float *pm = r0, *pl = r0 + l_at, *po = r0 + o_at;
         asm volatile("barrier.cluster.wait.aligned;" ::: "memory");  // every CTA of the cluster has started
-        if ((tid & 7) == 0) {
-            pm[split * 16 + row] = M;
-            pl[split * 16 + row] = L;
+        if ((tid & 7) == 0 && row_valid) {
+            pm[split * G + row] = M;
+            pl[split * G + row] = L;
         }
 #pragma unroll
         for (int j = 0; j < DPT; j += 4)
-            *reinterpret_cast<float4 *>(po + ((size_t)split * 16 + row) * D + d0 + j) =
-                make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
+            if (row_valid)
+                *reinterpret_cast<float4 *>(po + (split * G + row) * D + d0 + j) =
+                    make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         if (cl.block_rank() == 0 && row_valid) {
-            const float *lm = push, *ll = push + PS * 16, *lo = push + 2 * PS * 16;
+            const float *lm = push, *ll = push + l_at, *lo = push + o_at;
             float Mg = -INFINITY;
 #pragma unroll 4
-            for (int sp = 0; sp < p.nsplit; sp++) Mg = fmaxf(Mg, lm[sp * 16 + row]);
+            for (int sp = 0; sp < p.nsplit; sp++) Mg = fmaxf(Mg, lm[sp * G + row]);
             float Lg = 0.f;
 #pragma unroll
             for (int j = 0; j < DPT; j++) acc[j] = 0.f;
 #pragma unroll 4
             for (int sp = 0; sp < p.nsplit; sp++) {
-                const float ms = lm[sp * 16 + row];
+                const float ms = lm[sp * G + row];
                 const float wgt = ms == -INFINITY ? 0.f : expf(ms - Mg);
-                Lg += ll[sp * 16 + row] * wgt;
-                const float *ro = lo + ((size_t)sp * 16 + row) * D + d0;
+                Lg += ll[sp * G + row] * wgt;
+                const float *ro = lo + (sp * G + row) * D + d0;
 #pragma unroll
                 for (int j = 0; j < DPT; j += 4) {
                     const float4 v = *reinterpret_cast<const float4 *>(ro + j);
@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(kAttnThreads) attention_kernel(const AttnParam
 // cluster mode, the merge area of rank 0.  Every place that sets the kernel's limit uses this
 // value, so one launcher never lowers the limit another one needs.
 static constexpr size_t attention_smem_limit(int D) {
-    return (size_t)4 * kTileKeys * (D + 8) * sizeof(__half) + 128 + (size_t)16 * 16 * (D + 2) * sizeof(float);
+    return (size_t)4 * kTileKeys * (D + 8) * sizeof(__half) + 128 + ((size_t)16 * 16 * (D + 2) + 4) * sizeof(float);
 }
 
 template <typename V>
@@ -509,6 +509,32 @@ static int attention_wide_clusters(tlc_ctx *ctx, int D) {
     }
     cached[di][dev] = n;
     return n;
+}
+
+// Splits of a decode tile that merge within a cluster, 1 to 8: the fewest microseconds of
+//   tiles of a CTA x (the larger of a tile's latency and its share of the HBM, 44 KB/us for the CTAs of an SM)
+//   and the merge.
+// While all CTAs have an SM of their own any number of splits will do; beyond that clusters of 1, 2, 4 or 8, since
+// others leave holes in the GPCs, and at most four CTAs an SM (128 tiles of 2000 keys, D = 64: 17.4 us in two splits,
+// 21.8 in three, 15.5 in four, 20.3 in eight).  Two CTAs an SM whatever the number of tiles, the former rule, took
+// for 32 sequences of 2000 keys, one KV head of 128, 26.0 us, now 13.2; for 32 of 500 keys, four KV heads of 64, 8.9,
+// now 6.8; for 16 of 1000 8.4, now 7.0.
+static int cluster_splits(const tlc_ctx *ctx, int groups, int tiles, int D) {
+    const double latency = D == 64 ? 0.45 : 0.7, share = kTileKeys * D * 4 / 44e3;
+    int best = 1;
+    double best_t = 1e30;
+    for (int n = 1; n <= 8 && n <= tiles; n++) {
+        const int per = (tiles + n - 1) / n, at_once = (groups * n + ctx->sm_count - 1) / ctx->sm_count;
+        if (n > 1 && at_once > 1 && ((n & (n - 1)) != 0 || at_once > 4)) continue;
+        if ((n - 1) * per >= tiles) continue;  // a split would be empty
+        const double tile = latency > at_once * share ? latency : at_once * share;
+        const double t = per * (tile + 0.1) + (n > 1 ? 0.3 + 0.15 * n : 0.0);
+        if (t < best_t) {
+            best_t = t;
+            best = n;
+        }
+    }
+    return best;
 }
 
 // Host-side launcher shared by the ABI entry point and the decode runner.
@@ -568,7 +594,7 @@ int32_t tlc_launch_attention(tlc_ctx *ctx, tlc_kvcache *cache, int layer, const 
     }
     const int RQ = 16 / G;
     p.q_tiles = (I + RQ - 1) / RQ;
-    // Decode: split the keys so that about two CTAs per SM are busy.
+    // Decode: split the keys, into up to so many parts that two CTAs per SM are busy.
     int nsplit = 1;
     if (I == 1) {
         const int tiles = (T + kTileKeys - 1) / kTileKeys;
@@ -578,17 +604,20 @@ int32_t tlc_launch_attention(tlc_ctx *ctx, tlc_kvcache *cache, int layer, const 
         if (nsplit > 64) nsplit = 64;
     }
     // Up to 128 key tiles (8192 keys) the splits of a tile form one thread-block cluster
-    // (8 CTAs, up to 16 tiles each, walked with the double-buffered tile loop) and merge
+    // (up to 8 CTAs, up to 16 tiles each, walked with the double-buffered tile loop) and merge
     // through distributed shared memory; beyond that, up to 64 independent splits and the
     // global-memory merge.
     // A portable cluster holds eight splits.  With few (sequence, KV head) tiles -- one KV head
     // per rank of a tensor-parallel model, one sequence -- eight CTAs would walk a long context
     // alone on an otherwise idle GPU: such launches use clusters of sixteen (option attn_wide).
-    const bool cluster = I == 1 && nsplit > 1 && (T + kTileKeys - 1) / kTileKeys <= 128;
+    bool cluster = I == 1 && nsplit > 1 && (T + kTileKeys - 1) / kTileKeys <= 128;
     const bool wide = cluster && ctx->attn_wide && nsplit >= 16 && (T + kTileKeys - 1) / kTileKeys >= 24 &&
                       (long)batch * Hkv * 32 <= ctx->sm_count && attention_wide_clusters(ctx, D) > 0;
-    if (cluster && nsplit > (wide ? 16 : 8)) nsplit = wide ? 16 : 8;
-    p.push_splits = wide ? 16 : 8;
+    if (wide && nsplit > 16) nsplit = 16;
+    if (cluster && !wide) {
+        nsplit = cluster_splits(ctx, batch * Hkv, (T + kTileKeys - 1) / kTileKeys, D);
+        cluster = nsplit > 1;
+    }
     p.nsplit = nsplit;
     p.cluster = cluster ? 1 : 0;
     const int tiles_total = (T + kTileKeys - 1) / kTileKeys;
@@ -611,7 +640,7 @@ int32_t tlc_launch_attention(tlc_ctx *ctx, tlc_kvcache *cache, int layer, const 
     size_t smem_bytes = smem > smem_o ? smem : smem_o;
     if (cluster) {  // the merge area of rank 0 (every CTA of the launch has the same layout)
         p.push_offset = (int)((smem_bytes + 127) & ~(size_t)127);
-        smem_bytes = (size_t)p.push_offset + (size_t)p.push_splits * 16 * (D + 2) * sizeof(float);
+        smem_bytes = (size_t)p.push_offset + ((size_t)nsplit * G * (D + 2) + 4) * sizeof(float);
     }
     // All kernels of a decode step ask for the same (maximal) shared-memory
     // carve-out: switching the L1/shared split between consecutive launches
