@@ -299,6 +299,22 @@ def test_temperature_sample_builtin(dev, ref):
     assert temperature_sample(dev.tensor(lg), 1.0, [0.0])[0] == 0
 
 
+@pytest.mark.parametrize("vocab", [1, 7, 256, 8191, 8192, 8200, 16390, 40000])
+def test_temperature_sample_run_edges(dev, ref, vocab):
+    """Vocabularies around the runs of the sampling kernel (32 warps x 256 tokens), draws at the ends and in between."""
+    from tensorlogic_b200.api import temperature_sample
+    rng = np.random.default_rng(vocab)
+    lg = np.repeat((rng.standard_normal((1, vocab)) * 2).astype(np.float16), 5, axis=0)
+    us = np.array([0.0, 0.2501, 0.5003, 0.7504, 0.999], np.float32)
+    got = temperature_sample(dev.tensor(lg), 0.8, us)
+    for r, u in enumerate(us):
+        want, cdf = ref.temperature_sample(lg[r], 0.8, float(u), return_cdf=True)
+        if int(got[r]) != want:
+            lo, hi = sorted((int(got[r]), want))
+            # (the oracle adds 40000 values one after the other in f32)
+            assert np.all(np.abs(np.asarray(cdf[lo:hi], np.float64) - float(u)) < 5e-6), (vocab, u)
+
+
 def test_runner_temperature_sampling_is_reproducible(dev, ref):
     """Decode with temperature: tokens follow the oracle given the same uniform draws; same seed, same text."""
     from tensorlogic_b200 import synth
