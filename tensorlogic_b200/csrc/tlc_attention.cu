@@ -548,8 +548,8 @@ static int cluster_splits(const tlc_ctx *ctx, int groups, int tiles, int D) {
 //   launched the plain way: that kernel's wait returns when its predecessor is complete, and a
 //   grid is complete only when its threads have passed their own waits, back to the writer.  In
 //   the decode runner the writer is the previous step's sampling kernel and the kernel in between
-//   is the q/k/v GEMV (pdl_mode 2, 3 or 4) or, from 17 rows on, the plain-launched RMSNorm in
-//   front of the q/k/v GEMM; with pdl_mode 0 or 1 the runner passes false, and so does the
+//   is the q/k/v GEMV (pdl_mode 2, 3 or 4) or, from 17 rows on, the RMSNorm in front of the
+//   q/k/v GEMM, which lets its successor in after its wait; with pdl_mode 0 or 1 the runner passes false, and so does the
 //   builtin, whose caller may have written the positions with the kernel right before.
 int32_t tlc_launch_attention(tlc_ctx *ctx, tlc_kvcache *cache, int layer, const void *q_dev, void *out_dev,
                              int batch, int I, int n_heads, int q_pos0, const int *positions_dev, int max_keys,

@@ -479,7 +479,7 @@ int32_t tlc_launch_gemv(tlc_ctx *ctx, const tlc_gemv_args &a) {
         const __half *x = static_cast<const __half *>(a.x);
         if (a.norm_w) {
             if (int32_t rc = tlc_scratch_reserve(ctx, (size_t)a.m * k * 2)) return rc;
-            if (int32_t rc = tlc_rms_norm(ctx, a.x, a.norm_w, ctx->scratch, a.m, (int32_t)k, a.eps)) return rc;
+            if (int32_t rc = tlc_launch_rms_norm(ctx, a.x, a.norm_w, ctx->scratch, a.m, (int32_t)k, a.eps, true)) return rc;
             x = static_cast<const __half *>(ctx->scratch);
         }
         const int threads = 256;
@@ -519,7 +519,7 @@ int32_t tlc_launch_gemv(tlc_ctx *ctx, const tlc_gemv_args &a) {
         const __half *x = static_cast<const __half *>(a.x);
         if (a.norm_w) {
             if (int32_t rc = tlc_scratch_reserve(ctx, (size_t)a.m * k * 2)) return rc;
-            if (int32_t rc = tlc_rms_norm(ctx, a.x, a.norm_w, ctx->scratch, a.m, (int32_t)k, a.eps)) return rc;
+            if (int32_t rc = tlc_launch_rms_norm(ctx, a.x, a.norm_w, ctx->scratch, a.m, (int32_t)k, a.eps, true)) return rc;
             x = static_cast<const __half *>(ctx->scratch);
         }
         TLC_REQUIRE(((uintptr_t)x & 15) == 0, TLC_ERR_INVALID_OPERATION, "linear: activations must be 16-byte aligned");

@@ -217,6 +217,11 @@ __device__ __forceinline__ void tlc_pdl_prologue() {
 
 // ---- launchers implemented in the kernel translation units ----------------
 
+// y = rms_norm(x) of `rows` rows.  w_early: no kernel in flight writes the weights, which may then be read before
+// the dependency wait (the tensors of a model, not those of a program).
+int32_t tlc_launch_rms_norm(tlc_ctx *ctx, const void *x_dev, const void *w_dev, void *y_dev, int32_t rows, int32_t d, float eps,
+                            bool w_early);
+
 // One weight of a fused multi-GEMV launch.
 struct tlc_gemv_out {
     const tlc_qtensor *w;

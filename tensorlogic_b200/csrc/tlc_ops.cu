@@ -12,59 +12,75 @@
 namespace {
 
 // rms_norm_f16 (shaders/unified.metal:1785-1831) / Tensor::rms_norm_cpu
-// (src/ops/normalization.rs:199-248): one CTA per row.
-__global__ void rms_norm_kernel(const __half *__restrict__ x, const __half *__restrict__ w,
-                                __half *__restrict__ y, int d, float eps) {
-    tlc_pdl_after_wait();
-    __shared__ float warp_sums[32];
-    __shared__ float inv_s;
+// (src/ops/normalization.rs:199-248): one CTA per row.  A launch of a few rows is a chain of latencies: the row is
+// read once, a thread keeps its pieces, and the weights come with it, or before it where the caller vouches
+// that no kernel in flight writes them (w_early): 32 x 4096 3.4 -> 2.3 us.
+__global__ void __launch_bounds__(256) rms_norm_kernel(const __half *__restrict__ x, const __half *__restrict__ w,
+                                                       __half *__restrict__ y, int d, float eps, int w_early) {
+    constexpr int KEEP = 4;  // 16-byte pieces of the row a thread keeps: d = 8192
+    __shared__ float warp_sums[8];
+    const int tid = threadIdx.x, pieces = d >> 3;
     const __half *xr = x + (size_t)blockIdx.x * d;
     __half *yr = y + (size_t)blockIdx.x * d;
     // 16-byte accesses when the row allows it (d a multiple of 8, 16-byte aligned pointers)
     const bool vec = (d & 7) == 0 && ((((uintptr_t)x | (uintptr_t)w | (uintptr_t)y) & 15) == 0);
-    float sq = 0.f;
-    if (vec) {
-        for (int i = threadIdx.x; i < (d >> 3); i += blockDim.x) {
-            const uint4 raw = reinterpret_cast<const uint4 *>(xr)[i];
-            const __half2 *h = reinterpret_cast<const __half2 *>(&raw);
+    uint4 xv[KEEP], wv[KEEP];
+    auto load = [&](const __half *src, uint4 (&v)[KEEP]) {
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const float2 v = __half22float2(h[j]);
-                sq = fmaf(v.x, v.x, sq);
-                sq = fmaf(v.y, v.y, sq);
-            }
+        for (int r = 0; r < KEEP; r++) {
+            const int i = tid + r * 256;
+            v[r] = i < pieces ? reinterpret_cast<const uint4 *>(src)[i] : make_uint4(0, 0, 0, 0);
         }
+    };
+    if (vec && w_early) load(w, wv);
+    tlc_pdl_after_wait();
+    float sq = 0.f;
+    auto add = [&](const uint4 &raw) {
+        const __half2 *h = reinterpret_cast<const __half2 *>(&raw);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const float2 v = __half22float2(h[j]);
+            sq = fmaf(v.x, v.x, sq);
+            sq = fmaf(v.y, v.y, sq);
+        }
+    };
+    if (vec) {
+        load(xr, xv);
+        if (!w_early) load(w, wv);
+#pragma unroll
+        for (int r = 0; r < KEEP; r++) add(xv[r]);
+        for (int i = tid + KEEP * 256; i < pieces; i += 256) add(reinterpret_cast<const uint4 *>(xr)[i]);
     } else {
-        for (int i = threadIdx.x; i < d; i += blockDim.x) {
-            float v = __half2float(xr[i]);
+        for (int i = tid; i < d; i += 256) {
+            const float v = __half2float(xr[i]);
             sq = fmaf(v, v, sq);
         }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-    if ((threadIdx.x & 31) == 0) warp_sums[threadIdx.x >> 5] = sq;
+    if ((tid & 31) == 0) warp_sums[tid >> 5] = sq;
     __syncthreads();
-    if (threadIdx.x < 32) {
-        float v = threadIdx.x < (blockDim.x >> 5) ? warp_sums[threadIdx.x] : 0.f;
+    // (in the order of a shuffle tree over the eight sums)
+    const float *s = warp_sums;
+    const float total = ((s[0] + s[4]) + (s[2] + s[6])) + ((s[1] + s[5]) + (s[3] + s[7]));
+    const float inv = 1.0f / sqrtf(total / (float)d + eps);
+    auto store = [&](int i, const uint4 &raw, const uint4 &wraw) {
+        const __half *xh = reinterpret_cast<const __half *>(&raw), *wh = reinterpret_cast<const __half *>(&wraw);
+        __align__(16) __half o[8];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (threadIdx.x == 0) inv_s = 1.0f / sqrtf(v / (float)d + eps);
-    }
-    __syncthreads();
-    const float inv = inv_s;
+        for (int j = 0; j < 8; j++)
+            o[j] = __float2half_rn(__fmul_rn(__fmul_rn(__half2float(xh[j]), inv), __half2float(wh[j])));
+        reinterpret_cast<uint4 *>(yr)[i] = *reinterpret_cast<const uint4 *>(o);
+    };
     if (vec) {
-        for (int i = threadIdx.x; i < (d >> 3); i += blockDim.x) {
-            const uint4 raw = reinterpret_cast<const uint4 *>(xr)[i], wraw = reinterpret_cast<const uint4 *>(w)[i];
-            const __half *xh = reinterpret_cast<const __half *>(&raw), *wh = reinterpret_cast<const __half *>(&wraw);
-            __align__(16) __half o[8];
 #pragma unroll
-            for (int j = 0; j < 8; j++)
-                o[j] = __float2half_rn(__fmul_rn(__fmul_rn(__half2float(xh[j]), inv), __half2float(wh[j])));
-            reinterpret_cast<uint4 *>(yr)[i] = *reinterpret_cast<const uint4 *>(o);
-        }
+        for (int r = 0; r < KEEP; r++)
+            if (tid + r * 256 < pieces) store(tid + r * 256, xv[r], wv[r]);
+        for (int i = tid + KEEP * 256; i < pieces; i += 256)
+            store(i, reinterpret_cast<const uint4 *>(xr)[i], reinterpret_cast<const uint4 *>(w)[i]);
     } else {
-        for (int i = threadIdx.x; i < d; i += blockDim.x) {
-            float nrm = __fmul_rn(__half2float(xr[i]), inv);
+        for (int i = tid; i < d; i += 256) {
+            const float nrm = __fmul_rn(__half2float(xr[i]), inv);
             yr[i] = __float2half_rn(__fmul_rn(nrm, __half2float(w[i])));
         }
     }
@@ -219,6 +235,12 @@ inline unsigned blocks_for(size_t n, int threads) { return (unsigned)((n + threa
 
 }  // namespace
 
+int32_t tlc_launch_rms_norm(tlc_ctx *ctx, const void *x_dev, const void *w_dev, void *y_dev, int32_t rows, int32_t d, float eps,
+                            bool w_early) {
+    return launch_op(ctx, rms_norm_kernel, rows, 256, static_cast<const __half *>(x_dev), static_cast<const __half *>(w_dev),
+                     static_cast<__half *>(y_dev), d, eps, w_early ? 1 : 0);
+}
+
 extern "C" int32_t tlc_rms_norm(tlc_ctx *ctx, const void *x_dev, const void *w_dev, void *y_dev, int32_t rows,
                                 int32_t d, float eps) {
     if (int32_t rc = tlc_enter(ctx)) return rc;
@@ -226,9 +248,7 @@ extern "C" int32_t tlc_rms_norm(tlc_ctx *ctx, const void *x_dev, const void *w_d
     TLC_REQUIRE(x_dev && w_dev && y_dev, TLC_ERR_INVALID_OPERATION, "rms_norm: null pointer");
     TLC_REQUIRE(rows >= 0 && d > 0, TLC_ERR_INVALID_DIMENSION, "rms_norm: bad shape [%d, %d]", rows, d);
     if (rows == 0) return TLC_OK;
-    return launch_op(ctx, rms_norm_kernel, rows, 256, static_cast<const __half *>(x_dev),
-                                                   static_cast<const __half *>(w_dev),
-                                                   static_cast<__half *>(y_dev), d, eps);
+    return tlc_launch_rms_norm(ctx, x_dev, w_dev, y_dev, rows, d, eps, false);
 }
 
 extern "C" int32_t tlc_rope(tlc_ctx *ctx, const void *x_dev, void *y_dev, int32_t seq, int32_t heads,
