@@ -626,7 +626,7 @@ static int32_t forward(tlc_llama *L, int m, bool decode, int pos0, bool all_logi
             // positions[] is written by the previous step's sampling kernel (or by set_state / prefill);
             // the embedding gather and the q/k/v kernels lie between it and this launch.  The q/k/v GEMV
             // lets its successor in only after its own dependency wait (pdl_mode 2 and up), and the
-            // q/k/v GEMM of 17 rows and more comes behind a plain-launched RMSNorm: either way the
+            // q/k/v GEMM of 17 rows and more, like the RMSNorm in front of it, does so too: either way the
             // positions are final before this kernel can be scheduled
             if (int32_t rc = tlc_launch_attention(ctx, L->cache, l, L->q, L->attn, decode ? m : 1, decode ? 1 : m,
                                                   L->heads_local, pos0, positions, c.max_seq, scale,
@@ -915,7 +915,7 @@ extern "C" int32_t tlc_llama_decode_host(tlc_llama *L, int32_t batch, const int3
         next_ids_host[0] = L->host_next[0];
         return TLC_OK;
     }
-    if (ids_host && !logits_host && !L->cfg.no_graph && L->ctx->host_graph) {
+    if (ids_host && !L->cfg.no_graph && L->ctx->host_graph) {
         // The common call: token ids up, one step, sampled ids and the status word down --
         // all of it one graph (copy nodes around the step's kernels), one launch, one wait.
         tlc_ctx *ctx = L->ctx;
@@ -955,7 +955,15 @@ extern "C" int32_t tlc_llama_decode_host(tlc_llama *L, int32_t batch, const int3
         TLC_CUDA(cudaGraphLaunch(L->graph[key], ctx->stream));
         ctx->launches += (uint64_t)L->launches_in[7];
         bool seen = false;
-        if (ctx->host_poll) {
+        if (logits_host) {
+            // The caller's buffer is usually fresh memory: its pages are brought in while the GPU is busy,
+            // which the copy would otherwise wait for one by one (32 x 32000 values: 1.0 ms after a step of 3.2 ms, now 0.22).
+            const size_t bytes = (size_t)batch * L->cfg.vocab * 2;
+            volatile char *c = static_cast<char *>(logits_host);
+            for (size_t i = 0; i < bytes; i += 4096) c[i] = 0;
+            c[bytes - 1] = 0;
+            if (int32_t rc = copy_logits(L, logits_host, batch)) return rc;
+        } else if (ctx->host_poll) {
             // Watch the pinned words the last copy node writes; after 50 ms without them
             // (an error, a very long step) fall back to the stream synchronize below.
             const auto t0 = std::chrono::steady_clock::now();
