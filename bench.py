@@ -417,7 +417,7 @@ def run_ours(args, rank: int, world: int, local: int) -> None:
         assert llm.launches(1) == gemv_launches, (llm.launches(1), gemv_launches)
         kernel_us = g0.elapsed_time(g1) * 1e3 / (K * gemv_launches)
         bytes_per_launch = gemv_bytes / gemv_launches
-        kernel_name = "gemv_mma_kernel<Q4_0> (fused dequant-GEMV, M=1)"
+        kernel_name = "gemv_row1_kernel<Q4_0> (fused dequant-GEMV, M=1)"
         kernel_launches_per_step = gemv_launches
         traffic, traffic_src = profiled_traffic("tinyllama_decode_gemv")
     achieved = bytes_per_launch / (kernel_us * 1e-6) / 1e9
@@ -620,7 +620,7 @@ def run_tp(args, rank: int, world: int, local: int) -> None:
                 "d2h_bytes_per_step": 4 * batch, "ms_per_step": e2e_ms / K},
         "gpu_launches": int(gpu_launches),
         "clocks": clocks.summary(),
-        "roofline": {"bound": "hbm", "kernel": "gemv_mma_kernel<Q4_0> (per-rank shard" +
+        "roofline": {"bound": "hbm", "kernel": ("gemv_row1_kernel" if batch == 1 else "gemv_mma_kernel") + "<Q4_0> (per-rank shard" +
                      ("; the time includes the collectives interleaved with the GEMV launches)" if world > 1 else ")"),
                      "achieved": achieved, "peak": peak,
                      "peak_source": peak_src, "unit": "GB/s", "frac": achieved / peak,
