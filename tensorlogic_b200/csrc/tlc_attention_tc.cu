@@ -49,6 +49,7 @@ struct FlashParams {
     __half *out;
     int I, H, Hkv, G;
     int q_tiles, batch;
+    int splits;  // CTAs (of one cluster) that share a tile's keys
     int pos0;
     float scale;
     tlc_dev_status *status;
@@ -101,6 +102,17 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
         : "memory");
 }
 
+static_assert(kRows * (64 + 2) * 4 <= kRows * 64 * 2 + 2 * stages<64>() * kv_bytes<64>() &&
+                  kRows * (128 + 2) * 4 <= kRows * 128 * 2 + 2 * stages<128>() * kv_bytes<128>(),
+              "the merge takes the place of Q, K and V");
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void st_cluster(uint32_t at, uint32_t v) {
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(at), "r"(v) : "memory");
+}
+
 template <int D>
 __global__ void __launch_bounds__(kThreads, 2)
     attention_tc_kernel(const __grid_constant__ FlashParams p, const __grid_constant__ CUtensorMap q_map,
@@ -142,11 +154,14 @@ __global__ void __launch_bounds__(kThreads, 2)
     const uint32_t tmem = *tmem_slot;
 
     // The last queries of a sequence see the most keys: their tiles go first.
-    const int per = p.Hkv * p.batch, hb = blockIdx.x % per, qt = p.q_tiles - 1 - blockIdx.x / per;
+    const int split = blockIdx.x % p.splits, cta = blockIdx.x / p.splits;
+    const int per = p.Hkv * p.batch, hb = cta % per, qt = p.q_tiles - 1 - cta / per;
     const int hk = hb % p.Hkv, b = hb / p.Hkv;
     const int G = p.G, RQ = kRows / G;
     const int k_end = p.pos0 + min(p.I, (qt + 1) * RQ);
-    const int n = (k_end + kKeys - 1) / kKeys;
+    // key tiles of this CTA: [t0, t0 + n)
+    const int tiles = (k_end + kKeys - 1) / kKeys, share = (tiles + p.splits - 1) / p.splits, t0 = split * share;
+    const int n = max(0, min(tiles - t0, share));
 
     if (warp == 0) {
         // ------------------------------ Q, K, V ------------------------------
@@ -155,14 +170,14 @@ __global__ void __launch_bounds__(kThreads, 2)
         asm volatile("griddepcontrol.wait;" ::: "memory");
         const uint32_t el = elect_one();
         const uint32_t bar_q = smem_u32(q_full);
-        mbar_arrive_expect_tx_el(q_full, kRows * D * 2, el);
+        if (n > 0) mbar_arrive_expect_tx_el(q_full, kRows * D * 2, el);
 #pragma unroll
         for (int h = 0; h < HALVES; h++)
-            tma_load_3d_el(smem_u32(qs + h * kRows * 128), &q_map, 64 * h, hk * G, b * p.I + qt * RQ, bar_q, el);
+            if (n > 0) tma_load_3d_el(smem_u32(qs + h * kRows * 128), &q_map, 64 * h, hk * G, b * p.I + qt * RQ, bar_q, el);
         bool ok = true;
         int sk = 0, sv = 0;
         uint32_t pk = 1, pv = 1;
-        for (int j = 0; ok && j <= n; j++) {  // K of tile j, V of tile j - 1: the order in which they are used
+        for (int j = 0; ok && n > 0 && j <= n; j++) {  // K of tile j, V of tile j - 1: the order in which they are used
             if (j < n) {
                 ok = __all_sync(0xffffffffu, mbar_wait(&k_empty[sk], pk, abort_flag, p.status, 41, p.wait_ns));
                 if (!ok) break;
@@ -170,7 +185,7 @@ __global__ void __launch_bounds__(kThreads, 2)
                 mbar_arrive_expect_tx_el(&k_full[sk], KV, el);
 #pragma unroll
                 for (int h = 0; h < HALVES; h++)
-                    tma_load_4d_el(smem_u32(ks + sk * KV + h * kHalf), &k_map, 64 * h, hk, j * kKeys, b, bar, el);
+                    tma_load_4d_el(smem_u32(ks + sk * KV + h * kHalf), &k_map, 64 * h, hk, (t0 + j) * kKeys, b, bar, el);
                 if (++sk == ST) sk = 0, pk ^= 1u;
             }
             if (j > 0) {
@@ -180,7 +195,7 @@ __global__ void __launch_bounds__(kThreads, 2)
                 mbar_arrive_expect_tx_el(&v_full[sv], KV, el);
 #pragma unroll
                 for (int h = 0; h < HALVES; h++)
-                    tma_load_4d_el(smem_u32(vs + sv * KV + h * kHalf), &v_map, 64 * h, hk, (j - 1) * kKeys, b, bar, el);
+                    tma_load_4d_el(smem_u32(vs + sv * KV + h * kHalf), &v_map, 64 * h, hk, (t0 + j - 1) * kKeys, b, bar, el);
                 if (++sv == ST) sv = 0, pv ^= 1u;
             }
         }
@@ -191,7 +206,7 @@ __global__ void __launch_bounds__(kThreads, 2)
         const uint32_t idesc_s = idesc_for(kKeys), idesc_o = idesc_for(D) | 1u << 16;  // (V: N-major)
         constexpr uint32_t MN = (uint32_t)(kHalf >> 4) << 16;  // the next 64 values of d: the next box
         const uint32_t q0 = (smem_u32(qs) & 0x3FFFF) >> 4, k0 = (smem_u32(ks) & 0x3FFFF) >> 4, v0 = (smem_u32(vs) & 0x3FFFF) >> 4;
-        bool ok = mbar_wait(q_full, 0, abort_flag, p.status, 43, p.wait_ns);
+        bool ok = n > 0 && mbar_wait(q_full, 0, abort_flag, p.status, 43, p.wait_ns);
         int sk = 0, sv = 0;
         uint32_t pk = 0, pv = 0;
         auto scores = [&](int j) {  // S of tile j
@@ -211,7 +226,7 @@ __global__ void __launch_bounds__(kThreads, 2)
             umma_commit(&s_full[j & 1], el);
             if (++sk == ST) sk = 0, pk ^= 1u;
         };
-        scores(0);
+        if (n > 0) scores(0);
         for (int j = 0; j < n; j++) {
             if (j + 1 < n) scores(j + 1);
             ok = mbar_wait(&v_full[sv], pv, abort_flag, p.status, 46, p.wait_ns) && ok;
@@ -243,7 +258,7 @@ __global__ void __launch_bounds__(kThreads, 2)
         // The row's sum in four parts (pairs of keys in turn), each in the order of the keys.
         float m_run = -INFINITY, l_run[4] = {0.f, 0.f, 0.f, 0.f};
         for (int j = 0; j < n; j++) {
-            const int j0 = j * kKeys;
+            const int j0 = (t0 + j) * kKeys;
             const uint32_t ts = tl + (j & 1) * kKeys;
             mbar_wait(&s_full[j & 1], (uint32_t)(j >> 1) & 1u, abort_flag, p.status, 48, p.wait_ns);
             __syncwarp();
@@ -328,31 +343,94 @@ __global__ void __launch_bounds__(kThreads, 2)
             __syncwarp();
             if (lane == 0) mbar_arrive(&p_full[j & 1]);
         }
-        const bool ok = mbar_wait(&pv_done[(n - 1) & 1], (uint32_t)((n - 1) >> 1) & 1u, abort_flag, p.status, 50, p.wait_ns);
+        const bool ok = n == 0 || mbar_wait(&pv_done[(n - 1) & 1], (uint32_t)((n - 1) >> 1) & 1u, abort_flag, p.status, 50, p.wait_ns);
         __syncwarp();
         tc_fence_after();
-        const float l = (l_run[0] + l_run[1]) + (l_run[2] + l_run[3]), inv = l > 0.f ? 1.0f / l : 0.f;
-        __half *out = p.out + ((size_t)(b * (size_t)p.I + qi) * p.H + head) * D;
+        const float l = (l_run[0] + l_run[1]) + (l_run[2] + l_run[3]);
+        if (p.splits == 1) {
+            const float inv = l > 0.f ? 1.0f / l : 0.f;
+            __half *out = p.out + ((size_t)(b * (size_t)p.I + qi) * p.H + head) * D;
 #pragma unroll
-        for (int c = 0; c < D; c += 64) {
-            uint32_t o[2][32];
-            tmem_ld32_issue(tl + kColO + c, o[0]);
-            tmem_ld32_issue(tl + kColO + c + 32, o[1]);
-            tmem_ld_wait(o[0], o[1]);
-            if (ok && qi < p.I) {
+            for (int c = 0; c < D; c += 64) {
+                uint32_t o[2][32];
+                tmem_ld32_issue(tl + kColO + c, o[0]);
+                tmem_ld32_issue(tl + kColO + c + 32, o[1]);
+                tmem_ld_wait(o[0], o[1]);
+                if (ok && qi < p.I) {
 #pragma unroll
-                for (int e = 0; e < 64; e += 8) {
-                    __align__(16) __half2 h[4];
+                    for (int e = 0; e < 64; e += 8) {
+                        __align__(16) __half2 h[4];
 #pragma unroll
-                    for (int i = 0; i < 8; i += 2)
-                        h[i / 2] = __floats2half2_rn(__uint_as_float(o[e / 32][e % 32 + i]) * inv,
-                                                     __uint_as_float(o[e / 32][e % 32 + i + 1]) * inv);
-                    *reinterpret_cast<uint4 *>(out + c + e) = *reinterpret_cast<const uint4 *>(h);
+                        for (int i = 0; i < 8; i += 2)
+                            h[i / 2] = __floats2half2_rn(__uint_as_float(o[e / 32][e % 32 + i]) * inv,
+                                                         __uint_as_float(o[e / 32][e % 32 + i + 1]) * inv);
+                        *reinterpret_cast<uint4 *>(out + c + e) = *reinterpret_cast<const uint4 *>(h);
+                    }
+                }
+                __syncwarp();
+            }
+        } else {
+            // The CTAs of the cluster are done with their tiles, whose place now takes what the owner of a row
+            // adds up: [split][O, maximum, sum][row], so that the rows of a warp lie side by side.
+            cluster_barrier();
+            const int own = kRows / p.splits, owner = r / own, pitch = (D + 2) * own;
+            uint32_t to;
+            asm("mapa.shared::cluster.u32 %0, %1, %2;"
+                : "=r"(to)
+                : "r"(smem_u32(qs) + (uint32_t)(split * pitch + r - owner * own) * 4), "r"(owner));
+            st_cluster(to + D * own * 4, n == 0 ? 0xFF800000u : __float_as_uint(m_run));  // (-inf: no keys here)
+            st_cluster(to + (D + 1) * own * 4, __float_as_uint(l));
+            if (n > 0)
+#pragma unroll
+                for (int c = 0; c < D; c += 32) {
+                    uint32_t o[32];
+                    tmem_ld32(tl + kColO + c, o);
+#pragma unroll
+                    for (int e = 0; e < 32; e++) st_cluster(to + (c + e) * own * 4, o[e]);
+                    __syncwarp();
+                }
+            cluster_barrier();
+            // `splits` threads a row, D / splits values each (8 at least)
+            const int row = r % own, mine = split * own + row, d0 = r / own * (D / p.splits);
+            const float *part = reinterpret_cast<const float *>(qs) + row;
+            const int oq = qt * RQ + mine / G;
+            float M = -INFINITY, L = 0.f, w[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+                if (i < p.splits) M = fmaxf(M, part[i * pitch + D * own]);
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                w[i] = 0.f;
+                if (i < p.splits) {
+                    const float mi = part[i * pitch + D * own];
+                    if (mi > -INFINITY) w[i] = expf(mi - M);
+                    L += part[i * pitch + (D + 1) * own] * w[i];
                 }
             }
-            __syncwarp();
+            const float inv = L > 0.f ? 1.0f / L : 0.f;
+            __half *out = p.out + ((size_t)(b * (size_t)p.I + oq) * p.H + hk * G + mine % G) * D + d0;
+            for (int d = 0; d < D / p.splits; d += 8) {
+                float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+                    if (i < p.splits && w[i] > 0.f)  // (a split without keys has stored no O)
+#pragma unroll
+                        for (int e = 0; e < 8; e++) acc[e] += part[i * pitch + (d0 + d + e) * own] * w[i];
+                if (ok && oq < p.I) {
+                    __align__(16) __half2 h[4];
+#pragma unroll
+                    for (int e = 0; e < 4; e++) h[e] = __floats2half2_rn(acc[2 * e] * inv, acc[2 * e + 1] * inv);
+                    *reinterpret_cast<uint4 *>(out + d) = *reinterpret_cast<const uint4 *>(h);
+                }
+            }
         }
+        __syncwarp();
         tc_fence_before();
+    }
+    if (p.splits > 1 && warp < 2) {  // (every thread of the cluster takes part in its two barriers)
+        __syncwarp();
+        cluster_barrier();
+        cluster_barrier();
     }
     __syncthreads();
     if (warp == 1) {
@@ -370,8 +448,26 @@ int32_t launch(tlc_ctx *ctx, const FlashParams &p, const CUtensorMap &q, const C
                                       cudaSharedmemCarveoutMaxShared));
         configured[ctx->device & 63] = true;
     }
-    const dim3 grid((unsigned)(p.q_tiles * p.Hkv * p.batch));
-    const cudaError_t le = tlc_launch_pdl(ctx, attention_tc_kernel<D>, grid, dim3(kThreads), smem_bytes_tc<D>(), p, q, k, v);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(p.q_tiles * p.Hkv * p.batch * p.splits));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem_bytes_tc<D>();
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[2];
+    int na = 0;
+    if (p.splits > 1) {
+        attr[na].id = cudaLaunchAttributeClusterDimension;
+        attr[na].val.clusterDim.x = (unsigned)p.splits;
+        attr[na].val.clusterDim.y = 1;
+        attr[na++].val.clusterDim.z = 1;
+    }
+    if (ctx->use_pdl && ctx->pdl_small) {
+        attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[na++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = na;
+    const cudaError_t le = cudaLaunchKernelEx(&cfg, attention_tc_kernel<D>, p, q, k, v);
     if (le != cudaSuccess) {
         cudaGetLastError();
         return tlc_fail(TLC_ERR_CUDA, "attention launch failed: %s", cudaGetErrorString(le));
@@ -404,6 +500,22 @@ int32_t tlc_launch_attention_tc(tlc_ctx *ctx, const AttnTc &a) {
     p.q_tiles = (a.I + kRows / p.G - 1) / (kRows / p.G);
     p.batch = a.batch;
     p.pos0 = a.pos0;
+    // A short prompt behind a long context has few tiles of rows, each with many keys: the keys are shared out over
+    // the CTAs of a cluster, up to two CTAs an SM, by the microseconds of a CTA's key tiles, of the merge (3 to 5) and
+    // of what the next kernel's CTAs lose, which would have fetched weights on the idle SMs (4).  32 heads over 4 KV
+    // heads of 64: 32 tokens after 1000 20.7 us, 8 splits 10.1; 300 after 1000 28.2, 2 splits 22.6; 32 heads of 128, 128
+    // tokens after 1900 42.0, now 18.5.  TinyLlama, 20 tokens after 1500: 1.65 -> 1.35 ms; 77 after 391, where the kernel
+    // alone gains 2 us from 8 splits, the same.
+    const int ctas = p.q_tiles * p.Hkv * p.batch, tiles = (a.pos0 + a.I + kKeys - 1) / kKeys;
+    p.splits = 1;
+    double best = tiles * 0.95;
+    for (int s = 2; s <= 8 && ctas * s <= 2 * ctx->sm_count; s *= 2) {
+        const double t = (tiles + s - 1) / s * (ctas * s > ctx->sm_count ? 1.2 : 0.95) + (a.D == 64 ? 7.2 : 8.7);
+        if (t < best) {
+            best = t;
+            p.splits = s;
+        }
+    }
     p.scale = a.scale;
     p.status = ctx->dev_status;
     p.wait_ns = ctx->wait_ns;

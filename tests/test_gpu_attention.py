@@ -192,3 +192,29 @@ def test_prefill_attention_tile_edges(dev, ref, H, Hkv, D, B, I, pos0, rise):
         got = out.numpy().reshape(B, I, H, D)
         for b, (qb, k, v) in enumerate(seqs):
             assert rel_l2(got[b], ref.attention(qb, k, v, scale, q_pos0=pos0)) < TIGHT, (ptr, b)
+
+
+@pytest.mark.parametrize("H,Hkv,D", [(32, 4, 64), (8, 1, 128), (4, 4, 128)])
+@pytest.mark.parametrize("B,I,pos0", [(1, 2, 700), (1, 77, 391), (2, 33, 575), (1, 129, 1500), (1, 300, 1000)])
+def test_prefill_attention_split_keys(dev, ref, H, Hkv, D, B, I, pos0):
+    """A short prompt behind a long context: two to eight CTAs share the keys of a tile."""
+    import ctypes as C
+    from tensorlogic_b200._lib import check
+    from tensorlogic_b200.api import KVCache
+    if I == 300 and D == 128:
+        pytest.skip("covered by the 64-wide case; keeps the CPU oracle time down")
+    T, cap, row, scale = pos0 + I, pos0 + I + 3, Hkv * D, 1.0 / np.sqrt(D)
+    cache = KVCache(dev, 1, Hkv, D, max_seq=cap, max_batch=B)
+    kptr, vptr = C.c_void_p(), C.c_void_p()
+    check(dev.lib.tlc_kvcache_layer_ptrs(cache.handle, 0, C.byref(kptr), C.byref(vptr)))
+    seqs = [_qkv(I + 5 * b, I, T, H, Hkv, D) for b in range(B)]
+    for b, (q, k, v) in enumerate(seqs):
+        check(dev.lib.tlc_upload(dev.handle, kptr.value + b * cap * row * 2, k.ctypes.data, T * row * 2))
+        check(dev.lib.tlc_upload(dev.handle, vptr.value + b * cap * row * 2, v.ctypes.data, T * row * 2))
+    dev.synchronize()
+    q0 = dev.tensor(np.concatenate([s[0].ravel() for s in seqs]))
+    out = dev.tensor(np.zeros(B * I * H * D, np.float16))
+    check(dev.lib.tlc_attention(dev.handle, cache.handle, 0, q0.ptr, out.ptr, B, I, H, pos0, None, 0, scale))
+    got = out.numpy().reshape(B, I, H, D)
+    for b, (qb, k, v) in enumerate(seqs):
+        assert rel_l2(got[b], ref.attention(qb, k, v, scale, q_pos0=pos0)) < TIGHT, b
