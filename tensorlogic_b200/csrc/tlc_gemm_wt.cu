@@ -969,7 +969,9 @@ int32_t tlc_launch_gemm_wt(tlc_ctx *ctx, const tlc_gemv_args &a) {
     p.rope_base = (float)a.rope_base;
     p.status = ctx->dev_status;
     p.wait_ns = ctx->wait_ns;
-    const Plan plan = q4 ? choose_plan<kWtQ4>(ctx, a.m, tiles, p.steps, 0.3) : choose_plan<kWtQ8>(ctx, a.m, tiles, p.steps, 0.3);
+    // 0.42 us a K step is what the unpacking takes with all groups busy, 0.5 with the hand-overs of a short share (at 0.3
+    // the plans had too many small tiles: 11008 x 4096, 128 rows 30.3 us, now 23.3; 2048 x 5632, 512 rows 25.7, now 19.0)
+    const Plan plan = q4 ? choose_plan<kWtQ4>(ctx, a.m, tiles, p.steps, 0.5) : choose_plan<kWtQ8>(ctx, a.m, tiles, p.steps, 0.5);
     CUtensorMap x_map;
     WtMaps w_maps;
     memset(&w_maps, 0, sizeof w_maps);
