@@ -60,8 +60,8 @@ struct AttnParams {
     int push_offset; // cluster mode: byte offset of the merge area in dynamic shared memory
     int cluster;     // 1: the nsplit CTAs of a tile form a thread-block cluster and merge through
                      // distributed shared memory instead of global scratch
-    int pos_settled; // 1: the launcher vouches that positions[] was final before this kernel could start
-                     // (see tlc_launch_attention); the kernel then reads it once, before the wait
+    int settled;     // 1: the launcher vouches that positions[] and the cache rows of earlier steps were final before
+                     // this kernel could start (see tlc_launch_attention); they may then be read before the wait
     int key_limit;   // keys the launch was sized for (<= Tmax): a sequence whose position says it
                      // holds more is cut there and the status word (when given) says so
     tlc_dev_status *status;  // device word or null
@@ -123,18 +123,16 @@ __global__ void __launch_bounds__(kAttnThreads) attention_kernel(const AttnParam
     // the group size is a power of two (1 .. 16, checked by the launcher): shifts, not divisions
     const int G = p.G, gsh = 31 - __clz(p.G), RQ = 16 >> gsh;
 
-    // A decode step's query, its newest cache row AND its position come from earlier kernels
-    // of the stream.  Before griddepcontrol.wait the position word may still hold the previous
-    // step's value; positions only grow while kernels are in flight (the host resets them
-    // after a stream synchronize), so that value is a lower bound of the true one.  It is used
-    // for one thing only: a first K/V tile that lies entirely below it holds rows of earlier
-    // steps, whatever the true position turns out to be, and is fetched while the previous
-    // kernel is still running.  k_begin does not depend on the position at all.
+    // The query and the newest cache row come from the kernel in front of this one.  The position and the rows
+    // of earlier steps do so too in a program that calls the builtins one by one; only a launcher that knows
+    // what is in flight (p.settled) lets the kernel read them before griddepcontrol.wait: a first K/V tile that
+    // lies entirely below the position is then fetched while the previous kernel is still running.
+    // k_begin does not depend on the position at all.
     const int k_begin = split * p.keys_per_split;
     const __half *kbase = p.kc + ((size_t)b * p.Tmax * p.Hkv + hk) * D;
     const __half *vbase = p.vc + ((size_t)b * p.Tmax * p.Hkv + hk) * D;
     const size_t key_stride = (size_t)p.Hkv * D;
-    int k_end = 0;  // set below; the early tile is whole, so every key of it passes `< k_end`
+    int k_end = 0;  // set below
     auto load_tile = [&](int tile, int stage) {
         const int j0 = k_begin + tile * kTileKeys;
         constexpr int CHUNKS = kTileKeys * (D / 8);
@@ -155,11 +153,11 @@ __global__ void __launch_bounds__(kAttnThreads) attention_kernel(const AttnParam
     const int last_q = min(p.I, (qt + 1) * RQ) - 1;
     // Everything that depends on the position of query 0.
     int pos0 = 0, rpos_lo = 0, rpos_hi = 0, ntiles = 0;
-    auto derive = [&](int pos_raw, bool final_value) {
-        pos0 = pos_raw < 0 ? 0 : pos_raw;
-        if (pos0 + p.I > p.key_limit) {  // more keys than the launch (or the cache) holds: cut, and say so
+    auto derive = [&]() {
+        pos0 = max(p.positions ? p.positions[b] : p.q_pos0, 0);
+        if (pos0 > p.key_limit - p.I) {  // more keys than the launch (or the cache) holds: cut, and say so
             pos0 = p.key_limit - p.I;
-            if (final_value && p.status && tid == 0 && atomicCAS(&p.status->code, 0, TLC_DEV_INDEX) == 0)
+            if (p.status && tid == 0 && atomicCAS(&p.status->code, 0, TLC_DEV_INDEX) == 0)
                 p.status->where = 200 + b;
         }
         const int T = pos0 + p.I;  // keys in the cache (incl. the new ones)
@@ -170,23 +168,16 @@ __global__ void __launch_bounds__(kAttnThreads) attention_kernel(const AttnParam
         k_end = min(visible_end, k_begin + p.keys_per_split);
         ntiles = k_end > k_begin ? (k_end - k_begin + kTileKeys - 1) / kTileKeys : 0;
     };
-    // A launch argument is final; a device word is final before the wait only if the launcher vouches
-    // for it (tlc_launch_attention).  Then all of the above is worked out while the previous kernel
-    // still runs; otherwise the word is a lower bound, good for the early tile only, and is read
-    // again after the wait (an L2 round trip on the critical path of the layer).
-    const bool settled = !p.positions || p.pos_settled;
-    const int pos_seen = p.positions ? *reinterpret_cast<const volatile int *>(p.positions + b) : p.q_pos0;
-    derive(pos_seen, settled);
-    const bool early = p.I == 1 && ntiles > 0 && k_begin + kTileKeys <= pos0;
-    if (early) {
-        if (!settled) k_end = k_begin + kTileKeys;  // the tile is whole whatever the final position is
-        load_tile(0, 0);
-    }
+    // (Worked out while the previous kernel still runs, where that is allowed: the position is an L2 round trip.)
+    const bool known = p.settled || !p.positions;
+    if (known) derive();
+    const bool early = p.settled && p.I == 1 && ntiles > 0 && k_begin + kTileKeys <= pos0;
+    if (early) load_tile(0, 0);
     asm volatile("griddepcontrol.wait;" ::: "memory");
     // The next kernel of the stream (a GEMV: its producer warp streams weights, the rest waits) may be
     // scheduled from here on; letting it in before this wait was 0.2 % slower on the decode step.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    if (!settled) derive(*reinterpret_cast<const volatile int *>(p.positions + b), true);
+    if (!known) derive();
 
     // Q fragments (A operand), straight from global memory.
     uint32_t qa[KSTEPS][4];
@@ -541,19 +532,19 @@ static int cluster_splits(const tlc_ctx *ctx, int groups, int tiles, int D) {
 //   batch sequences, I queries each (I == 1 when positions_dev is given).
 //   nsplit_hint <= 0: choose from the key count; with positions_dev the key
 //   count is only known on the device, so max_keys bounds it.
-//   positions_settled: the caller vouches that positions_dev[] is final before this kernel can
-//   be scheduled, not merely before its dependency wait returns.  A kernel can be scheduled once
-//   every CTA of its predecessor has let dependents in, so this holds when some kernel between
-//   the writer of the positions and this one does that only after its own dependency wait, or is
-//   launched the plain way: that kernel's wait returns when its predecessor is complete, and a
-//   grid is complete only when its threads have passed their own waits, back to the writer.  In
-//   the decode runner the writer is the previous step's sampling kernel and the kernel in between
-//   is the q/k/v GEMV (pdl_mode 2, 3 or 4) or, from 17 rows on, the RMSNorm in front of the
-//   q/k/v GEMM, which lets its successor in after its wait; with pdl_mode 0 or 1 the runner passes false, and so does the
-//   builtin, whose caller may have written the positions with the kernel right before.
+//   settled: the caller vouches that positions_dev[] and the cache rows below the newest one are final
+//   before this kernel can be scheduled, not merely before its dependency wait returns.  A kernel can
+//   be scheduled once every CTA of its predecessor has let dependents in, so this holds when some kernel
+//   between their writers and this one does that only after its own dependency wait, or is launched the plain
+//   way: that kernel's wait returns when its predecessor is complete, and a grid is complete only when
+//   its threads have passed their own waits, back to the writers.  In the decode runner the writers are
+//   the previous step's sampling and q/k/v kernels (or a prompt's), and the kernel in between is this step's q/k/v
+//   GEMV (pdl_mode 2, 3 or 4) or, from two rows on, the RMSNorm in front of it, which lets its successor in
+//   after its wait; with pdl_mode 0 or 1 the runner passes false, and so does the builtin, whose caller may have
+//   written positions and rows with the kernel right before (a `cache.append` lets this kernel in before it stores).
 int32_t tlc_launch_attention(tlc_ctx *ctx, tlc_kvcache *cache, int layer, const void *q_dev, void *out_dev,
                              int batch, int I, int n_heads, int q_pos0, const int *positions_dev, int max_keys,
-                             float scale, bool positions_settled) {
+                             float scale, bool settled) {
     TLC_REQUIRE(cache && q_dev && out_dev, TLC_ERR_INVALID_OPERATION, "attention: null pointer");
     TLC_REQUIRE(layer >= 0 && layer < cache->n_layers, TLC_ERR_INDEX, "Index out of bounds: index %d, size %d",
                 layer, cache->n_layers);
@@ -585,7 +576,7 @@ int32_t tlc_launch_attention(tlc_ctx *ctx, tlc_kvcache *cache, int layer, const 
     p.q_pos0 = q_pos0;
     p.positions = positions_dev;
     p.scale = scale;
-    p.pos_settled = positions_settled ? 1 : 0;
+    p.settled = settled ? 1 : 0;
     p.key_limit = T;  // <= max_seq (checked above); a position beyond it is cut on the device
     p.status = ctx->dev_status;
     if (I > 1) {  // prefill: the tcgen05 kernel; attention_kernel serves addresses TMA cannot take

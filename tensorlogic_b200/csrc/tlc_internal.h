@@ -277,4 +277,4 @@ size_t tlc_gemv_scratch_bytes(int64_t k);
 struct tlc_kvcache;
 int32_t tlc_launch_attention(tlc_ctx *ctx, tlc_kvcache *cache, int layer, const void *q_dev, void *out_dev,
                              int batch, int n_queries, int n_heads, int q_pos0, const int *positions_dev,
-                             int max_keys, float scale, bool positions_settled);
+                             int max_keys, float scale, bool settled);

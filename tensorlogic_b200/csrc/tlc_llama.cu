@@ -623,14 +623,14 @@ static int32_t forward(tlc_llama *L, int m, bool decode, int pos0, bool all_logi
             if (int32_t rc = tlc_launch_gemv(ctx, a)) return rc;
         }
         if (parts & 2)
-            // positions[] is written by the previous step's sampling kernel (or by set_state / prefill);
-            // the embedding gather and the q/k/v kernels lie between it and this launch.  The q/k/v GEMV
-            // lets its successor in only after its own dependency wait (pdl_mode 2 and up), and the
-            // q/k/v GEMM of 17 rows and more, like the RMSNorm in front of it, does so too: either way the
-            // positions are final before this kernel can be scheduled
+            // positions[] is written by the previous step's sampling kernel (or by set_state / prefill), the cache
+            // rows of earlier steps by their q/k/v kernels; the embedding gather and this layer's q/k/v kernels
+            // lie between them and this launch (unless `parts` leaves these out).  The q/k/v GEMV lets its
+            // successor in only after its own dependency wait (pdl_mode 2 and up), and so does the RMSNorm in front of
+            // its forms for two and more rows: either way all of it is final before this kernel can be scheduled
             if (int32_t rc = tlc_launch_attention(ctx, L->cache, l, L->q, L->attn, decode ? m : 1, decode ? 1 : m,
                                                   L->heads_local, pos0, positions, c.max_seq, scale,
-                                                  !ctx->use_pdl || ctx->pdl_mode >= 2))
+                                                  (parts & 1) && (!ctx->use_pdl || ctx->pdl_mode >= 2)))
                 return rc;
         if (parts & 1) {
             tlc_gemv_args a;

@@ -1,0 +1,55 @@
+"""The builtins are launched dependent: a kernel may be resident, and past everything it does before its dependency
+wait, while the one in front of it still stores.  What a program has just computed must not be read that early.  Each
+program below is queued behind work that keeps the GPU busy, with all operands on the device (an upload in between
+would order the kernels by itself), and gives the bits that it gives with dependent launch off."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _both(dev, program):
+    """The program's results with dependent launch on and off: lists of arrays."""
+    got = []
+    for pdl in (1, 0):
+        dev.set_option("pdl", pdl)
+        try:
+            got.append([t.numpy() for t in program()])
+        finally:
+            dev.set_option("pdl", 1)
+    return got
+
+
+def _busy(dev):
+    """A few products of some ten microseconds: the host runs ahead of the GPU from here on."""
+    from tensorlogic_b200.api import matmul
+    a = dev.tensor(np.ones((2048, 2048), np.float16))
+
+    def queue():
+        for _ in range(8):
+            matmul(a, a)
+    return queue
+
+
+@pytest.mark.parametrize("H,Hkv,D", [(32, 4, 64), (8, 1, 128), (8, 8, 64)])
+@pytest.mark.parametrize("rows", [100, 640, 2000])
+def test_attention_right_after_append(dev, H, Hkv, D, rows):
+    """One query at the last of the rows that the append in front of it stores: none of them is there before."""
+    from tensorlogic_b200.api import KVCache
+    rng = np.random.default_rng(rows + D)
+    normal = lambda *shape: dev.tensor(rng.standard_normal(shape).astype(np.float16))
+    sets = [(normal(rows, Hkv, D), normal(rows, Hkv, D)) for _ in range(3)]
+    q, cache, queue = normal(1, H, D), KVCache(dev, 1, Hkv, D, max_seq=2048), _busy(dev)
+
+    def program():
+        out = []
+        for k, v in sets * 4:
+            queue()
+            cache.lengths[0] = 0
+            cache.append(0, k, v)
+            out.append(cache.attention(0, q, H, q_pos0=rows - 1))
+        return out
+
+    on, off = _both(dev, program)
+    for i, (a, b) in enumerate(zip(on, off)):
+        assert np.array_equal(a.view(np.uint16), b.view(np.uint16)), i
