@@ -668,7 +668,7 @@ int32_t tlc_launch_gemm(tlc_ctx *ctx, const tlc_gemv_args &a) {
     int noff = 0;
     const __half *x = static_cast<const __half *>(a.x);
     if (a.norm_w) {
-        if (int32_t rc = tlc_launch_rms_norm(ctx, a.x, a.norm_w, scratch, a.m, (int32_t)k, a.eps, true)) return rc;
+        if (int32_t rc = tlc_launch_rms_norm(ctx, a.x, a.norm_w, scratch, a.m, (int32_t)k, a.eps, a.norm_early)) return rc;
         x = reinterpret_cast<const __half *>(scratch);
     }
     TLC_REQUIRE(((uintptr_t)x & 15) == 0, TLC_ERR_INVALID_OPERATION, "gemm: activations must be 16-byte aligned");

@@ -479,7 +479,7 @@ int32_t tlc_launch_gemv(tlc_ctx *ctx, const tlc_gemv_args &a) {
         const __half *x = static_cast<const __half *>(a.x);
         if (a.norm_w) {
             if (int32_t rc = tlc_scratch_reserve(ctx, (size_t)a.m * k * 2)) return rc;
-            if (int32_t rc = tlc_launch_rms_norm(ctx, a.x, a.norm_w, ctx->scratch, a.m, (int32_t)k, a.eps, true)) return rc;
+            if (int32_t rc = tlc_launch_rms_norm(ctx, a.x, a.norm_w, ctx->scratch, a.m, (int32_t)k, a.eps, a.norm_early)) return rc;
             x = static_cast<const __half *>(ctx->scratch);
         }
         const int threads = 256;
@@ -519,7 +519,7 @@ int32_t tlc_launch_gemv(tlc_ctx *ctx, const tlc_gemv_args &a) {
         const __half *x = static_cast<const __half *>(a.x);
         if (a.norm_w) {
             if (int32_t rc = tlc_scratch_reserve(ctx, (size_t)a.m * k * 2)) return rc;
-            if (int32_t rc = tlc_launch_rms_norm(ctx, a.x, a.norm_w, ctx->scratch, a.m, (int32_t)k, a.eps, true)) return rc;
+            if (int32_t rc = tlc_launch_rms_norm(ctx, a.x, a.norm_w, ctx->scratch, a.m, (int32_t)k, a.eps, a.norm_early)) return rc;
             x = static_cast<const __half *>(ctx->scratch);
         }
         TLC_REQUIRE(((uintptr_t)x & 15) == 0, TLC_ERR_INVALID_OPERATION, "linear: activations must be 16-byte aligned");
@@ -591,6 +591,7 @@ int32_t tlc_launch_gemv(tlc_ctx *ctx, const tlc_gemv_args &a) {
         p.m = mc;
         p.x = static_cast<const __half *>(a.x) + (size_t)m0 * k;
         p.norm_w = static_cast<const __half *>(a.norm_w);
+        p.norm_early = a.norm_early ? 1 : 0;
         p.eps = a.eps;
         p.epilogue = a.epilogue;
         p.bias = static_cast<const __half *>(a.bias);
@@ -608,8 +609,9 @@ int32_t tlc_launch_gemv(tlc_ctx *ctx, const tlc_gemv_args &a) {
             if (int32_t rc = tlc_scratch_reserve(ctx, frag_total_bytes(nblk, nt))) return rc;
             uint4 *frag = static_cast<uint4 *>(ctx->scratch);
             float *start = reinterpret_cast<float *>(static_cast<uint8_t *>(ctx->scratch) + frag_bytes(nblk, nt));
-            const cudaError_t le = tlc_launch_pdl(ctx, q4 ? frag_rows_kernel<TLC_TYPE_Q4_0> : frag_rows_kernel<TLC_TYPE_Q8_0>, dim3(8 * nt),
-                                                  dim3(512), 0, p.x, p.norm_w, mc, (int)k, a.eps, frag, start, nt);
+            auto *fn = a.norm_early ? (q4 ? frag_rows_kernel<TLC_TYPE_Q4_0, true> : frag_rows_kernel<TLC_TYPE_Q8_0, true>)
+                                    : (q4 ? frag_rows_kernel<TLC_TYPE_Q4_0, false> : frag_rows_kernel<TLC_TYPE_Q8_0, false>);
+            const cudaError_t le = tlc_launch_pdl(ctx, fn, dim3(8 * nt), dim3(512), 0, p.x, p.norm_w, mc, (int)k, a.eps, frag, start, nt);
             if (le != cudaSuccess) {
                 cudaGetLastError();
                 return tlc_fail(TLC_ERR_CUDA, "gemv: RMSNorm launch failed: %s", cudaGetErrorString(le));

@@ -88,6 +88,7 @@ struct GemvParams {
     int round, n_rounds;  // cluster: slabs (of one CTA) per exchange, exchanges of a launch
     // tlc_gemv_splitk_finish: f32 shares [ksplit][m][ntot] of a split-K GEMM
     int ntot;
+    int norm_early;  // one row: norm_w may be read before the dependency wait (tlc_gemv_args)
     float *partial;
 };
 

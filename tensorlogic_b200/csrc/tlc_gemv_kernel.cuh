@@ -69,7 +69,8 @@ __device__ __forceinline__ float start_value(const uint4 &f) {
 // RMSNorm of the activation rows and their fragment order, once per call instead of once per CTA of the GEMV
 // (8 rows of K = 8192: the GEMV's CTAs took 8 us over it, more than over the weights of a TP8 rank's
 // projection).  One CTA per row; rows past m are written as zeros.  Bound by the latency of one pass over the row.
-template <int QT>
+// W_EARLY: see norm_early of tlc_gemv_args.
+template <int QT, bool W_EARLY>
 __global__ void __launch_bounds__(512) frag_rows_kernel(const __half *__restrict__ x, const __half *__restrict__ w, int m, int k,
                                                         float eps, uint4 *__restrict__ frag, float *__restrict__ start, int nt) {
     __shared__ float part[16];
@@ -77,9 +78,9 @@ __global__ void __launch_bounds__(512) frag_rows_kernel(const __half *__restrict
     const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, items = k / 8;
     const __half *xr = x + (size_t)row * k;
     uint4 nw = make_uint4(0, 0, 0, 0);
-    if (tid < items) nw = load_piece<QT>(w + (tid >> 2) * 32, tid & 3);
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (W_EARLY && tid < items) nw = load_piece<QT>(w + (tid >> 2) * 32, tid & 3);
+    tlc_pdl_after_wait();
+    if (!W_EARLY && tid < items) nw = load_piece<QT>(w + (tid >> 2) * 32, tid & 3);
     const bool live = row < m;
     uint4 v[KEEP];
     float sq = 0.f;

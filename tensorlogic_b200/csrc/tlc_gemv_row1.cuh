@@ -137,13 +137,14 @@ __global__ void __launch_bounds__((CW + 1) * 32, CW == 8 ? 2 : 1) gemv_row1_kern
         }
         return *reinterpret_cast<const uint4 *>(r + 8 * t);
     };
-    // The norm weights do not come from the previous kernel: the first round's are fetched
+    // The norm weights of a model do not come from the previous kernel: the first round's are fetched
     // (the later rounds' brought into the cache) while that kernel is still running.
     uint4 nw_first = make_uint4(0, 0, 0, 0);
-    if (do_norm) {
+    auto fetch_norm = [&]() {
         if (ctid < live_items) nw_first = piece(p.norm_w, ctid);
         for (int idx = ctid + CT; idx < live_items; idx += CT) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.norm_w + (idx >> 2) * 32));
-    }
+    };
+    if (do_norm && p.norm_early) fetch_norm();
     pdl_wait();  // the activations (and residual) come from the previous kernel
     // Mode 3: the successor may be scheduled while this CTA does its own work, but not before the
     // predecessor is done (its CTAs then never wait behind two grids).
@@ -157,6 +158,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, CW == 8 ? 2 : 1) gemv_row1_kern
     }
     float inv = 1.f;
     if (do_norm) {
+        if (!p.norm_early) fetch_norm();
         float sq = 0.f;
         auto add = [&](const uint4 &v) {
             const __half2 *h = reinterpret_cast<const __half2 *>(&v);

@@ -246,6 +246,9 @@ struct tlc_gemv_args {
     const void *x = nullptr;  // f16 [m, K]
     int32_t m = 0;
     const void *norm_w = nullptr;  // f16 [K] or null
+    // No kernel in flight writes norm_w, which may then be read before the dependency wait: the caller's word for the
+    // tensors of a model.  A program may have computed its norm weights with the kernel right before.
+    bool norm_early = false;
     float eps = 0.f;
     int32_t epilogue = TLC_EPI_STORE;
     const void *bias = nullptr;      // f16 [N] (STORE, single output)

@@ -615,6 +615,7 @@ static int32_t forward(tlc_llama *L, int m, bool decode, int pos0, bool all_logi
             a.x = L->x;
             a.m = m;
             a.norm_w = w.attn_norm->data;
+            a.norm_early = true;
             a.eps = c.rms_eps;
             a.pos_offset = pos0;
             a.rope_base = c.rope_base;
@@ -656,6 +657,7 @@ static int32_t forward(tlc_llama *L, int m, bool decode, int pos0, bool all_logi
             a.x = L->x1;
             a.m = m;
             a.norm_w = w.ffn_norm->data;
+            a.norm_early = true;
             a.eps = c.rms_eps;
             a.epilogue = TLC_EPI_SWIGLU;
             if (int32_t rc = tlc_launch_gemv(ctx, a)) return rc;
@@ -686,6 +688,7 @@ static int32_t forward(tlc_llama *L, int m, bool decode, int pos0, bool all_logi
         a.x = L->x + (size_t)(m - rows) * d;
         a.m = rows;
         a.norm_w = L->out_norm->data;
+        a.norm_early = true;
         a.eps = c.rms_eps;
         if (parts & 1) {
             if (int32_t rc = tlc_launch_gemv(ctx, a)) return rc;

@@ -53,3 +53,38 @@ def test_attention_right_after_append(dev, H, Hkv, D, rows):
     on, off = _both(dev, program)
     for i, (a, b) in enumerate(zip(on, off)):
         assert np.array_equal(a.view(np.uint16), b.view(np.uint16)), i
+
+
+@pytest.mark.parametrize("m", [1, 5, 16, 40])
+@pytest.mark.parametrize("qtype", [1, 2, 8, 14])
+def test_norm_weights_computed_right_before(dev, qtype, m):
+    """mul -> norm_linear_multi and mul -> swiglu_gate_up: the norm weights are the product, in every form that norms
+    (one row, two to sixteen, the GEMM, dense and Q6_K weights)."""
+    from tensorlogic_b200 import synth
+    from tensorlogic_b200.api import QTensor, mul, norm_linear_multi, swiglu_gate_up
+    k, n = 8192, 96
+    rng = np.random.default_rng(qtype + m)
+    if qtype == 14:
+        raw = rng.integers(0, 256, (n * k // 256, 210), dtype=np.uint8)
+        raw[:, 208:210] = rng.uniform(1e-5, 2e-5, (raw.shape[0], 1)).astype(np.float16).view(np.uint8)
+        w = QTensor.from_blocks(dev, 14, n, k, raw)
+    elif qtype == 1:
+        w = QTensor.normal_f16(dev, n, k, 3, synth.tensor_id("dw"), 0.0, 0.02)
+    else:
+        w = QTensor.synthetic(dev, qtype, n, k, 3, synth.tensor_id("dw"), scale_log2=-3 if qtype == 2 else -7)
+    normal = lambda *shape: dev.tensor(rng.standard_normal(shape).astype(np.float16))
+    x, norms, scale, queue = normal(m, k), [normal(k) for _ in range(3)], normal(k), _busy(dev)
+
+    def program():
+        out = []
+        for nw in norms * 4:
+            queue()
+            out += norm_linear_multi(x, [w], mul(nw, scale), 1e-5)
+            if qtype in (2, 8):
+                queue()
+                out.append(swiglu_gate_up(x, w, w, mul(nw, scale), 1e-5))
+        return out
+
+    on, off = _both(dev, program)
+    for i, (a, b) in enumerate(zip(on, off)):
+        assert np.array_equal(a.view(np.uint16), b.view(np.uint16)), i
