@@ -449,8 +449,8 @@ static constexpr size_t attention_smem_limit(int D) {
 }
 
 template <typename V>
-__global__ void kv_append_kernel(const V *__restrict__ k, const V *__restrict__ v, V *__restrict__ kc, V *__restrict__ vc, int m,
-                                 int row_elems, int tmax, int pos_offset, const int *__restrict__ positions, int batched) {
+__global__ void kv_append_kernel(const V *k, const V *v, V *__restrict__ kc, V *__restrict__ vc, int m,
+                                 int row_elems, int tmax, int pos_offset, const int *positions, int batched) {
     tlc_pdl_after_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)m * row_elems) return;

@@ -80,9 +80,8 @@ __global__ void linear_generic_kernel(const uint8_t *__restrict__ w, size_t pitc
 // per weight; K must be a multiple of 8 and rows 16-byte aligned.  (More rows: tlc_gemm_wt.cu.)
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) linear_f16_kernel(const uint8_t *__restrict__ w, size_t pitch, int n_rows, int k,
-                                                         const __half *__restrict__ x, __half *__restrict__ y,
-                                                         const __half *__restrict__ bias,
-                                                         const __half *__restrict__ residual) {
+                                                         const __half *x, __half *__restrict__ y, const __half *bias,
+                                                         const __half *residual) {
     tlc_pdl_prologue();
     const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;

@@ -71,7 +71,7 @@ __device__ __forceinline__ float start_value(const uint4 &f) {
 // projection).  One CTA per row; rows past m are written as zeros.  Bound by the latency of one pass over the row.
 // W_EARLY: see norm_early of tlc_gemv_args.
 template <int QT, bool W_EARLY>
-__global__ void __launch_bounds__(512) frag_rows_kernel(const __half *__restrict__ x, const __half *__restrict__ w, int m, int k,
+__global__ void __launch_bounds__(512) frag_rows_kernel(const __half *x, const __half *w, int m, int k,
                                                         float eps, uint4 *__restrict__ frag, float *__restrict__ start, int nt) {
     __shared__ float part[16];
     constexpr int KEEP = 4;  // pieces of the row a thread keeps: K = 16384
@@ -282,13 +282,13 @@ __global__ void __launch_bounds__(CW * 32, CW == 8 ? 2 : 1) gemv_mma_kernel(cons
         for (int b = 0; b < NB; b++)
 #pragma unroll
             for (int nt = 0; nt < NT; nt++) {
-                const uint4 v = b < my_blocks ? __ldg(p.frag + ((size_t)(wb0 + b) * NT + nt) * 32 + lane) : make_uint4(0, 0, 0, 0);
+                const uint4 v = b < my_blocks ? p.frag[((size_t)(wb0 + b) * NT + nt) * 32 + lane] : make_uint4(0, 0, 0, 0);
                 xb[nt][b][0] = v.x;
                 xb[nt][b][1] = v.y;
                 xb[nt][b][2] = v.z;
                 xb[nt][b][3] = v.w;
             }
-        for (int i = lane; i < NB * MP; i += 32) ci_w[i] = i < my_blocks * MP ? __ldg(p.start + (size_t)wb0 * MP + i) : 0.f;
+        for (int i = lane; i < NB * MP; i += 32) ci_w[i] = i < my_blocks * MP ? p.start[(size_t)wb0 * MP + i] : 0.f;
     } else {
 #pragma unroll
         for (int nt = 0; nt < NT; nt++) {

@@ -165,7 +165,9 @@ int32_t tlc_scratch_reserve(tlc_ctx *ctx, size_t bytes);
 // Launches `kernel` on the context's stream, with programmatic stream
 // serialization when the context allows it: the kernel may then be scheduled
 // before its predecessor has finished and must execute griddepcontrol.wait
-// before it reads or overwrites anything the predecessor touches.
+// before it reads or overwrites anything the predecessor touches.  What a predecessor
+// may write is read through plain loads: the read-only path (`const T *__restrict__`,
+// __ldg) is defined only for data that nothing writes while the kernel is resident.
 template <typename... KArgs, typename... Args>
 inline cudaError_t tlc_launch_pdl(tlc_ctx *ctx, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
                                   Args &&...args) {

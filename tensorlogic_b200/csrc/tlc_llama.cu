@@ -105,7 +105,7 @@ __device__ __forceinline__ void report_to_host(const HostReport &hr, int b, int 
 }
 
 __global__ void embed_kernel(const uint8_t *__restrict__ table, size_t pitch, int vocab, int d,
-                             const int *__restrict__ ids, int m, __half *__restrict__ y) {
+                             const int *ids, int m, __half *__restrict__ y) {
     tlc_pdl_prologue();  // ids are written by the previous step's sampling kernel
     const int vec = d >> 3;
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -122,7 +122,7 @@ __global__ void embed_kernel(const uint8_t *__restrict__ table, size_t pitch, in
 // back as the next input and advances the sequence position.
 // With tensor parallelism the logits arrive as gathered vocabulary shards
 // [shard][row][vocab_per_shard]; token index = shard * vocab_per_shard + i.
-__global__ void argmax_advance_kernel(const __half *__restrict__ logits, int vocab, int shards, int rows,
+__global__ void argmax_advance_kernel(const __half *logits, int vocab, int shards, int rows,
                                       int *__restrict__ next_ids, int *__restrict__ ids,
                                       int *__restrict__ positions, int advance, HostReport hr) {
     __shared__ float sv[32];
@@ -223,9 +223,9 @@ __host__ __device__ inline float tlc_sample_uniform(uint64_t seed, uint32_t pos,
 // boundary).  (One run per thread instead, read value by value, touched a line
 // of its own per lane and load: 32000 tokens 29 us, this form 12.7.)
 // u comes from `uniforms[b]` when given, else from tlc_sample_uniform.
-__global__ void __launch_bounds__(1024) sample_advance_kernel(const __half *__restrict__ logits, int vocab, int shards,
+__global__ void __launch_bounds__(1024) sample_advance_kernel(const __half *logits, int vocab, int shards,
                                                               int rows, float temperature, uint64_t seed,
-                                                              const float *__restrict__ uniforms, int fixed_pos,
+                                                              const float *uniforms, int fixed_pos,
                                                               int *__restrict__ next_ids, int *__restrict__ ids,
                                                               int *__restrict__ positions, int advance, HostReport hr) {
     __shared__ float red[32];

@@ -15,7 +15,7 @@ namespace {
 // (src/ops/normalization.rs:199-248): one CTA per row.  A launch of a few rows is a chain of latencies: the row is
 // read once, a thread keeps its pieces, and the weights come with it, or before it where the caller vouches
 // that no kernel in flight writes them (w_early): 32 x 4096 3.4 -> 2.3 us.
-__global__ void __launch_bounds__(256) rms_norm_kernel(const __half *__restrict__ x, const __half *__restrict__ w,
+__global__ void __launch_bounds__(256) rms_norm_kernel(const __half *x, const __half *w,
                                                        __half *__restrict__ y, int d, float eps, int w_early) {
     constexpr int KEEP = 4;  // 16-byte pieces of the row a thread keeps: d = 8192
     __shared__ float warp_sums[8];
@@ -87,8 +87,8 @@ __global__ void __launch_bounds__(256) rms_norm_kernel(const __half *__restrict_
 }
 
 // rope_f16 (shaders/unified.metal:2355-2417): one thread per pair.
-__global__ void rope_kernel(const __half *__restrict__ x, __half *__restrict__ y, int seq, int heads, int d,
-                            int pos_offset, float base, const int *__restrict__ positions) {
+__global__ void rope_kernel(const __half *x, __half *__restrict__ y, int seq, int heads, int d,
+                            int pos_offset, float base, const int *positions) {
     tlc_pdl_after_wait();
     const int half_d = d >> 1;
     const size_t total = (size_t)seq * heads * half_d;
@@ -112,8 +112,8 @@ __global__ void rope_kernel(const __half *__restrict__ x, __half *__restrict__ y
 // cosines and sines read from f16 tables instead of being worked out.  Pair p of position s
 // reads table[s * pitch + p] -- exactly the shader's index arithmetic (`seq_idx * head_dim +
 // dim_pair_idx`, i.e. pitch = head_dim there).  One thread per pair.
-__global__ void rope_table_kernel(const __half *__restrict__ x, const __half *__restrict__ cos_t,
-                                  const __half *__restrict__ sin_t, __half *__restrict__ y, int seq, int heads, int d,
+__global__ void rope_table_kernel(const __half *x, const __half *cos_t,
+                                  const __half *sin_t, __half *__restrict__ y, int seq, int heads, int d,
                                   int pitch) {
     tlc_pdl_after_wait();
     const int half_d = d >> 1;
@@ -145,7 +145,7 @@ struct OpSwiglu {  // silu(g) * u with the three f16 roundings of sigmoid, mul, 
     static __device__ __forceinline__ __half run(__half g, __half u) { return __hmul(__hmul(g, OpSigmoid::run(g, g)), u); }
 };
 template <class OP, bool TWO>
-__global__ void __launch_bounds__(256) elementwise_kernel(const __half *__restrict__ a, const __half *__restrict__ b,
+__global__ void __launch_bounds__(256) elementwise_kernel(const __half *a, const __half *b,
                                                           __half *__restrict__ y, size_t n, int vec) {
     tlc_pdl_after_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(256) elementwise_kernel(const __half *__restri
 // softmax_simple_f16 (shaders/unified.metal:2150-2200): finite-only f32 max and
 // sum, exponentials rounded to f16 before the divide, uniform row when the sum
 // degenerates.
-__global__ void softmax_kernel(const __half *__restrict__ x, __half *__restrict__ y, int rows, int last) {
+__global__ void softmax_kernel(const __half *x, __half *__restrict__ y, int rows, int last) {
     tlc_pdl_after_wait();
     const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -200,7 +200,7 @@ __global__ void softmax_kernel(const __half *__restrict__ x, __half *__restrict_
 }
 
 // embedding_lookup_f16 (shaders/unified.metal:658-675): 16-byte vector gather.
-__global__ void embedding_kernel(const __half *__restrict__ table, const int *__restrict__ ids, int d,
+__global__ void embedding_kernel(const __half *table, const int *ids, int d,
                                  int m, __half *__restrict__ y) {
     tlc_pdl_after_wait();
     const int vec_per_row = d >> 3;
@@ -210,7 +210,7 @@ __global__ void embedding_kernel(const __half *__restrict__ table, const int *__
     reinterpret_cast<uint4 *>(y + (size_t)r * d)[c] =
         reinterpret_cast<const uint4 *>(table + (size_t)ids[r] * d)[c];
 }
-__global__ void embedding_scalar_kernel(const __half *__restrict__ table, const int *__restrict__ ids, int d,
+__global__ void embedding_scalar_kernel(const __half *table, const int *ids, int d,
                                         int m, __half *__restrict__ y) {
     tlc_pdl_after_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
