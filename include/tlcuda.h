@@ -222,7 +222,8 @@ TLC_API int32_t tlc_qtensor_create(tlc_ctx *ctx, int32_t type, int64_t n_rows, i
                                    int32_t tp_size, int32_t split, tlc_qtensor **out);
 /* Same, but the shard is filled on the device from the counter-based
  * generator of the benchmark configurations (weights too large to stage on
- * the host).  Only Q4_0 / Q8_0.  Block scales are U[0.002, 0.02] * 2^scale_log2. */
+ * the host).  Only Q4_0 / Q8_0.  Block scales are U[0.002, 0.02] * 2^scale_log2.
+ * Like every call that creates a tensor it returns when the weights are in place. */
 TLC_API int32_t tlc_qtensor_create_synthetic(tlc_ctx *ctx, int32_t type, int64_t n_rows,
                                              int64_t n_cols, uint64_t seed, uint64_t tensor_id,
                                              int32_t scale_log2, int32_t tp_rank, int32_t tp_size,

@@ -420,10 +420,12 @@ extern "C" int32_t tlc_qtensor_create_synthetic(tlc_ctx *ctx, int32_t type, int6
         tlc_synth_key(seed, tensor_id), scale_log2);
     ctx->launches++;
     e = cudaGetLastError();
+    // The weights are there before their handle is: kernels fetch weights in front of their dependency wait.
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) {
         cudaFree(qt->data);
         delete qt;
-        return tlc_fail(TLC_ERR_CUDA, "generator launch failed: %s", cudaGetErrorString(e));
+        return tlc_fail(TLC_ERR_CUDA, "weight generator failed: %s", cudaGetErrorString(e));
     }
     *out = qt;
     return TLC_OK;
@@ -482,7 +484,12 @@ extern "C" int32_t tlc_qtensor_create_normal_f16(tlc_ctx *ctx, int64_t n_rows, i
     tlc_qtensor *qt = nullptr;
     if (int32_t rc = alloc_qtensor(ctx, TLC_TYPE_F16, n_rows, n_cols, n_rows, n_cols, 0, 1, TLC_SPLIT_NONE, &qt)) return rc;
     // n_cols % 8 == 0 makes the row pitch equal to the row size: one flat fill.
-    if (int32_t rc = tlc_fill_normal_f16(ctx, qt->data, (size_t)n_rows * n_cols, seed, tensor_id, mean, std)) {
+    int32_t rc = tlc_fill_normal_f16(ctx, qt->data, (size_t)n_rows * n_cols, seed, tensor_id, mean, std);
+    if (!rc) {  // (as above: norm weights are fetched early too)
+        const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+        if (e != cudaSuccess) rc = tlc_fail(TLC_ERR_CUDA, "weight generator failed: %s", cudaGetErrorString(e));
+    }
+    if (rc) {
         cudaFree(qt->data);
         delete qt;
         return rc;

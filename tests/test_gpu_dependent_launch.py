@@ -88,3 +88,20 @@ def test_norm_weights_computed_right_before(dev, qtype, m):
     on, off = _both(dev, program)
     for i, (a, b) in enumerate(zip(on, off)):
         assert np.array_equal(a.view(np.uint16), b.view(np.uint16)), i
+
+
+def test_generated_weights_are_there_when_their_handle_is(dev):
+    """Kernels fetch weights and a model's norm weights in front of their dependency wait: nothing that writes them
+    may be in flight once the call that creates them has returned."""
+    import torch
+    from tensorlogic_b200 import synth
+    from tensorlogic_b200.api import QTensor
+    stream = torch.cuda.ExternalStream(dev.stream)
+    queue = _busy(dev)
+    for make in (lambda: QTensor.synthetic(dev, 2, 8192, 28672, 1, synth.tensor_id("g4")),
+                 lambda: QTensor.synthetic(dev, 8, 8192, 28672, 1, synth.tensor_id("g8")),
+                 lambda: QTensor.normal_f16(dev, 8192, 8192, 1, synth.tensor_id("gf"), 1.0, 0.02)):
+        queue()
+        w = make()
+        assert stream.query()
+        del w
