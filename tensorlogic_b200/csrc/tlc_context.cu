@@ -296,6 +296,7 @@ int32_t tlc_scratch_reserve(tlc_ctx *ctx, size_t bytes) {
     if (ctx->scratch) TLC_CUDA(cudaFree(ctx->scratch));
     ctx->scratch = nullptr;
     ctx->scratch_bytes = 0;
+    ctx->scratch_moves++;
     size_t want = (bytes + ((size_t)1 << 20) - 1) & ~(((size_t)1 << 20) - 1);
     cudaError_t e = cudaMalloc(&ctx->scratch, want);
     if (e != cudaSuccess) {

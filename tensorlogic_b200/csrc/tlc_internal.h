@@ -51,6 +51,7 @@ struct tlc_ctx {
     // Reusable scratch for kernels that need global workspace (grows on demand).
     void *scratch = nullptr;
     size_t scratch_bytes = 0;
+    uint64_t scratch_moves = 0;  // how often `scratch` has been replaced: a captured graph holds its address
     // tlc_gemm_wt.cu: the f32 sums of a tile's parts (one slot of 256 x 128 per SM) and their flags
     // (zero between launches; cleared by the host after a wait that ran out).
     float *wt_partial = nullptr;

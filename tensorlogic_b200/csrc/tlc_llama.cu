@@ -72,6 +72,7 @@ struct tlc_llama {
     int32_t *host_ids;  // pinned staging
     int32_t *host_next;
     std::map<int, cudaGraphExec_t> graph;  // decode graphs keyed by batch * 8 + parts (1000 + batch: the host step)
+    uint64_t graph_scratch = 0;            // the context's scratch_moves when they were captured
     const int *ids_src = nullptr;          // set while the host step is captured: token ids read from pinned memory
     HostReport report{};                   //   and results reported straight to pinned memory
     int launches_in[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // kernels per step, by parts mask
@@ -557,12 +558,17 @@ extern "C" int32_t tlc_llama_create(tlc_ctx *ctx, tlc_model *model, const tlc_ll
     return TLC_OK;
 }
 
+static void drop_graphs(tlc_llama *L) {
+    for (auto &g : L->graph)
+        if (g.second) cudaGraphExecDestroy(g.second);
+    L->graph.clear();
+}
+
 extern "C" int32_t tlc_llama_destroy(tlc_llama *L) {
     if (!L) return TLC_OK;
     cudaSetDevice(L->ctx->device);
     cudaStreamSynchronize(L->ctx->stream);
-    for (auto &g : L->graph)
-        if (g.second) cudaGraphExecDestroy(g.second);
+    drop_graphs(L);
     tlc_kvcache_destroy(L->cache);
     void *bufs[] = {L->x, L->x1, L->q, L->attn, L->act, L->logits, L->ids, L->positions, L->next_ids,
                     L->part, L->logits_full, L->step_ws, L->step_layers, L->step_trace};
@@ -810,6 +816,16 @@ static int32_t reserve_positions(tlc_llama *L, int batch, int steps) {
     return TLC_OK;
 }
 
+// Captured steps hold the address of the context's scratch (normalised rows, key splits), which any other call on
+// the context may have made larger and thereby replaced: such graphs are captured again.
+static int32_t drop_stale_graphs(tlc_llama *L) {
+    if (L->graph_scratch == L->ctx->scratch_moves) return TLC_OK;
+    TLC_CUDA(cudaStreamSynchronize(L->ctx->stream));
+    drop_graphs(L);
+    L->graph_scratch = L->ctx->scratch_moves;
+    return TLC_OK;
+}
+
 // Enqueues `steps` greedy decode steps for `batch` sequences (graph replay);
 // nothing is read back.  parts != 7 replays only some of the step's launches
 // (for per-kernel timing) and leaves tokens and positions untouched.
@@ -831,11 +847,13 @@ static int32_t decode_enqueue(tlc_llama *L, int32_t batch, int32_t steps, int pa
         return step_launch(L, steps, nullptr, nullptr, nullptr);
     }
     const int key = batch * 8 + parts;
+    if (int32_t rc = drop_stale_graphs(L)) return rc;
     if (!L->graph.count(key) && !L->cfg.no_graph) {
         // Warm every kernel configuration (function attributes, scratch growth)
         // outside the capture, on a throw-away step that does not advance.
         if (int32_t rc = forward(L, batch, true, 0, false, true, false, parts)) return rc;
         TLC_CUDA(cudaStreamSynchronize(ctx->stream));
+        if (int32_t rc = drop_stale_graphs(L)) return rc;  // (that step may have needed more scratch)
         const uint64_t launches_before = ctx->launches;
         TLC_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
         int32_t rc = forward(L, batch, true, 0, false, true, advance, parts);
@@ -924,6 +942,7 @@ extern "C" int32_t tlc_llama_decode_host(tlc_llama *L, int32_t batch, const int3
         tlc_ctx *ctx = L->ctx;
         if (int32_t rc = reserve_positions(L, batch, 1)) return rc;  // before anything is launched
         const int key = 1000 + batch;
+        if (int32_t rc = drop_stale_graphs(L)) return rc;
         if (!L->graph.count(key)) {
             if (int32_t rc = decode_enqueue(L, batch, 0, 7)) return rc;  // warms the kernels, captures the plain step
             TLC_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -1019,9 +1038,7 @@ extern "C" int32_t tlc_llama_set_sampling(tlc_llama *L, float temperature, uint6
     if (int32_t rc = tlc_enter(L->ctx)) return rc;
     TLC_CUDA(cudaStreamSynchronize(L->ctx->stream));
     // captured decode graphs hold the old sampling kernel and its arguments
-    for (auto &g : L->graph)
-        if (g.second) cudaGraphExecDestroy(g.second);
-    L->graph.clear();
+    drop_graphs(L);
     L->temperature = temperature;
     L->sample_seed = seed;
     return TLC_OK;

@@ -388,3 +388,31 @@ def test_weight_cache_lru(dev, ref, tmp_path):
     with pytest.raises(TensorError):
         WeightCache(dev, tmp_path / "missing.gguf", 2)
     cache.close()
+
+
+def test_captured_steps_survive_growth_of_the_scratch(dev):
+    """A captured step of several sequences holds the address of the context's scratch (its normalised rows).  Another
+    call that needs more scratch replaces it: the next steps must not touch the memory that was given back."""
+    from tensorlogic_b200 import synth
+    from tensorlogic_b200.api import matmul
+    from tensorlogic_b200.model import Llama, model_from_host, synthetic_host_weights
+    arch = _small_arch()
+    llm = Llama(dev, model_from_host(dev, synthetic_host_weights(arch, seed=5)), arch, max_seq=32, max_batch=4)
+    ids = synth.token_ids(5, "grow", 3, arch.vocab)
+
+    def steps():
+        llm.set_state(ids, [4, 5, 6])
+        out = [llm.decode(ids, return_logits=True)[1].copy() for _ in range(2)]
+        llm.set_state(ids, [4, 5, 6])
+        llm.decode_enqueue(3, 3)
+        return out + [llm.read_state(3)[0].copy()]
+
+    before = steps()
+    # rows of odd length: matmul copies them to scratch, 256 MB, more than any other test asks for
+    matmul(dev.tensor(np.zeros((131072, 1023), np.float16)), dev.tensor(np.zeros((1023, 8), np.float16)))
+    taken = [dev.tensor(np.full((1 << 20,), 7.0, np.float16)) for _ in range(16)]  # the freed memory has new owners
+    after = steps()
+    for x, y in zip(before, after):
+        assert np.array_equal(x, y)
+    for t in taken:
+        assert np.all(t.numpy() == np.float16(7.0))
