@@ -623,15 +623,11 @@ bool tlc_gemm_eligible(const tlc_ctx *ctx, const tlc_gemv_args &a) {
     // zero padding (rows are padded to 16 bytes with zeros at upload) against zero-filled activations
     if (w0->n_cols % 32 != 0 || w0->n_cols < kBK) return false;
     if (ctx->gemm_min_m > 0) return a.m >= ctx->gemm_min_m;
-    // From 17 rows on the GEMV would read the weights again.  Up to eight it is the faster form everywhere, with 9
-    // to 16 rows while its registers hold the activations of a short K: a long one it shares out over clusters,
-    // whose CTAs wait for one another, and the GEMM wins although it starts later.  Q4_0 4096 x 11008 at 9 / 16 rows
-    // 17.4 / 20.2 us, GEMM 16.0 (Q8_0 18.5 / 19.0, 16.0); 1280 x 8192 at 16 rows 12.3, GEMM 8.3; 22016 x 4096 at 9 rows
-    // 24.1 both.  A decode step of 7B in Q4_0 at 9 / 12 rows 2.85 / 2.95 ms, with ffn_down by the GEMM 2.43 / 2.51 (with
-    // every projection 2.70); a rank of 70B in TP8 in Q8_0 (K = 8192) at 12 rows 6.63 -> 4.94 ms, in Q4_0 the same;
-    // TinyLlama's 2048 x 5632 makes no difference.
-    const int64_t held = (w0->type == TLC_TYPE_Q8_0 ? 72 : 96) * 1024;
-    return a.m > 16 || (a.m > 8 && a.m * w0->n_cols >= held);
+    // Up to 16 rows one pass of the GEMV reads the weights once and multiplies d * (q - 8) as it is; the GEMM
+    // multiplies that rounded to f16.  With a long K the GEMM would be faster from 9 rows on (Q4_0 4096 x 11008 at 9 / 16
+    // rows 15.2 us, GEMV 18.1 / 19.8; 1280 x 8192 at 16 rows 8.0 and 11.5), but against 64 bits its results are off
+    // by 2.8e-4 (Q8_0 2.9e-4) where the GEMV's are by 2.1e-4, the rounding of the output: precision goes first.
+    return a.m > 16;
 }
 
 // Same contract as tlc_launch_gemv for m activation rows on the tensor cores:

@@ -59,3 +59,27 @@ def test_q6_k_windows(dev, ref, n, k, m):
     x = synth.activations(9, f"q6x{m}x{k}", (m, k))
     got = linear(dev.tensor(x), QTensor.from_blocks(dev, 14, n, k, raw)).numpy()
     assert rel_l2(got, ref.linear_q(14, raw.reshape(-1), n, k, x)) < TIGHT
+
+
+def _exact_product(qtype, raw, x):
+    """x . W^T in 64 bits with the weights d * (q - 8) as the blocks define them, rounded once to f16."""
+    d = raw[..., :2].copy().view(np.float16).astype(np.float64)
+    if qtype == 2:
+        q = np.concatenate([(raw[..., 2:] & 15).astype(np.float64), (raw[..., 2:] >> 4).astype(np.float64)], -1) - 8
+    else:
+        q = raw[..., 2:].view(np.int8).astype(np.float64)
+    return (x.astype(np.float64) @ (q * d).reshape(raw.shape[0], -1).T).astype(np.float16)
+
+
+@pytest.mark.parametrize("qtype", [2, 8])
+@pytest.mark.parametrize("m,n,k", [(2, 200, 2048), (9, 200, 11008), (16, 200, 8192), (12, 100, 28672)])
+def test_weights_are_not_rounded(dev, qtype, m, n, k):
+    """Up to sixteen rows d * (q - 8) is multiplied as it is.  The f32 sum of K terms is then off by about 1e-6 of the
+    output, which moves about one in a hundred of the roundings to f16 (steps of 5e-4 to 1e-3); weights rounded to
+    f16 first, each by up to 2^-11, would move about four in ten."""
+    from tensorlogic_b200 import synth
+    from tensorlogic_b200.api import QTensor, linear
+    raw = synth.blocks(qtype, 7, synth.tensor_id(f"nr{n}x{k}"), n, k, scale_log2=-3 if qtype == 2 else -7)
+    x = synth.activations(7, f"nx{m}x{k}", (m, k))
+    got = linear(dev.tensor(x), QTensor.from_blocks(dev, qtype, n, k, raw)).numpy()
+    assert np.mean(got == _exact_product(qtype, raw, x)) > 0.95
