@@ -627,7 +627,23 @@ bool tlc_gemm_eligible(const tlc_ctx *ctx, const tlc_gemv_args &a) {
     // multiplies that rounded to f16.  With a long K the GEMM would be faster from 9 rows on (Q4_0 4096 x 11008 at 9 / 16
     // rows 15.2 us, GEMV 18.1 / 19.8; 1280 x 8192 at 16 rows 8.0 and 11.5), but against 64 bits its results are off
     // by 2.8e-4 (Q8_0 2.9e-4) where the GEMV's are by 2.1e-4, the rounding of the output: precision goes first.
-    return a.m > 16;
+    // For the same reason 17 to 48 rows stay in passes of sixteen where they have always been so, and their callers have
+    // exact weights: outputs of less than half a wave of 128-row tiles, and a K that is short, or short for the
+    // number of products, or so many outputs together that a wave has no room to share K out.  (8192 x 1024 at 17 /
+    // 32 / 48 rows 10.4 / 12.6 / 19.4 us, GEMM 7.3 / 7.4 / 7.7; 2048 x 512 at 17 rows 6.6, GEMM 6.2.)
+    if (a.m > 48) return true;
+    if (a.m <= 16) return false;
+    const bool pair = a.epilogue == TLC_EPI_SWIGLU;
+    int64_t widest = 0, outputs = 0, tiles = 0;
+    for (int i = 0; i < a.n_out; i++) {
+        const int64_t n = a.outs[i].w->n_rows;
+        widest = n > widest ? n : widest;
+        outputs += n;
+        tiles += pair ? (n + 127) / 128 * (i == 0) : (n + 255) / 256;
+    }
+    const bool exact = (widest + 127) / 128 * 2 < ctx->sm_count &&
+                       (tiles * 2 > ctx->sm_count || a.m * outputs >= 650 * (w0->n_cols - 1216));
+    return !exact;
 }
 
 // Same contract as tlc_launch_gemv for m activation rows on the tensor cores:

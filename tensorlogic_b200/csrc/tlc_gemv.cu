@@ -556,7 +556,7 @@ int32_t tlc_launch_gemv(tlc_ctx *ctx, const tlc_gemv_args &a) {
 
     if (tlc_gemm_eligible(ctx, a)) return tlc_launch_gemm(ctx, a);
 
-    // (rows beyond sixteen come here only when an option keeps them from the GEMM)
+    // (more than sixteen rows, where tlc_gemm_eligible leaves them here: passes over the weights)
     const int64_t nt2_tiles = kMaxCluster * (type == TLC_TYPE_Q4_0 ? max_window<TLC_TYPE_Q4_0>(2, 16) : max_window<TLC_TYPE_Q8_0>(2, 16));
     const int max_m = w0->k_tiles <= nt2_tiles ? 16 : 8;
     for (int m0 = 0; m0 < a.m; m0 += max_m) {

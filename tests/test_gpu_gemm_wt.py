@@ -12,10 +12,13 @@ TIGHT = 1e-3
 
 @pytest.fixture(params=[0, 1, 3, 8, 9], ids=["auto", "ks1", "ks3", "ks8", "stream"])
 def form(request, dev):
-    """CTAs per tile of the cluster form, or 9: the stream form."""
+    """CTAs per tile of the cluster form, or 9: the stream form.  (Small products of 17 to 48 rows are the GEMV's by
+    default.)"""
     dev.set_option("gemm_wt_ks", request.param)
+    dev.set_option("gemm_min_m", 1)
     yield request.param
     dev.set_option("gemm_wt_ks", 0)
+    dev.set_option("gemm_min_m", 0)
 
 
 @pytest.mark.parametrize("qtype,n,k,m", [(2, 1, 64, 17), (2, 129, 96, 33), (8, 300, 2080, 130), (8, 127, 160, 257),

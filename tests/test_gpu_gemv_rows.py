@@ -72,9 +72,10 @@ def _exact_product(qtype, raw, x):
 
 
 @pytest.mark.parametrize("qtype", [2, 8])
-@pytest.mark.parametrize("m,n,k", [(2, 200, 2048), (9, 200, 11008), (16, 200, 8192), (12, 100, 28672)])
+@pytest.mark.parametrize("m,n,k", [(2, 200, 2048), (9, 200, 11008), (16, 200, 8192), (12, 100, 28672), (17, 300, 64),
+                                   (33, 4100, 1216), (48, 9344, 1504)])
 def test_weights_are_not_rounded(dev, qtype, m, n, k):
-    """Up to sixteen rows d * (q - 8) is multiplied as it is.  The f32 sum of K terms is then off by about 1e-6 of the
+    """Up to sixteen rows, and up to 48 of a short K, d * (q - 8) is multiplied as it is.  The f32 sum of K terms is then off by about 1e-6 of the
     output, which moves about one in a hundred of the roundings to f16 (steps of 5e-4 to 1e-3); weights rounded to
     f16 first, each by up to 2^-11, would move about four in ten."""
     from tensorlogic_b200 import synth
