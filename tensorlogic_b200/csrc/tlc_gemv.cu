@@ -522,9 +522,9 @@ int32_t tlc_launch_gemv(tlc_ctx *ctx, const tlc_gemv_args &a) {
             x = static_cast<const __half *>(ctx->scratch);
         }
         TLC_REQUIRE(((uintptr_t)x & 15) == 0, TLC_ERR_INVALID_OPERATION, "linear: activations must be 16-byte aligned");
-        // (17 to 24 rows stay three passes of eight, the launch count callers have been promised; sixteen rows
-        // cost 1.6 times eight: 32000 x 2048 takes 18.2 us at 8 rows and 28.3 us at 16, 85.7 and 167.9 us before.)
-        const int pass = a.m > 16 && a.m <= 24 ? 8 : 16;
+        // (Sixteen rows cost 1.6 times eight, so passes of sixteen: 32000 x 2048 at 17 / 19 / 24 / 32 rows takes 43.2 / 43.5 /
+        // 45.3 / 54.5 us, in passes of eight 50.4 / 50.9 / 52.3 / 69.3.)
+        constexpr int pass = 16;
         for (int m0 = 0; m0 < a.m; m0 += pass) {
             GemvParams p{};
             p.m = a.m - m0 < pass ? a.m - m0 : pass;

@@ -114,7 +114,7 @@ def test_q6_k_fused_linear(dev, ref, n, k):
         want = ref.linear_q(Q6K, raw, n, k, x)
         l0 = dev.launch_count
         y = linear(dev.tensor(x), w).numpy()
-        assert dev.launch_count - l0 == (m + 7) // 8
+        assert dev.launch_count - l0 == (m + 15) // 16          # sixteen rows a pass over the weights
         assert y.shape == (m, n) and rel_l2(y, want) < 2e-3, m
         assert rel_l2(y, linear(dev.tensor(x), w16).numpy()) < 1e-3
     x = rng.standard_normal((3, k)).astype(np.float16)
