@@ -284,7 +284,9 @@ TLC_API int32_t tlc_matmul(tlc_ctx *ctx, const void *a_dev, const void *b_dev, v
  * f16 in/out, f32 accumulation, one rounding; optional bias [N] added as a
  * separate f16 add like the builtin does (builtin_math.rs:109-117).
  * x_cols is the caller's K and must equal W's columns
- * (TLC_ERR_INVALID_OPERATION otherwise, matmul.rs:266-273). */
+ * (TLC_ERR_INVALID_OPERATION otherwise, matmul.rs:266-273).  Quantized weights want
+ * activations (and fused norm weights) that are 16-byte aligned, Q4_0 on up to 16 rows
+ * 8-byte aligned; other addresses are TLC_ERR_INVALID_OPERATION. */
 TLC_API int32_t tlc_linear(tlc_ctx *ctx, tlc_qtensor *w, const void *x_dev, int32_t m,
                            int64_t x_cols, void *y_dev, const void *bias_dev);
 /* Host-buffer variant: uploads x, runs, downloads y, waits. */

@@ -557,6 +557,7 @@ int32_t tlc_launch_attention(tlc_ctx *ctx, tlc_kvcache *cache, int layer, const 
     TLC_REQUIRE(G == 1 || G == 2 || G == 4 || G == 8 || G == 16, TLC_ERR_INVALID_OPERATION,
                 "attention: group size %d unsupported (1, 2, 4, 8, 16)", G);
     TLC_REQUIRE(D == 64 || D == 128, TLC_ERR_INVALID_OPERATION, "attention: head_dim %d unsupported (64, 128)", D);
+    TLC_REQUIRE(((uintptr_t)q_dev & 3) == 0, TLC_ERR_INVALID_OPERATION, "attention: queries must be 4-byte aligned");
     TLC_REQUIRE(I >= 1 && (positions_dev == nullptr || I == 1), TLC_ERR_INVALID_OPERATION,
                 "attention: per-sequence positions need one query per sequence");
     const int T = positions_dev ? max_keys : q_pos0 + I;
@@ -820,6 +821,8 @@ extern "C" int32_t tlc_attention_decode_static(void *stream, const void *q_dev, 
     TLC_REQUIRE(D == 64 || D == 128, TLC_ERR_INVALID_OPERATION, "attention: head_dim %d unsupported (64, 128)", D);
     TLC_REQUIRE(max_keys >= 1 && max_keys <= max_seq, TLC_ERR_INDEX, "Index out of bounds: index %d, size %d", max_keys,
                 max_seq);
+    TLC_REQUIRE(((uintptr_t)q_dev & 3) == 0 && (((uintptr_t)k_cache_dev | (uintptr_t)v_cache_dev) & 15) == 0,
+                TLC_ERR_INVALID_OPERATION, "attention_decode_static: queries must be 4-byte, caches 16-byte aligned");
     int device = 0;
     TLC_CUDA(cudaGetDevice(&device));
     TLC_REQUIRE(device >= 0 && device < 64, TLC_ERR_DEVICE, "device ordinal %d out of range", device);

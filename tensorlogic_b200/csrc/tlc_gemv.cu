@@ -556,6 +556,9 @@ int32_t tlc_launch_gemv(tlc_ctx *ctx, const tlc_gemv_args &a) {
 
     if (tlc_gemm_eligible(ctx, a)) return tlc_launch_gemm(ctx, a);
 
+    // (a lane's eight values of a block: two 8-byte pieces of Q4_0, one of 16 bytes of Q8_0)
+    TLC_REQUIRE((((uintptr_t)a.x | (uintptr_t)a.norm_w) & (type == TLC_TYPE_Q4_0 ? 7 : 15)) == 0, TLC_ERR_INVALID_OPERATION,
+                "linear: activations and norm weights must be %d-byte aligned", type == TLC_TYPE_Q4_0 ? 8 : 16);
     // (more than sixteen rows, where tlc_gemm_eligible leaves them here: passes over the weights)
     const int64_t nt2_tiles = kMaxCluster * (type == TLC_TYPE_Q4_0 ? max_window<TLC_TYPE_Q4_0>(2, 16) : max_window<TLC_TYPE_Q8_0>(2, 16));
     const int max_m = w0->k_tiles <= nt2_tiles ? 16 : 8;

@@ -421,3 +421,44 @@ def test_split_k_for_many_rows_of_a_wide_input(dev, ref, qtype, n, k):
             want_q = ref.rope(ref.linear_q(qtype, raw, n, k, xn).reshape(m, n // 64, 64), 0, 10000, positions=pos).reshape(m, n)
             assert rel_l2(q.numpy(), want_q) < 2 * TIGHT
             assert rel_l2(v.numpy(), ref.linear_q(qtype, raw2, n, k, xn)) < 2 * TIGHT
+
+
+@pytest.mark.parametrize("qtype,align", [(Q4, 8), (Q8, 16), (14, 16)])
+@pytest.mark.parametrize("m", [1, 5, 16, 20])
+def test_misaligned_activations_are_refused(dev, qtype, align, m):
+    """Addresses the vector loads cannot take are an error from the host, with nothing launched; the smallest
+    alignment they can take works."""
+    import ctypes as C
+    from tensorlogic_b200 import _lib
+    from tensorlogic_b200.api import KVCache, QTensor, TensorError, check
+    n, k = 64, 256
+    if qtype == 14:
+        rng = np.random.default_rng(1)
+        raw = rng.integers(0, 256, (n, 210), dtype=np.uint8)
+        raw[:, 208:210] = np.full((n, 1), 1e-5, np.float16).view(np.uint8)
+    else:
+        raw = _weights(qtype, n, k, seed=9)
+    w = QTensor.from_blocks(dev, qtype, n, k, raw)
+    x = _x(m, k, seed=9)
+    flat = lambda off: dev.tensor(np.concatenate([np.zeros(off // 2, np.float16), x.ravel()]))
+    y, nw = dev.empty((m, n)), dev.tensor(np.ones(k + 8, np.float16))
+    run = lambda xp: check(dev.lib.tlc_linear(dev.handle, w.handle, xp, m, k, y.ptr, None))
+    run(flat(0).ptr)
+    want = y.numpy()
+    for off in (2, align // 2):
+        x_off, before = flat(off), dev.launch_count
+        with pytest.raises(TensorError) as e:
+            run(x_off.ptr + off)
+        assert e.value.code == _lib.ERR_INVALID_OPERATION and dev.launch_count == before
+    x_off = flat(align)
+    run(x_off.ptr + align)
+    assert np.array_equal(y.numpy().view(np.uint16), want.view(np.uint16))
+    if qtype != 14 and m <= 16:
+        wh, yh, rh = (C.c_void_p * 1)(w.handle), (C.c_void_p * 1)(y.ptr), (C.c_int32 * 1)(0)
+        x0, before = flat(0), dev.launch_count
+        with pytest.raises(TensorError):
+            check(dev.lib.tlc_norm_linear_multi(dev.handle, 1, wh, yh, rh, x0.ptr, m, nw.ptr + 2, 1e-5, 0, 10000, None))
+        assert dev.launch_count == before
+    cache, q = KVCache(dev, 1, 1, 64, max_seq=16), dev.tensor(np.zeros(65, np.float16))
+    with pytest.raises(TensorError):
+        check(dev.lib.tlc_attention(dev.handle, cache.handle, 0, q.ptr + 2, y.ptr, 1, 1, 1, 0, None, 1, 0.125))
