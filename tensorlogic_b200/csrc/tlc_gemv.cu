@@ -110,6 +110,39 @@ __global__ void __launch_bounds__(256) linear_f16_kernel(const uint8_t *__restri
     }
 }
 
+// Q6_K rows of more than 65536 columns, whose activations a launch of the GEMV cannot hold: one warp per output row,
+// any K and any number of activation rows, the arithmetic of the GEMV (integers times the group's scale, f32 sums).
+__global__ void __launch_bounds__(256) linear_q6k_long_kernel(const uint8_t *__restrict__ w, size_t pitch, int n_rows, int k,
+                                                              const __half *x, int m, __half *__restrict__ y, const __half *bias,
+                                                              const __half *residual) {
+    tlc_pdl_after_wait();
+    const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (row >= n_rows) return;
+    for (int mm = 0; mm < m; mm++) {
+        const __half *xr = x + (size_t)mm * k + lane;
+        float acc = 0.f;
+        for (int sb = 0; sb < k >> 8; sb++) {
+            const uint8_t *blk = w + (size_t)row * pitch + (size_t)sb * 224;
+            const float d = __half2float(*reinterpret_cast<const __half *>(blk + 208));
+#pragma unroll
+            for (int g = 0; g < 8; g++) {  // elements 32 g + lane: half h, quarter j of it
+                const int h = g >> 2, j = g & 3;
+                const int lo = blk[64 * h + 32 * (j & 1) + lane] >> (j >= 2 ? 4 : 0) & 15, hi = blk[128 + 32 * h + lane] >> (2 * j) & 3;
+                const float scale = d * (float)reinterpret_cast<const int8_t *>(blk + 192)[8 * h + (lane >> 4) + 2 * j];
+                acc = fmaf(scale, (float)((lo | hi << 4) - 32) * __half2float(xr[sb * 256 + 32 * g]), acc);
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (lane == 0) {
+            __half v = __float2half_rn(acc);
+            if (bias) v = __hadd(v, bias[row]);
+            if (residual) v = __hadd(v, residual[(size_t)mm * n_rows + row]);
+            y[(size_t)mm * n_rows + row] = v;
+        }
+    }
+}
+
 // Second half of a split-K launch (GemvParams::ksplit > 1): one thread per output adds the K
 // windows' f32 shares in window order (so the result does not depend on scheduling) and applies
 // the epilogue of gemv_mma_kernel -- f16 rounding, then bias / residual / SiLU(gate)*up /
@@ -522,6 +555,18 @@ int32_t tlc_launch_gemv(tlc_ctx *ctx, const tlc_gemv_args &a) {
             x = static_cast<const __half *>(ctx->scratch);
         }
         TLC_REQUIRE(((uintptr_t)x & 15) == 0, TLC_ERR_INVALID_OPERATION, "linear: activations must be 16-byte aligned");
+        if (k / 256 > kMaxCluster * max_window<TLC_TYPE_Q6_K>(1, 16)) {
+            const cudaError_t le = tlc_launch_pdl(ctx, linear_q6k_long_kernel, dim3((unsigned)((w0->n_rows + 7) / 8)), dim3(256), 0,
+                                                  static_cast<const uint8_t *>(w0->data), w0->row_pitch, (int)w0->n_rows, (int)k, x, a.m,
+                                                  static_cast<__half *>(a.outs[0].y), static_cast<const __half *>(a.bias),
+                                                  a.epilogue == TLC_EPI_RESIDUAL ? static_cast<const __half *>(a.residual) : nullptr);
+            if (le != cudaSuccess) {
+                cudaGetLastError();
+                return tlc_fail(TLC_ERR_CUDA, "Q6_K linear launch failed: %s", cudaGetErrorString(le));
+            }
+            TLC_CHECK_LAUNCH(ctx);
+            return TLC_OK;
+        }
         // (Sixteen rows cost 1.6 times eight, so passes of sixteen: 32000 x 2048 at 17 / 19 / 24 / 32 rows takes 43.2 / 43.5 /
         // 45.3 / 54.5 us, in passes of eight 50.4 / 50.9 / 52.3 / 69.3.)
         constexpr int pass = 16;

@@ -43,7 +43,7 @@ def test_dependent_kernels_read_their_operands_through_plain_loads():
             seen.add(name)
             for p in params.split(","):
                 m = re.search(r"const\s+\w+\s*\*\s*__restrict__\s+(\w+)", p)
-                assert not m or (m.group(1) in WEIGHTS and name in ("linear_f16_kernel", "embed_kernel")), (path, name, p)
+                assert not m or (m.group(1) in WEIGHTS and name in ("linear_f16_kernel", "linear_q6k_long_kernel", "embed_kernel")), (path, name, p)
         for line in text.splitlines():  # (the GEMMs' producers and the one-row f16 linear: weight tiles and rows)
             if "__ldg(" in line:
                 assert re.search(r"__ldg\((?:reinterpret_cast<const \w+ \*>\()?(?:tile|wr) \+", line), (path, line)

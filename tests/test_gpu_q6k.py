@@ -127,3 +127,23 @@ def test_q6_k_fused_linear(dev, ref, n, k):
     nw = synth.norm_weight(3, "q6norm", k)
     (got,) = norm_linear_multi(dev.tensor(x), [w], dev.tensor(nw), 1e-5)
     assert rel_l2(got.numpy(), ref.linear_q(Q6K, raw, n, k, ref.rms_norm(x, nw, 1e-5))) < 2e-3
+
+
+@pytest.mark.parametrize("k", [65536, 65792])
+@pytest.mark.parametrize("m", [1, 3, 19])
+def test_q6_k_longest_rows(dev, ref, k, m):
+    """The longest K the tensor-core form holds, and the first beyond it, with bias, norm and residual."""
+    from tensorlogic_b200 import synth
+    from tensorlogic_b200.api import QTensor, linear, linear_residual, norm_linear_multi
+    n = 21
+    rng = np.random.default_rng(k + m)
+    raw = _q6k_blocks(rng, n, k, 1e-5, 1e-4)
+    w = QTensor.from_blocks(dev, Q6K, n, k, raw)
+    x = rng.standard_normal((m, k)).astype(np.float16)
+    want = ref.linear_q(Q6K, raw, n, k, x)
+    bias, res = rng.standard_normal(n).astype(np.float16), rng.standard_normal((m, n)).astype(np.float16)
+    assert rel_l2(linear(dev.tensor(x), w, dev.tensor(bias)).numpy(), ref.add(want, np.broadcast_to(bias, (m, n)))) < 2e-3
+    assert rel_l2(linear_residual(dev.tensor(x), w, dev.tensor(res)).numpy(), ref.add(res, want)) < 2e-3
+    nw = synth.norm_weight(3, "q6long", k)
+    (got,) = norm_linear_multi(dev.tensor(x), [w], dev.tensor(nw), 1e-5)
+    assert rel_l2(got.numpy(), ref.linear_q(Q6K, raw, n, k, ref.rms_norm(x, nw, 1e-5))) < 2e-3
