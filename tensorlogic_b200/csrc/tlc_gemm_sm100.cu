@@ -631,7 +631,8 @@ bool tlc_gemm_eligible(const tlc_ctx *ctx, const tlc_gemv_args &a) {
     // exact weights: outputs of less than half a wave of 128-row tiles, and a K that is short, or short for the
     // number of products, or so many outputs together that a wave has no room to share K out.  (8192 x 1024 at 17 /
     // 32 / 48 rows 10.4 / 12.6 / 19.4 us, GEMM 7.3 / 7.4 / 7.7; 2048 x 512 at 17 rows 6.6, GEMM 6.2.)
-    if (a.m > 48) return true;
+    // Nine and more rows of a K that no cluster of the GEMV holds the activations of (98304) have nowhere else to go.
+    if (a.m > 48 || (a.m > 8 && w0->k_tiles > tlc_gemv_max_tiles(w0->type))) return true;
     if (a.m <= 16) return false;
     const bool pair = a.epilogue == TLC_EPI_SWIGLU;
     int64_t widest = 0, outputs = 0, tiles = 0;

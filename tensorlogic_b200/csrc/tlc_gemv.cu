@@ -438,6 +438,10 @@ int32_t tlc_selftest_mbarrier_wait(tlc_ctx *ctx) {
     return TLC_OK;
 }
 
+int64_t tlc_gemv_max_tiles(int32_t type) {
+    return kMaxCluster * (type == TLC_TYPE_Q4_0 ? max_window<TLC_TYPE_Q4_0>(1, 16) : max_window<TLC_TYPE_Q8_0>(1, 16));
+}
+
 // Scratch the RMSNorm of 2..16 rows of width k takes (their fragment order).
 size_t tlc_gemv_scratch_bytes(int64_t k) { return frag_total_bytes(k / 32, 2); }
 
@@ -606,7 +610,8 @@ int32_t tlc_launch_gemv(tlc_ctx *ctx, const tlc_gemv_args &a) {
                 "linear: activations and norm weights must be %d-byte aligned", type == TLC_TYPE_Q4_0 ? 8 : 16);
     // (more than sixteen rows, where tlc_gemm_eligible leaves them here: passes over the weights)
     const int64_t nt2_tiles = kMaxCluster * (type == TLC_TYPE_Q4_0 ? max_window<TLC_TYPE_Q4_0>(2, 16) : max_window<TLC_TYPE_Q8_0>(2, 16));
-    const int max_m = w0->k_tiles <= nt2_tiles ? 16 : 8;
+    // (the longest K: even passes of up to eight rows, not eight and a last one, which the one-row kernel cannot hold)
+    const int passes = (a.m + 7) / 8, max_m = w0->k_tiles <= nt2_tiles ? 16 : (a.m + passes - 1) / passes;
     for (int m0 = 0; m0 < a.m; m0 += max_m) {
         const int mc = a.m - m0 < max_m ? a.m - m0 : max_m;
         GemvParams p{};

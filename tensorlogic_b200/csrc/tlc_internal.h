@@ -277,6 +277,8 @@ int32_t tlc_launch_gemm(tlc_ctx *ctx, const tlc_gemv_args &a);
 size_t tlc_gemm_scratch_bytes(const tlc_ctx *ctx, int m, int64_t k, int64_t n_total);
 // Adds the ksplit f32 shares in partial[ksplit][m][sum of N] and applies the epilogue of `a` (tlc_gemv.cu).
 int32_t tlc_gemv_splitk_finish(tlc_ctx *ctx, const tlc_gemv_args &a, int ksplit, float *partial);
+// Tiles along K of the longest Q4_0 / Q8_0 rows that 2 to 8 rows can be multiplied with on the GEMV.
+int64_t tlc_gemv_max_tiles(int32_t type);
 // Scratch the RMSNorm in front of a GEMV of 2..16 rows of width k takes.
 size_t tlc_gemv_scratch_bytes(int64_t k);
 

@@ -84,3 +84,16 @@ def test_weights_are_not_rounded(dev, qtype, m, n, k):
     x = synth.activations(7, f"nx{m}x{k}", (m, k))
     got = linear(dev.tensor(x), QTensor.from_blocks(dev, qtype, n, k, raw)).numpy()
     assert np.mean(got == _exact_product(qtype, raw, x)) > 0.95
+
+
+@pytest.mark.parametrize("qtype", [2, 8])
+@pytest.mark.parametrize("m,k", [(9, 65536), (16, 65664), (8, 98304), (9, 98304), (9, 98432), (16, 98432)])
+def test_longest_rows(dev, ref, qtype, m, k):
+    """K where sixteen rows no longer fit one launch, where eight do not, and beyond."""
+    from tensorlogic_b200 import synth
+    from tensorlogic_b200.api import QTensor, linear
+    n = 20
+    raw = synth.blocks(qtype, 6, synth.tensor_id(f"lr{k}"), n, k, scale_log2=-3 if qtype == 2 else -7)
+    x = synth.activations(6, f"lx{m}x{k}", (m, k))
+    got = linear(dev.tensor(x), QTensor.from_blocks(dev, qtype, n, k, raw)).numpy()
+    assert rel_l2(got, ref.linear_q(qtype, raw, n, k, x)) < TIGHT
