@@ -104,19 +104,13 @@ TLC_API int32_t tlc_destroy(tlc_ctx *ctx);
  *                 or kernel by kernel, five launches per layer (0, default: faster on a B200).
  *   "gemm_tma"    the GEMM's activation tiles arrive by TMA (1, default) or through cp.async
  *                 loader warps (0);
- *   "gemm_pg"     weight-producer groups of the GEMM: 0 (default) = two groups taking alternate K
- *                 steps where the K steps of a tile are shared out ("gemm_splitk"), one group
- *                 otherwise; 1 = one group and no sharing; 2 = two groups wherever possible;
  *   "perf"        per-op timing on (1) / off (0, default): see tlc_perf_report;
  *   "comm_ll"     peer-memory all-reduces of up to 262144 values send data and flag in one word and
  *                 poll the data (1, default) or use stores + fences + flags (0);
- *   "gemm_splitk" GEMMs of up to 128 activation rows whose weight gives fewer tiles than SMs share
- *                 the K steps over several CTAs per tile where a cost model says it pays, one finishing
- *                 kernel adds (1, default); 2 = wherever possible; 0 = off;
  *   "gemm_pair"   from 129 activation rows on, the GEMM runs on CTA pairs (tcgen05 cta_group::2,
  *                 persistent, two accumulators in tensor memory) (1) or on single CTAs (0,
  *                 default: faster on a B200);
- *   "gemm_wt_max_m" activation rows up to which quantized linears of 17 and more rows put the weight
+ *   "gemm_wt_max_m" activation rows up to which quantized linears on the GEMM put the weight
  *                 rows on the M side of the MMA (default: decided from the shape; the options above
  *                 that force a detail of the other form ask for that form);
  *   "gemm_wt_bn"  activation rows per tile of that form (a multiple of 16 up to 256; 0 = from the shape);
@@ -124,6 +118,9 @@ TLC_API int32_t tlc_destroy(tlc_ctx *ctx);
  *   "gemv_splitk" accepted and without effect: 2 to 16 rows always take one pass over the weights;
  *   "gemv_f8"     accepted and without effect: one row always runs on the f16 form;
  *   "l2_hint"     accepted and without effect: the weight copies always carry the evict-first L2 hint;
+ *   "gemm_splitk" accepted and without effect: the CTAs that share K add within a cluster or a stream
+ *                 ("gemm_wt_ks");
+ *   "gemm_pg"     (0, 1 or 2) accepted and without effect: one group of weight producers a CTA;
  *   "q6k_resident" Q6_K tensors stay quantized in HBM (1, default) or become f16 at upload (0);
  *   "attn_wide"   decode attention of one sequence with at most four KV heads over a long
  *                 context runs on clusters of sixteen key splits (1) or eight (0, default: no slower).

@@ -84,9 +84,7 @@ extern "C" int32_t tlc_init(int32_t ordinal, tlc_ctx **out) {
     if (const char *e = getenv("TLC_PERF")) ctx->perf = atoi(e) != 0;
     else if (getenv("TL_PERF")) ctx->perf = true;  // the reference's own switch
     if (const char *e = getenv("TLC_COMM_LL")) ctx->comm_ll = atoi(e) != 0;
-    if (const char *e = getenv("TLC_GEMM_SPLITK")) ctx->gemm_splitk = atoi(e);
     if (const char *e = getenv("TLC_GEMM_WT_MAX_M")) ctx->gemm_wt_max_m = atoi(e);
-    if (const char *e = getenv("TLC_GEMM_PG")) ctx->gemm_pg = atoi(e);
     if (const char *e = getenv("TLC_GEMM_TMA")) ctx->gemm_tma = atoi(e) != 0;
     if (const char *e = getenv("TLC_ATTN_WIDE")) ctx->attn_wide = atoi(e);
     if (const char *e = getenv("TLC_HOST_GRAPH")) ctx->host_graph = atoi(e) != 0;
@@ -115,11 +113,8 @@ extern "C" int32_t tlc_set_option(tlc_ctx *ctx, const char *name, int64_t value)
         ctx->perf = value != 0;
     else if (n == "comm_ll")
         ctx->comm_ll = value != 0;
-    else if (n == "gemm_splitk")
-        ctx->gemm_splitk = (int)value;
     else if (n == "gemm_pg") {
         TLC_REQUIRE(value >= 0 && value <= 2, TLC_ERR_INVALID_OPERATION, "set_option: gemm_pg must be 0, 1 or 2");
-        ctx->gemm_pg = (int)value;
     } else if (n == "gemm_wt_bn") {
         TLC_REQUIRE(value >= 0 && value <= 256 && value % 16 == 0, TLC_ERR_INVALID_OPERATION,
                     "set_option: gemm_wt_bn must be a multiple of 16 up to 256");
@@ -144,7 +139,7 @@ extern "C" int32_t tlc_set_option(tlc_ctx *ctx, const char *name, int64_t value)
         ctx->host_poll = value != 0;
     else if (n == "step_kernel")
         ctx->step_kernel = value != 0;
-    else if (n == "gemv_f8" || n == "gemv_splitk" || n == "l2_hint")
+    else if (n == "gemv_f8" || n == "gemv_splitk" || n == "l2_hint" || n == "gemm_splitk")
         ;  // forms that no longer exist (see the header)
     else if (n == "q6k_resident")
         ctx->q6k_resident = value != 0;

@@ -155,118 +155,11 @@ __device__ __forceinline__ void produce_b(const GemmParams &p, uint8_t *btiles, 
     }
 }
 
-// B producer for the form with two producer groups (PG = 2): the warps of group g fill the K
-// steps kt = g, g + 2, ...  A thread still owns one weight row, but only every other ring stage,
-// so twice as many warps share the dequantization of a K step sequence: the per-step latency of
-// the producers, which bounds the GEMM when the tensor cores have little to do (one sub-tile of
-// activation rows), halves.  Per own step a thread fetches its row's quants (32 bytes of Q4_0 in
-// four 8-byte loads, 64 bytes of Q8_0) and scale word two own steps ahead.
-template <int QT, int STAGES, int STAGE_BYTES>
-__device__ __forceinline__ void produce_b_alt(const GemmParams &p, uint8_t *btiles, uint64_t *full, uint64_t *empty,
-                                              volatile int *abort_flag, const uint8_t *wbase, int wrow, int row, int KT,
-                                              int lane, int group, int kt0) {
-    // KT: K steps of this CTA, the first one being step kt0 of the weight (split K)
-    constexpr int TILE = QT == TLC_TYPE_Q4_0 ? 1152 : 1088;
-    constexpr int PF = 2;                             // own steps fetched ahead
-    constexpr int QW = QT == TLC_TYPE_Q4_0 ? 8 : 16;  // quant words of a row per K step
-    const bool row_ok = wrow < p.n;
-    const int r16 = wrow & 15;
-    const uint8_t *slab = wbase + (size_t)(row_ok ? wrow >> 4 : 0) * p.w_pitch;
-    const uint32_t qoff = (uint32_t)((r16 >> 3) * 512 + (r16 & 7) * 64);
-    const uint32_t soff = 1024u + (uint32_t)r16 * (QT == TLC_TYPE_Q4_0 ? 8u : 4u);
-    uint32_t piece[8];
-#pragma unroll
-    for (int j = 0; j < 8; j++) piece[j] = (uint32_t)(row * 128 + ((j ^ (row & 7)) << 4));
-    uint32_t qn[PF][QW], sn[PF];
-    auto fetch = [&](int kl, uint32_t (&qw)[QW], uint32_t &sc) {
-        const int kt = kt0 + kl;
-        const int wt = QT == TLC_TYPE_Q4_0 ? kt >> 1 : kt;
-        const bool ok = row_ok && kl < KT && wt < p.k_tiles;
-        const uint8_t *tile = slab + (size_t)(ok ? wt : 0) * TILE;
-        if (QT == TLC_TYPE_Q4_0) {
-            const int half = kt & 1;  // which pair of the tile's four blocks
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const uint2 v = ok ? __ldg(reinterpret_cast<const uint2 *>(tile + qoff + 16 * i + 8 * half)) : make_uint2(0, 0);
-                qw[2 * i] = v.x;
-                qw[2 * i + 1] = v.y;
-            }
-            sc = ok ? __ldg(reinterpret_cast<const uint32_t *>(tile + soff + 4 * half)) : 0u;
-        } else {
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const uint4 v = ok ? __ldg(reinterpret_cast<const uint4 *>(tile + qoff) + i) : make_uint4(0, 0, 0, 0);
-                qw[4 * i] = v.x;
-                qw[4 * i + 1] = v.y;
-                qw[4 * i + 2] = v.z;
-                qw[4 * i + 3] = v.w;
-            }
-            sc = ok ? __ldg(reinterpret_cast<const uint32_t *>(tile + soff)) : 0u;
-        }
-    };
-#pragma unroll
-    for (int u = 0; u < PF; u++) fetch(group + 2 * u, qn[u], sn[u]);
-#pragma unroll 1
-    for (int base = group; base < KT; base += 2 * PF) {
-#pragma unroll
-        for (int u = 0; u < PF; u++) {
-            const int kt = base + 2 * u;
-            if (kt >= KT) break;
-            uint32_t cw[QW];
-#pragma unroll
-            for (int i = 0; i < QW; i++) cw[i] = qn[u][i];
-            const uint32_t scw = sn[u];
-            fetch(kt + 2 * PF, qn[u], sn[u]);
-            const int s = kt % STAGES;
-            mbar_wait(&empty[s], ((kt / STAGES) & 1u) ^ 1u, abort_flag, p.status, 15, p.wait_ns);
-            uint8_t *bt = btiles + (size_t)s * STAGE_BYTES;
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const __half d = __ushort_as_half((unsigned short)(e == 0 ? scw & 0xFFFFu : scw >> 16));
-                if (QT == TLC_TYPE_Q4_0) {
-                    uint32_t qb[4];
-#pragma unroll
-                    for (int i = 0; i < 4; i++) qb[i] = cw[2 * i + e];
-                    dequant_block<QT>(qb, d, bt, piece, e);
-                } else {
-                    uint32_t qb[8];
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        qb[2 * i] = cw[4 * i + 2 * e];
-                        qb[2 * i + 1] = cw[4 * i + 2 * e + 1];
-                    }
-                    dequant_block<QT>(qb, d, bt, piece, e);
-                }
-            }
-            fence_async_proxy();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&full[s]);
-        }
-    }
-}
-
 // SW: the SiLU.mul pair.  The weight tile holds 128 rows of the gate weight (tile rows
 // 0-127) and the same 128 rows of the up weight (tile rows 128-255); the epilogue reads
 // both accumulators and stores silu(gate) * up for the 128 output columns of the CTA.
-// 32 consecutive f32 accumulators of one activation row to the split-K partial sums.
-__device__ __forceinline__ void store_partial(float *dst, const uint32_t (&r)[32], bool ok, bool vec, int left) {
-    if (!ok) return;
-    if (vec) {
-#pragma unroll
-        for (int v = 0; v < 8; v++)
-            *reinterpret_cast<uint4 *>(dst + 4 * v) = make_uint4(r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3]);
-    } else {
-#pragma unroll
-        for (int e = 0; e < 32; e++)
-            if (e < left) dst[e] = __uint_as_float(r[e]);
-    }
-}
-
-// PG: producer groups.  1: the 4*NT producer warps fill every K step.  2: twice the warps, each
-// group every other step (produce_b_alt) -- for tiles of one activation sub-tile, where the
-// producers and not the MMAs set the pace.
-template <int QT, int MT, int NT, bool SW, int PG>
-__global__ void __launch_bounds__(gemm_threads(NT, PG), 1)
+template <int QT, int MT, int NT, bool SW>
+__global__ void __launch_bounds__(gemm_threads(NT), 1)
     gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap x_map) {
     static_assert(!SW || NT == 2, "the gate/up pair fills a 256-row weight tile");
     constexpr int BN = 128 * NT;
@@ -275,7 +168,7 @@ __global__ void __launch_bounds__(gemm_threads(NT, PG), 1)
     constexpr int kStages = stages_for(MT, NT);
     constexpr uint32_t TMEM_COLS = MT * BN;  // 128, 256 or 512: a power of two
     constexpr uint32_t IDESC = idesc_for(BN);
-    constexpr int MMA_WARP = 4 + 4 * NT * PG;  // 12 with NT = 2, PG = 1 (eight producer warps) or NT = 1, PG = 2
+    constexpr int MMA_WARP = 4 + 4 * NT;
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t *tiles = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -287,15 +180,7 @@ __global__ void __launch_bounds__(gemm_threads(NT, PG), 1)
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int n0 = blockIdx.x * (SW ? 128 : BN), m0 = blockIdx.y * 128 * MT;
-    const int KT_all = (p.k + kBK - 1) / kBK;  // K is a multiple of 32: the last step may hold one block only
-    // split K (two-group form only): this CTA's share of the K steps, never empty
-    int kt0 = 0, KT = KT_all;
-    const bool split = PG == 2 && p.ksplit > 1;
-    if (split) {
-        const int per = (KT_all + p.ksplit - 1) / p.ksplit;
-        kt0 = (int)blockIdx.z * per;
-        KT = KT_all - kt0 < per ? KT_all - kt0 : per;
-    }
+    const int KT = (p.k + kBK - 1) / kBK;  // K is a multiple of 32: the last step may hold one block only
 
     if (tid == 0) {
         for (int s = 0; s < kStages; s++) {
@@ -320,15 +205,11 @@ __global__ void __launch_bounds__(gemm_threads(NT, PG), 1)
     const uint32_t tmem_base = *tmem_slot;
     tlc_pdl_prologue();  // x (and residual) come from the previous kernel of the stream
 
-    if (warp >= 4 && warp < 4 + 4 * NT * PG) {
+    if (warp >= 4 && warp < MMA_WARP) {
         const int trow = (tid - 128) % BN;  // row of the weight tile
         const uint8_t *wbase = SW && trow >= 128 ? p.w2 : p.w;
         const int wrow = SW ? n0 + (trow & 127) : n0 + trow;
-        if (PG == 1)
-            produce_b<QT, kStages, STAGE_BYTES>(p, tiles + A_BYTES, full, empty, abort_flag, wbase, wrow, trow, KT, lane);
-        else
-            produce_b_alt<QT, kStages, STAGE_BYTES>(p, tiles + A_BYTES, full, empty, abort_flag, wbase, wrow, trow, KT,
-                                                    lane, (tid - 128) / BN, kt0);
+        produce_b<QT, kStages, STAGE_BYTES>(p, tiles + A_BYTES, full, empty, abort_flag, wbase, wrow, trow, KT, lane);
     } else if (warp < 4 && p.a_tma) {
         // ------------------------------ A tile by TMA ------------------------------
         // One warp issues, per K step, MT boxes of 128 rows x 64 columns with the 128-byte
@@ -346,7 +227,7 @@ __global__ void __launch_bounds__(gemm_threads(NT, PG), 1)
                 mbar_arrive_expect_tx_el(&full[s], A_BYTES, el);
 #pragma unroll
                 for (int i = 0; i < MT; i++)
-                    tma_load_2d_el(abase + i * (128 * 128), &x_map, (kt0 + j) * kBK, m0 + 128 * i, bar, el);
+                    tma_load_2d_el(abase + i * (128 * 128), &x_map, j * kBK, m0 + 128 * i, bar, el);
                 if (++s == kStages) {
                     s = 0;
                     ph ^= 1u;
@@ -365,8 +246,8 @@ __global__ void __launch_bounds__(gemm_threads(NT, PG), 1)
             for (int it = 0; it < 8 * MT; it++) {
                 const int row = it * 16 + (tid >> 3), c = tid & 7;
                 // rows past M and, in a last step of one block, columns past K are zero-filled
-                const bool ok = m0 + row < p.m && (kt0 + j) * kBK + c * 8 < p.k;
-                const __half *src = p.x + (ok ? (size_t)(m0 + row) * p.k + (size_t)(kt0 + j) * kBK + c * 8 : 0);
+                const bool ok = m0 + row < p.m && j * kBK + c * 8 < p.k;
+                const __half *src = p.x + (ok ? (size_t)(m0 + row) * p.k + (size_t)j * kBK + c * 8 : 0);
                 cp_async16(abase + row * 128 + ((c ^ (row & 7)) << 4), src, ok);
             }
         };
@@ -418,8 +299,7 @@ __global__ void __launch_bounds__(gemm_threads(NT, PG), 1)
 
     // ------------------------------ epilogue ------------------------------
     // Warp w reads tensor-memory lanes 32*(w%4) .. +31 (= activation rows of a
-    // sub-tile); the warps of a lane quarter (three, or five with two producer groups of a
-    // 256-row weight tile) take the 32-column pieces in turn.
+    // sub-tile); the warps of a lane quarter (two or three) take the 32-column pieces in turn.
     if (warp < MMA_WARP) {
         mbar_wait(accum_bar, 0, abort_flag, p.status, 13, p.wait_ns);
         __syncwarp();  // the lanes leave a wait one by one; tcgen05.ld is for a whole warp
@@ -443,18 +323,6 @@ __global__ void __launch_bounds__(gemm_threads(NT, PG), 1)
             __half *ybase = p.y + (size_t)((long long)row * p.row_stride + (long long)pos * p.pos_stride);
             uint32_t r[32];
             tmem_ld32(tmem_base + ((uint32_t)(32 * wq) << 16) + (uint32_t)(BN * i + c0), r);
-            if (split) {
-                // this CTA's f32 share; the finishing kernel rounds and applies the epilogue
-                float *dst = p.partial + ((size_t)blockIdx.z * p.m + (row < p.m ? row : 0)) * p.ntot + p.noff + n0 + c0;
-                const bool ok = row < p.m && n0 + c0 < p.n;
-                const bool vec = ok && n0 + c0 + 32 <= p.n && ((p.ntot | p.noff | p.n) & 3) == 0;
-                store_partial(dst, r, ok, vec, p.n - (n0 + c0));
-                if (SW) {
-                    tmem_ld32(tmem_base + ((uint32_t)(32 * wq) << 16) + (uint32_t)(BN * i + 128 + c0), r);
-                    store_partial(dst + p.n, r, ok, vec, p.n - (n0 + c0));
-                }
-                continue;
-            }
             if (SW) {
                 // s = sigmoid(g) (f32, RNE); a = g*s; act = a*u: three f16 roundings as in
                 // debug/chat_demo_with_kvcache.tl:26-41 (the GEMV's SiLU.mul epilogue does the same)
@@ -475,29 +343,24 @@ __global__ void __launch_bounds__(gemm_threads(NT, PG), 1)
     }
 }
 
-template <int QT, int MT, int NT, bool SW, int PG>
-int32_t launch_tile_pg(tlc_ctx *ctx, const GemmParams &p) {
+template <int QT, int MT, int NT, bool SW = false>
+int32_t launch_tile(tlc_ctx *ctx, const GemmParams &p) {
     const size_t smem = smem_bytes(MT, NT);
     static bool configured[64] = {};
     if (!configured[ctx->device & 63]) {
-        TLC_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<QT, MT, NT, SW, PG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        TLC_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<QT, MT, NT, SW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)smem));
-        TLC_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<QT, MT, NT, SW, PG>,
+        TLC_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<QT, MT, NT, SW>,
                                       cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
         configured[ctx->device & 63] = true;
     }
     const int out_cols = SW ? 128 : 128 * NT;  // output columns per CTA
     GemmParams q = p;
-    if (PG != 2 || q.ksplit < 2) {  // split K exists in the two-group form only
-        q.ksplit = 1;
-        q.partial = nullptr;
-    }
-    const dim3 grid((unsigned)((p.n + out_cols - 1) / out_cols), (unsigned)((p.m + 128 * MT - 1) / (128 * MT)),
-                    (unsigned)q.ksplit);
+    const dim3 grid((unsigned)((p.n + out_cols - 1) / out_cols), (unsigned)((p.m + 128 * MT - 1) / (128 * MT)));
     CUtensorMap x_map;
     memset(&x_map, 0, sizeof x_map);
     q.a_tma = ctx->gemm_tma && encode_x_map(&x_map, p) ? 1 : 0;
-    cudaError_t le = tlc_launch_pdl(ctx, gemm_tcgen05_kernel<QT, MT, NT, SW, PG>, grid, dim3(gemm_threads(NT, PG)), smem, q,
+    cudaError_t le = tlc_launch_pdl(ctx, gemm_tcgen05_kernel<QT, MT, NT, SW>, grid, dim3(gemm_threads(NT)), smem, q,
                                     x_map);
     if (le != cudaSuccess) {
         cudaGetLastError();
@@ -505,16 +368,6 @@ int32_t launch_tile_pg(tlc_ctx *ctx, const GemmParams &p) {
     }
     TLC_CHECK_LAUNCH(ctx);
     return TLC_OK;
-}
-
-// Two producer groups (the form split K exists in) when the K steps of a tile are shared out, or
-// when option "gemm_pg" = 2 forces them; one group otherwise (1 = forced, and no split K).  On
-// unsplit launches two groups measured no faster (8192 -> 28672, 32 rows: 86 against 80 us).
-template <int QT, int MT, int NT, bool SW = false>
-int32_t launch_tile(tlc_ctx *ctx, const GemmParams &p) {
-    const bool two = MT == 1 && (ctx->gemm_pg == 2 || (ctx->gemm_pg == 0 && p.ksplit > 1));
-    if (two) return launch_tile_pg<QT, 1, NT, SW, 2>(ctx, p);
-    return launch_tile_pg<QT, MT, NT, SW, 1>(ctx, p);
 }
 
 template <int QT>
@@ -563,58 +416,9 @@ inline size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
 }  // namespace
 
-// Split K for the GEMM: with at most 128 activation rows a weight of few rows gives few CTAs (a
-// 2048-row projection: eight), each walking all of K at the producers' pace.  The K steps are
-// then shared out over gridDim.z CTAs per tile, at most enough to fill the SMs, at least eight
-// steps each; f32 shares go to scratch and gemv_splitk_finish_kernel finishes.  `tiles`: weight
-// tiles of 256 rows over all outputs of the call, `n_total`: their output columns.  1: no split.
-static int gemm_choose_ksplit(const tlc_ctx *ctx, int m, int64_t k, int64_t tiles, int64_t n_total) {
-    if (!ctx->gemm_splitk || m > 128 || ctx->gemm_pg == 1 || ctx->gemm_tile == 22 || tiles < 1) return 1;
-    const int KT = (int)((k + kBK - 1) / kBK);
-    int64_t ks_max = ctx->sm_count / tiles;
-    if (ks_max > KT / 8) ks_max = KT / 8;
-    if (ks_max > 16) ks_max = 16;
-    // Cost in microseconds: K steps of a CTA at 0.45 us, plus, when split, the finishing launch and
-    // the f32 shares written and read back (about 3 TB/s through the L2).  128 rows of a
-    // 2048 -> 8192 projection are faster unsplit (18 against 28 us), 32 rows split (18 against 30 us).
-    int best = 1;
-    double best_t = KT * 0.45;
-    for (int ks = 2; ks <= ks_max; ks++) {
-        const int per = (KT + ks - 1) / ks;
-        if ((KT + per - 1) / per != ks) continue;  // a share would be empty
-        const double t = per * 0.45 + 4.0 + (double)ks * m * (double)n_total * 8.0 / 3.0e6;
-        if (t < best_t || ctx->gemm_splitk == 2) {  // 2: the most shares, whatever they cost (tests)
-            best_t = t;
-            best = ks;
-        }
-    }
-    return best;
-}
-static int64_t gemm_tiles(const tlc_gemv_args &a) {
-    if (a.epilogue == TLC_EPI_SWIGLU) return (a.outs[0].w->n_rows + 127) / 128;
-    int64_t t = 0;
-    for (int i = 0; i < a.n_out; i++) t += (a.outs[i].w->n_rows + 255) / 256;
-    return t;
-}
-
-// Context scratch the GEMM form of a linear over m rows of width k with n_total outputs (all
-// outputs of a fused call; the SiLU.mul pair counts twice) may need: the normalized rows and
-// the split-K partial sums.  Callers that capture graphs reserve it up front.
-size_t tlc_gemm_scratch_bytes(const tlc_ctx *ctx, int m, int64_t k, int64_t n_total) {
-    const int mp = m < 128 ? m : 128;
-    // the most shares any row count and any tiling of n_total outputs can get, whatever the options
-    // say when the launch comes
-    int ks = 1;
-    {
-        const int KT = (int)((k + kBK - 1) / kBK);
-        const int64_t tiles = (n_total + 255) / 256 > 0 ? (n_total + 255) / 256 : 1;
-        int64_t ks_max = ctx->sm_count / tiles;
-        if (ks_max > KT / 8) ks_max = KT / 8;
-        if (ks_max > 16) ks_max = 16;
-        if (ks_max > 1) ks = (int)ks_max;
-    }
-    return align256((size_t)m * k * 2) + (ks > 1 ? align256((size_t)ks * mp * (size_t)n_total * sizeof(float)) : 0);
-}
+// Context scratch the GEMM form of a linear over m rows of width k may need: the normalised rows.
+// Callers that capture graphs reserve it up front.
+size_t tlc_gemm_scratch_bytes(int m, int64_t k) { return align256((size_t)m * k * 2); }
 
 bool tlc_gemm_eligible(const tlc_ctx *ctx, const tlc_gemv_args &a) {
     const tlc_qtensor *w0 = a.outs[0].w;
@@ -655,16 +459,12 @@ int32_t tlc_launch_gemm(tlc_ctx *ctx, const tlc_gemv_args &a) {
     const tlc_qtensor *w0 = a.outs[0].w;
     const int64_t k = w0->n_cols;
     const bool swiglu = a.epilogue == TLC_EPI_SWIGLU;
-    const size_t norm_bytes = a.norm_w ? align256((size_t)a.m * k * 2) : 0;
-    int64_t ntot = 0;
-    for (int i = 0; i < a.n_out; i++) ntot += a.outs[i].w->n_rows;
     // Which form: the one with 128 activation rows on the M side of the MMA (this file) moves half the
     // activation bytes per MMA, but only in 256 x 256 tiles, and pays off where these fill the waves of SMs:
     // 8192 -> 28672 at 256 rows (112 tiles) 112 us against 134, 4096 -> 4096 at 2048 rows (128) 57 against
     // 64; but 4096 -> 11008 at 1024 rows (172 tiles, 58 % of two waves) 124 us against 100.
     // (An option that forces a detail of that form asks for the form.)
-    bool wt = a.m <= ctx->gemm_wt_max_m && ctx->gemm_tile == 0 && !ctx->gemm_pair && ctx->gemm_pg == 0 && ctx->gemm_tma &&
-              ctx->gemm_splitk == 1;
+    bool wt = a.m <= ctx->gemm_wt_max_m && ctx->gemm_tile == 0 && !ctx->gemm_pair && ctx->gemm_tma;
     if (wt && ctx->gemm_wt_max_m == INT_MAX && a.m >= 192) {
         int64_t tiles = 0;
         for (int i = 0; i < a.n_out; i++) tiles = tiles > a.outs[i].w->n_rows ? tiles : a.outs[i].w->n_rows;
@@ -672,17 +472,11 @@ int32_t tlc_launch_gemm(tlc_ctx *ctx, const tlc_gemv_args &a) {
         const int64_t slots = (tiles + ctx->sm_count - 1) / ctx->sm_count * ctx->sm_count;
         wt = tiles < 100 || tiles * 10 < slots * 7;
     }
-    const int ksplit = wt ? 1 : gemm_choose_ksplit(ctx, a.m, k, gemm_tiles(a), ntot);
-    const size_t part_bytes = ksplit > 1 ? align256((size_t)ksplit * a.m * (size_t)ntot * sizeof(float)) : 0;
-    if (norm_bytes + part_bytes > 0)
-        if (int32_t rc = tlc_scratch_reserve(ctx, norm_bytes + part_bytes)) return rc;
-    uint8_t *scratch = static_cast<uint8_t *>(ctx->scratch);
-    float *partial = ksplit > 1 ? reinterpret_cast<float *>(scratch + norm_bytes) : nullptr;
-    int noff = 0;
     const __half *x = static_cast<const __half *>(a.x);
     if (a.norm_w) {
-        if (int32_t rc = tlc_launch_rms_norm(ctx, a.x, a.norm_w, scratch, a.m, (int32_t)k, a.eps, a.norm_early)) return rc;
-        x = reinterpret_cast<const __half *>(scratch);
+        if (int32_t rc = tlc_scratch_reserve(ctx, tlc_gemm_scratch_bytes(a.m, k))) return rc;
+        if (int32_t rc = tlc_launch_rms_norm(ctx, a.x, a.norm_w, ctx->scratch, a.m, (int32_t)k, a.eps, a.norm_early)) return rc;
+        x = static_cast<const __half *>(ctx->scratch);
     }
     TLC_REQUIRE(((uintptr_t)x & 15) == 0, TLC_ERR_INVALID_OPERATION, "gemm: activations must be 16-byte aligned");
     if (wt) {
@@ -724,13 +518,7 @@ int32_t tlc_launch_gemm(tlc_ctx *ctx, const tlc_gemv_args &a) {
         p.rope_base = (float)a.rope_base;
         p.vec_ok = ((p.row_stride | p.pos_stride | (long long)p.n) & 7) == 0 && ((uintptr_t)p.y & 15) == 0 &&
                    ((uintptr_t)p.residual & 15) == 0;
-        p.partial = partial;
-        p.ksplit = ksplit;
-        p.ntot = (int)ntot;
-        p.noff = noff;
-        noff += p.n;
         if (int32_t rc = launch_one(ctx, p, w->type)) return rc;
     }
-    if (ksplit > 1) return tlc_gemv_splitk_finish(ctx, a, ksplit, partial);
     return TLC_OK;
 }

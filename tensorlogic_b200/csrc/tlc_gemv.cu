@@ -49,20 +49,16 @@ namespace {
 // Generic path for dense f16 weights: any M, no alignment assumptions.  One
 // warp per output row -- correct but far from the roofline.
 // ---------------------------------------------------------------------------
-__global__ void linear_generic_kernel(const uint8_t *__restrict__ w, size_t pitch, int type, int n_rows,
-                                      int k, const __half *__restrict__ x, int m, __half *__restrict__ y,
+__global__ void linear_generic_kernel(const uint8_t *__restrict__ w, size_t pitch, int n_rows, int k, const __half *__restrict__ x, int m, __half *__restrict__ y,
                                       const __half *__restrict__ bias) {
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (warp >= n_rows) return;
-    const uint8_t *row = w + (size_t)warp * pitch;
+    const __half *wr = reinterpret_cast<const __half *>(w + (size_t)warp * pitch);
     for (int mm = 0; mm < m; mm++) {
         const __half *xr = x + (size_t)mm * k;
         float acc = 0.f;
-        if (type == TLC_TYPE_F16) {
-            const __half *wr = reinterpret_cast<const __half *>(row);
-            for (int i = lane; i < k; i += 32) acc = fmaf(__half2float(wr[i]), __half2float(xr[i]), acc);
-        }
+        for (int i = lane; i < k; i += 32) acc = fmaf(__half2float(wr[i]), __half2float(xr[i]), acc);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
         if (lane == 0) {
@@ -140,67 +136,6 @@ __global__ void __launch_bounds__(256) linear_q6k_long_kernel(const uint8_t *__r
             if (residual) v = __hadd(v, residual[(size_t)mm * n_rows + row]);
             y[(size_t)mm * n_rows + row] = v;
         }
-    }
-}
-
-// Second half of a split-K launch (GemvParams::ksplit > 1): one thread per output adds the K
-// windows' f32 shares in window order (so the result does not depend on scheduling) and applies
-// the epilogue of gemv_mma_kernel -- f16 rounding, then bias / residual / SiLU(gate)*up /
-// interleaved RoPE, dense or (sequence, position) addressing.
-__global__ void __launch_bounds__(256) gemv_splitk_finish_kernel(const GemvParams p) {
-    tlc_pdl_prologue();
-    const int nout = p.subs == 2 ? p.t[0].n : p.ntot;
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)p.m * nout) return;
-    const int col = (int)(i / nout), nn = (int)(i % nout);
-    int ti = 0, n = nn;
-    if (p.subs == 1) {
-        if (n >= p.t[0].n) { n -= p.t[0].n; ti = 1; }
-        if (ti == 1 && n >= p.t[1].n) { n -= p.t[1].n; ti = 2; }
-    }
-    const int noff = nn - n;
-    auto sum = [&](int off) {
-        float v = 0.f;
-#pragma unroll 4
-        for (int w = 0; w < p.ksplit; w++) v += p.partial[((size_t)w * p.m + col) * p.ntot + off];
-        return v;
-    };
-    const int wn = ti == 0 ? p.t[0].n : ti == 1 ? p.t[1].n : p.t[2].n;
-    __half *yout = ti == 0 ? p.t[0].y : ti == 1 ? p.t[1].y : p.t[2].y;
-    const long long rstride = ti == 0 ? p.t[0].row_stride : ti == 1 ? p.t[1].row_stride : p.t[2].row_stride;
-    const long long pstride = ti == 0 ? p.t[0].pos_stride : ti == 1 ? p.t[1].pos_stride : p.t[2].pos_stride;
-    const int rheads = ti == 0 ? p.t[0].rope_heads : ti == 1 ? p.t[1].rope_heads : p.t[2].rope_heads;
-    const int hdim = ti == 0 ? p.t[0].head_dim : ti == 1 ? p.t[1].head_dim : p.t[2].head_dim;
-    __half h = __float2half_rn(sum(noff + n));
-    const size_t oidx = (size_t)col * wn + n;
-    const int pos = p.positions ? p.positions[col] : p.pos_offset + col;
-    const size_t yidx = (size_t)((long long)col * rstride + (long long)pos * pstride) + n;
-    if (pstride != 0 && p.max_pos > 0 && (pos < 0 || pos >= p.max_pos)) {
-        if (atomicCAS(&p.status->code, 0, TLC_DEV_INDEX) == 0) p.status->where = 302;
-        return;
-    }
-    if (rheads > 0) {
-        const __half hp = __float2half_rn(sum(noff + (n ^ 1)));
-        const int dim = n % hdim;
-        const int pair = dim >> 1;
-        const float x0 = __half2float((dim & 1) ? hp : h);
-        const float x1 = __half2float((dim & 1) ? h : hp);
-        const float exponent = (float)(2 * pair) / (float)hdim;
-        const float freq = 1.0f / powf(p.rope_base, exponent);
-        const float theta = (float)(unsigned)pos * freq;
-        const float cs = cosf(theta), sn = sinf(theta);
-        const float r = (dim & 1) ? __fadd_rn(__fmul_rn(x0, sn), __fmul_rn(x1, cs))
-                                  : __fsub_rn(__fmul_rn(x0, cs), __fmul_rn(x1, sn));
-        yout[yidx] = __float2half_rn(r);
-    } else if (p.epilogue == TLC_EPI_RESIDUAL) {
-        yout[yidx] = __hadd(h, p.residual[oidx]);
-    } else if (p.epilogue == TLC_EPI_SWIGLU) {
-        const __half up = __float2half_rn(sum(p.t[0].n + n));
-        const __half sg = __float2half_rn(1.0f / (1.0f + expf(-__half2float(h))));
-        p.t[0].y[oidx] = __hmul(__hmul(h, sg), up);
-    } else {
-        if (p.bias) h = __hadd(h, p.bias[n]);
-        yout[yidx] = h;
     }
 }
 
@@ -445,43 +380,6 @@ int64_t tlc_gemv_max_tiles(int32_t type) {
 // Scratch the RMSNorm of 2..16 rows of width k takes (their fragment order).
 size_t tlc_gemv_scratch_bytes(int64_t k) { return frag_total_bytes(k / 32, 2); }
 
-int32_t tlc_gemv_splitk_finish(tlc_ctx *ctx, const tlc_gemv_args &a, int ksplit, float *partial) {
-    GemvParams p{};
-    p.n_out = a.n_out;
-    p.ntot = 0;
-    for (int i = 0; i < a.n_out; i++) {
-        const tlc_qtensor *w = a.outs[i].w;
-        p.t[i].n = (int)w->n_rows;
-        p.t[i].row_stride = a.outs[i].row_stride >= 0 ? a.outs[i].row_stride : (long long)w->n_rows;
-        p.t[i].pos_stride = a.outs[i].pos_stride;
-        p.t[i].y = static_cast<__half *>(a.outs[i].y);
-        p.t[i].rope_heads = a.outs[i].rope_heads;
-        p.t[i].head_dim = a.outs[i].rope_heads > 0 ? (int)(w->n_rows / a.outs[i].rope_heads) : 0;
-        p.ntot += p.t[i].n;
-    }
-    p.subs = a.epilogue == TLC_EPI_SWIGLU ? 2 : 1;
-    p.m = a.m;
-    p.epilogue = a.epilogue;
-    p.bias = static_cast<const __half *>(a.bias);
-    p.residual = static_cast<const __half *>(a.residual);
-    p.pos_offset = a.pos_offset;
-    p.rope_base = (float)a.rope_base;
-    p.positions = a.positions;
-    p.max_pos = a.max_pos;
-    p.status = ctx->dev_status;
-    p.ksplit = ksplit;
-    p.partial = partial;
-    const int nout = p.subs == 2 ? p.t[0].n : p.ntot;
-    const size_t total = (size_t)a.m * nout;
-    cudaError_t le = tlc_launch_pdl(ctx, gemv_splitk_finish_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, p);
-    if (le != cudaSuccess) {
-        cudaGetLastError();
-        return tlc_fail(TLC_ERR_CUDA, "split-K finish launch failed: %s", cudaGetErrorString(le));
-    }
-    TLC_CHECK_LAUNCH(ctx);
-    return TLC_OK;
-}
-
 int32_t tlc_launch_gemv(tlc_ctx *ctx, const tlc_gemv_args &a) {
     TLC_REQUIRE(a.n_out >= 1 && a.n_out <= 3, TLC_ERR_INVALID_OPERATION, "gemv: %d outputs", a.n_out);
     TLC_REQUIRE(a.m >= 1, TLC_ERR_INVALID_OPERATION, "gemv: m = %d", a.m);
@@ -528,7 +426,7 @@ int32_t tlc_launch_gemv(tlc_ctx *ctx, const tlc_gemv_args &a) {
         if (!vec) {
             TLC_REQUIRE(!residual, TLC_ERR_INVALID_OPERATION, "residual epilogue needs 16-byte aligned f16 rows");
             linear_generic_kernel<<<grid, threads, 0, ctx->stream>>>(
-                static_cast<const uint8_t *>(w0->data), w0->row_pitch, type, (int)w0->n_rows, (int)k, x, a.m,
+                static_cast<const uint8_t *>(w0->data), w0->row_pitch, (int)w0->n_rows, (int)k, x, a.m,
                 static_cast<__half *>(a.outs[0].y), static_cast<const __half *>(a.bias));
             TLC_CHECK_LAUNCH(ctx);
             return TLC_OK;

@@ -74,8 +74,8 @@ struct GemvParams {
     int pos_offset;
     float rope_base;
     const int *positions;
-    int max_pos;   // > 0: positions of outputs addressed by position are brought into [0, max_pos) (the one-pass
-                   // kernel; the attention kernel reports them) or dropped with status TLC_DEV_INDEX (split-K finish)
+    int max_pos;   // > 0: positions of outputs addressed by position are brought into [0, max_pos) (the attention
+                   // kernel reports them)
     int nstages, stage_bytes;
     int contig;    // 1: each CTA takes a contiguous range of units, 0: units blockIdx.x, + gridDim.x, ...
     int pdl_mode;  // 1: let the next kernel be scheduled at once, 2: only when this CTA's last slab is done, 3: after this CTA's own dependency wait
@@ -86,10 +86,7 @@ struct GemvParams {
     int batch;  // slabs per cross-warp reduction
     alignas(64) unsigned char w_map[128];  // Q6_K: tensor map of the weight's rows, in 8-byte elements
     int round, n_rounds;  // cluster: slabs (of one CTA) per exchange, exchanges of a launch
-    // tlc_gemv_splitk_finish: f32 shares [ksplit][m][ntot] of a split-K GEMM
-    int ntot;
     int norm_early;  // one row: norm_w may be read before the dependency wait (tlc_gemv_args)
-    float *partial;
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -137,14 +134,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
     if (atomicCAS(&status->code, 0, 1) == 0) status->where = where;
     return false;
 }
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            smem_u32(dst)),
-        "l"(src), "r"(bytes), "r"(smem_u32(bar))
-        : "memory");
-}
-// The same copy with an L2 eviction hint: weight tiles are read once per launch, so they
+// A bulk copy with an L2 eviction hint: weight tiles are read once per launch, so they
 // are marked evict-first and leave the L2 to activations, norm weights and the KV cache.
 __device__ __forceinline__ uint64_t l2_evict_first_policy() {
     uint64_t pol;

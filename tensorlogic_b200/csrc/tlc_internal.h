@@ -80,12 +80,10 @@ struct tlc_ctx {
     uint64_t wait_ns = 2000000000ull;
     bool gemm_pair = false;  // GEMM tiles of 256 x 256 on CTA pairs (tcgen05 cta_group::2) from 129 rows on; measured slower
     bool comm_ll = true;  // peer-memory all-reduces of up to 256 Ki values use flagged words instead of fences + flags
-    int gemm_splitk = 1;  // GEMMs of up to 128 rows and few weight tiles share K over several CTAs per tile: 0 off, 1 where a cost model says it pays, 2 wherever possible
     // The form with the weight rows on the M side of the MMA (tlc_gemm_wt.cu): activation rows per tile
     // and CTAs per tile (9: the stream form), 0 = from the shape (tests force the others).
     int gemm_wt_bn = 0, gemm_wt_ks = 0;
     int gemm_wt_max_m = INT_MAX;  // activation rows up to which quantized linears take that form (INT_MAX: by shape)
-    int gemm_pg = 0;  // producer groups of the GEMM: 0 = two where K is shared out over CTAs, else one; 1 / 2 = forced
     bool gemm_tma = true;  // activation tiles of the GEMM by TMA (false: cp.async loader warps)
     int gemm_tile = 0;  // 0: pick the GEMM tile from the shape; 11, 12, 22: force 128x128, 128x256, 256x256
     // Option "q6k_resident" / TLC_Q6K_RESIDENT=0: Q6_K tensors are expanded to f16 at upload (what
@@ -260,9 +258,9 @@ struct tlc_gemv_args {
     uint32_t rope_base = 10000;
     const int32_t *positions = nullptr;  // device int32 [m] or null
     // Outputs addressed by position (pos_stride != 0, a KV cache): a position outside [0, max_pos)
-    // never reaches memory outside the cache -- the one-pass GEMV stores at the last row instead (the
-    // attention kernel that follows reports the position), the split-K finish and the GEMM drop the
-    // row and raise TLC_DEV_INDEX themselves.  0: no limit.
+    // never reaches memory outside the cache -- the GEMV stores at the last row instead (the attention
+    // kernel that follows reports the position), the GEMM drops the row and raises TLC_DEV_INDEX
+    // itself.  0: no limit.
     int32_t max_pos = 0;
 };
 
@@ -272,11 +270,9 @@ int32_t tlc_launch_gemv(tlc_ctx *ctx, const tlc_gemv_args &a);
 // tlc_launch_gemv forwards to it when tlc_gemm_eligible says so.
 bool tlc_gemm_eligible(const tlc_ctx *ctx, const tlc_gemv_args &a);
 int32_t tlc_launch_gemm(tlc_ctx *ctx, const tlc_gemv_args &a);
-// Scratch the GEMM path needs for m rows of width k with a fused RMSNorm and a
-// SiLU.mul pair of n_swiglu outputs (reserve it before capturing a graph).
-size_t tlc_gemm_scratch_bytes(const tlc_ctx *ctx, int m, int64_t k, int64_t n_total);
-// Adds the ksplit f32 shares in partial[ksplit][m][sum of N] and applies the epilogue of `a` (tlc_gemv.cu).
-int32_t tlc_gemv_splitk_finish(tlc_ctx *ctx, const tlc_gemv_args &a, int ksplit, float *partial);
+// Scratch the GEMM path needs for m rows of width k with a fused RMSNorm (reserve it before
+// capturing a graph).
+size_t tlc_gemm_scratch_bytes(int m, int64_t k);
 // Tiles along K of the longest Q4_0 / Q8_0 rows that 2 to 8 rows can be multiplied with on the GEMV.
 int64_t tlc_gemv_max_tiles(int32_t type);
 // Scratch the RMSNorm in front of a GEMV of 2..16 rows of width k takes.

@@ -531,20 +531,8 @@ extern "C" int32_t tlc_llama_create(tlc_ctx *ctx, tlc_model *model, const tlc_ll
     }
     // The tensor-core path of the linears (many rows) works through scratch;
     // reserve it now so that no allocation happens inside a graph capture.
-    {
-        const int64_t kmax = d > qd ? d : qd;
-        {
-            const int64_t shapes[][2] = {{d, qd + 2 * kvd}, {qd, d}, {d, 2 * (int64_t)L->ffn_local}, {L->ffn_local, d},
-                                         {d, L->vocab_local}};
-            size_t need = tlc_gemm_scratch_bytes(ctx, L->max_rows, kmax, 0);
-            for (auto &sh : shapes) {
-                const size_t b = tlc_gemm_scratch_bytes(ctx, L->max_rows, sh[0], sh[1]);
-                need = b > need ? b : need;
-            }
-            need = tlc_gemv_scratch_bytes(d) > need ? tlc_gemv_scratch_bytes(d) : need;
-            if (int32_t rc = tlc_scratch_reserve(ctx, need)) return rc;
-        }
-    }
+    const size_t gemm_need = tlc_gemm_scratch_bytes(L->max_rows, d), gemv_need = tlc_gemv_scratch_bytes(d);
+    if (int32_t rc = tlc_scratch_reserve(ctx, gemm_need > gemv_need ? gemm_need : gemv_need)) return rc;
     // Same shared-memory carve-out as the GEMV and attention kernels they run between.
     TLC_CUDA(cudaFuncSetAttribute(embed_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                   cudaSharedmemCarveoutMaxShared));

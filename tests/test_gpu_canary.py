@@ -1,8 +1,8 @@
 """Out-of-bounds stand-in for a memory checker: every output of the linear paths is written into
 the middle of a larger buffer whose guard bands (one output row's worth before, a row plus 64
 elements after) hold a bit pattern no kernel produces.  After the call the bands must be intact and
-the interior must match the oracle -- for ragged N and M on the GEMV (one pass, split K), the tcgen05
-GEMM (single CTA, split K, CTA pairs) and the fused epilogues."""
+the interior must match the oracle -- for ragged N and M on the GEMV (one pass, several, clusters), the tcgen05
+GEMM (single CTA, K shared over CTAs, CTA pairs) and the fused epilogues."""
 import ctypes as C
 
 import numpy as np
@@ -58,7 +58,7 @@ def test_linear_writes_only_its_output(dev, ref, qtype, n, k, m):
 def test_fused_epilogues_write_only_their_output(dev, ref, qtype, m):
     from tensorlogic_b200 import synth
     from tensorlogic_b200.api import QTensor, check
-    n, k = 328, 2048                     # ragged N (not a multiple of 16), K wide enough for split K
+    n, k = 328, 2048                     # ragged N (not a multiple of 16), K wide enough to be shared over CTAs
     raw = synth.blocks(qtype, 42, synth.tensor_id("cg"), n, k, scale_log2=-3)
     raw2 = synth.blocks(qtype, 42, synth.tensor_id("cu"), n, k, scale_log2=-3)
     w, w2 = QTensor.from_blocks(dev, qtype, n, k, raw), QTensor.from_blocks(dev, qtype, n, k, raw2)

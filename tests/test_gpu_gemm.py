@@ -107,17 +107,13 @@ def test_every_tile_shape(dev, ref, qtype, tile, n, k, m):
     want_t = ref.dequant(qtype, raw, n * k).reshape(n, k).T[:m]
     dev.set_option("gemm_tile", tile)
     try:
-        # one producer group, and (tiles of one activation sub-tile) two groups taking alternate K steps
-        for pg in (1, 2):
-            dev.set_option("gemm_pg", pg)
-            with gemm_from(dev, 1):
-                y = linear(dev.tensor(x), w).numpy()
-                yt = linear(dev.tensor(np.eye(k, dtype=np.float16)[:m]), w).numpy()
-            assert rel_l2(y, want) < TIGHT, pg
-            assert np.array_equal(_bits(yt), _bits(want_t)), pg
+        with gemm_from(dev, 1):
+            y = linear(dev.tensor(x), w).numpy()
+            yt = linear(dev.tensor(np.eye(k, dtype=np.float16)[:m]), w).numpy()
+        assert rel_l2(y, want) < TIGHT
+        assert np.array_equal(_bits(yt), _bits(want_t))
     finally:
         dev.set_option("gemm_tile", 0)
-        dev.set_option("gemm_pg", 0)
 
 
 @pytest.mark.parametrize("qtype", [Q4, Q8])
@@ -153,33 +149,29 @@ def test_cta_pair_tiles(dev, ref, qtype, n, k, m):
 @pytest.mark.parametrize("qtype", [Q4, Q8])
 @pytest.mark.parametrize("n,k,m", [(512, 2048, 100), (200, 4096, 37), (2048, 8192, 128), (96, 1088, 64), (300, 1056, 17)])
 def test_gemm_split_k(dev, ref, qtype, n, k, m):
-    """Up to 128 rows against a weight of few tiles: the K steps are shared out over several CTAs
-    per tile (f32 shares in scratch, one finishing kernel).  Same answer as the oracle and as the
-    unsplit GEMM (option gemm_splitk = 0); ragged N, K with a last step of one block, uneven shares."""
+    """Up to 128 rows against a weight of few tiles: the K steps are shared out over the CTAs of a cluster that add
+    their f32 sums.  Eight CTAs a tile, one, and the choice by cost give the oracle's answer in one launch; ragged N, K
+    with a last step of one block, uneven shares."""
     from tensorlogic_b200.api import QTensor, linear
     raw = _weights(qtype, n, k, seed=21, name=f"s{n}x{k}")
     x = _x(m, k, seed=21, name=f"sx{m}x{k}")
     w = QTensor.from_blocks(dev, qtype, n, k, raw)
     want = ref.linear_q(qtype, raw, n, k, x)
+    got = {}
     with gemm_from(dev, 1):
-        try:
-            dev.set_option("gemm_splitk", 2)  # share K wherever possible, also where the cost model would not
-            l0 = dev.launch_count
-            y = linear(dev.tensor(x), w).numpy()
-            launches = dev.launch_count - l0
-            yt = linear(dev.tensor(np.eye(k, dtype=np.float16)[:m]), w).numpy()
-            dev.set_option("gemm_splitk", 1)  # the default: by cost
-            y2 = linear(dev.tensor(x), w).numpy()
-            dev.set_option("gemm_splitk", 0)
-            l0 = dev.launch_count
-            y1 = linear(dev.tensor(x), w).numpy()
-            assert dev.launch_count - l0 == 1
-        finally:
-            dev.set_option("gemm_splitk", 1)
-    assert launches == 2, launches            # the GEMM with K shared out + the finishing kernel
-    assert rel_l2(y2, want) < TIGHT
-    assert rel_l2(y, want) < TIGHT and rel_l2(y1, want) < TIGHT
-    assert rel_l2(y, y1) < 1e-4
+        for ks in (8, 1, 0):
+            dev.set_option("gemm_wt_ks", ks)
+            try:
+                l0 = dev.launch_count
+                got[ks] = linear(dev.tensor(x), w).numpy()
+                assert dev.launch_count - l0 == 1
+                if ks == 8:
+                    yt = linear(dev.tensor(np.eye(k, dtype=np.float16)[:m]), w).numpy()
+            finally:
+                dev.set_option("gemm_wt_ks", 0)
+    for ks, y in got.items():
+        assert rel_l2(y, want) < TIGHT, ks
+    assert rel_l2(got[8], got[1]) < 1e-4
     assert np.array_equal(_bits(yt), _bits(ref.dequant(qtype, raw, n * k).reshape(n, k).T[:m]))
 
 
@@ -187,7 +179,7 @@ def test_gemm_split_k(dev, ref, qtype, n, k, m):
 @pytest.mark.parametrize("n,k,m", [(300, 640, 300), (512, 2048, 100), (2100, 96, 2500), (64, 1376, 40)])
 def test_gemm_with_cp_async_activation_loaders(dev, ref, qtype, n, k, m):
     """Option gemm_tma = 0: four warps copy the activation tile with cp.async instead of the TMA
-    boxes (the path taken when no tensor map can be made); one and two producer groups, split K."""
+    boxes (the path taken when no tensor map can be made)."""
     from tensorlogic_b200.api import QTensor, linear
     raw = _weights(qtype, n, k, seed=22, name=f"c{n}x{k}")
     x = _x(m, k, seed=22, name=f"cx{m}x{k}")
@@ -265,8 +257,12 @@ def test_fused_contract_on_cta_pairs(dev, ref, qtype):
 
 @pytest.mark.parametrize("qtype", [Q4, Q8])
 def test_fused_contract_on_split_k_gemm(dev, ref, qtype):
-    """The same contract with K = 2048 and 45 rows: every GEMM of it shares K over several CTAs."""
-    _fused_contract(dev, qtype, 45, d=2048)
+    """The same contract with K = 2048 and 45 rows, K shared over the four CTAs of a cluster in every GEMM of it."""
+    dev.set_option("gemm_wt_ks", 4)
+    try:
+        _fused_contract(dev, qtype, 45, d=2048)
+    finally:
+        dev.set_option("gemm_wt_ks", 0)
 
 
 def _fused_contract(dev, qtype, m, d=256):
