@@ -5,6 +5,7 @@ measured configurations themselves:
 
   * the TinyLlama-1.1B shape with a 512-token prompt and 128 greedy decode steps (every one of
     the 129 logit rows is compared);
+  * the same shape in Q8_0, decode steps of 1 to 22 sequences;
   * the Llama-2-7B-shape prefill GEMMs at 2048 activation rows, whole and as 8-way
     tensor-parallel shards, on sub-sampled outputs;
   * one Llama-2-70B-shape layer plus an lm_head shard, unsharded through the runner (prefill,
@@ -99,6 +100,28 @@ def test_tinyllama_512_token_prompt_and_128_greedy_steps(dev, ref):
         top2 = np.partition(w, -2)[-2:]
         if top2[1] - top2[0] > 2 * float(np.abs(got[r].astype(np.float32) - w).max()):
             assert ref.argmax_last(want[r]) == toks[r], r
+
+
+def test_tinyllama_q8_0_several_sequences(dev, ref):
+    """The TinyLlama shape in Q8_0, decode steps of 1, 5, 16 and 22 sequences (one row, one and two tiles of rows, the
+    GEMM): every logit row against the oracle.  The oracle multiplies weights rounded to f16, as the reference's loader
+    keeps them; what that makes of the logits over 22 layers is the same for every number of rows, so no row may be
+    off by more than twice what a single sequence is (the order of the sums differs)."""
+    from tensorlogic_b200 import synth
+    from tensorlogic_b200.model import TINYLLAMA, Llama, synthetic_host_weights, synthetic_model
+    arch, seed = TINYLLAMA, 6
+    oracle = _ref_model(ref, synthetic_host_weights(arch, seed=seed, qtype=8), arch)
+    llm = Llama(dev, synthetic_model(dev, arch, seed=seed, qtype=8), arch, max_seq=64, max_batch=22)
+    one = 0.0
+    for B in (1, 5, 16, 22):
+        caches = oracle.empty_caches(B)
+        llm.set_state([0] * B, [0] * B)
+        for step in range(3):
+            ids = synth.token_ids(seed, f"q8.{B}.{step}", B, arch.vocab)
+            lg, want = llm.decode(ids, return_logits=True)[1], oracle.forward_batch(ids, caches)
+            worst = max(rel_l2(lg[b], want[b]) for b in range(B))
+            one = max(one, worst) if B == 1 else one
+            assert worst < TOL and worst < 2 * one, (B, step, worst, one)
 
 
 def _sample(n, count, rng):
