@@ -398,11 +398,10 @@ def run_ours(args, rank: int, world: int, local: int) -> None:
         traffic, traffic_src = None, None
         tpath = os.path.join(ROOT, "profiles", "decode_step_traffic.json")
         if os.path.exists(tpath):
-            # DRAM bytes per decode step from one ncu capture of a short run of this workload
-            # (profiles/decode_step_kernel_tinyllama.md gives the command), scaled to K steps.
+            # DRAM bytes per decode step from one ncu capture of a short run of this workload, scaled to K steps
             t = json.load(open(tpath))
             traffic = float(t["dram_bytes_per_step"]) * K
-            traffic_src = t.get("source", "ncu capture, see profiles/decode_step_kernel_tinyllama.md") + \
+            traffic_src = t.get("source", "ncu capture (profiles/decode_step_traffic.json)") + \
                 "; not measured in this run, scaled by the steps per launch"
     else:
         # ---- dominant kernel: replay only the GEMV launches of a step ----

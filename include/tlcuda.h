@@ -96,7 +96,7 @@ TLC_API int32_t tlc_destroy(tlc_ctx *ctx);
  *   "pdl_mode"    when a GEMV lets the next kernel of the stream be scheduled: 1 = at once,
  *                 2 = after its last slab, 3 = after its own dependency wait, 4 (default) = 3 for
  *                 kernels that stream 40 MB of weights or more and 2 for shorter ones;
- *   "host_graph"  tlc_llama_decode_host runs as one graph launch with copy nodes (1, default)
+ *   "host_graph"  tlc_llama_decode_host runs as one graph launch without copies (1, default)
  *                 or as copy + graph + copy (0);
  *   "host_poll"   with host_graph: the host watches the pinned result words (1, default)
  *                 instead of synchronizing the stream (0).

@@ -18,8 +18,8 @@
 // every CTA streams its activation tile from L2, and at 128 x 128 that traffic
 // (16 KB per 64-wide K step and SM) saturates the L2 long before the tensor
 // cores; 256 x 256 halves it per MMA.  Per 64-wide K step:
-//   warps 0-3   A loaders: cp.async of the activation rows into the 128-byte
-//               swizzled K-major tile, several steps ahead;
+//   warp 0      activation rows by TMA into the 128-byte swizzled K-major tile, several
+//               steps ahead (without a tensor map: warps 0-3 by cp.async);
 //   warps 4-11  B producers (4*NT of them work): thread r dequantizes row r of
 //               the weight tile (2 blocks = 64 values) into the same layout; the
 //               row's quants (64 contiguous bytes per tile of the tiled weight

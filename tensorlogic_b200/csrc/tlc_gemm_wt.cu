@@ -3,7 +3,7 @@
 //   y[m, n] = sum_k W[n, k] . x[m, k]        W in Q4_0 / Q8_0 blocks or f16; or x . B with B [K, N]
 //
 // for the activation counts where tlc_gemm_kernel.cuh, which puts 128 activation rows on the M
-// side, either pads most of its tile (17 .. 100 rows) or has too few tiles for 148 SMs.
+// side, either pads most of its tile (up to 100 rows) or has too few tiles for 148 SMs.
 // A tile is 128 weight rows x bn activation rows (bn any multiple of 16 up to 256).  Two ways to fill 148 SMs:
 //   cluster  each tile's K steps are shared out over the ks CTAs of a thread-block cluster, which add their
 //            sums through distributed shared memory: small weights, where a call is a few microseconds;
@@ -24,8 +24,9 @@
 //
 // Warps:  0  x producer: TMA boxes of 64 columns x bn rows (128-byte swizzle), after the
 //            dependency wait (x comes from the previous kernel)
-//         1  weight producer, started before that wait (weights are never written by a kernel): one
-//            TMA box of eight slabs x one tile.  The box takes 16 bytes of the next tile along, so
+//         1  producer of quantized weights, started before that wait (weights are never written by a kernel): one
+//            TMA box of eight slabs x one tile.  (Dense operands come with the activations, by warp 0 behind the
+//            wait: matmul's may be what the previous kernel computed.)  The box takes 16 bytes of the next tile along, so
 //            that slabs lie off a multiple of 128 bytes apart and the eight lanes of a 16-byte shared
 //            load, which own rows of four slabs, meet different banks.
 //         2  tensor memory and MMA issue

@@ -926,7 +926,7 @@ extern "C" int32_t tlc_llama_decode_host(tlc_llama *L, int32_t batch, const int3
     }
     if (ids_host && !L->cfg.no_graph && L->ctx->host_graph) {
         // The common call: token ids up, one step, sampled ids and the status word down --
-        // all of it one graph (copy nodes around the step's kernels), one launch, one wait.
+        // all of it one graph, one launch, one wait.
         tlc_ctx *ctx = L->ctx;
         if (int32_t rc = reserve_positions(L, batch, 1)) return rc;  // before anything is launched
         const int key = 1000 + batch;
@@ -974,7 +974,7 @@ extern "C" int32_t tlc_llama_decode_host(tlc_llama *L, int32_t batch, const int3
             c[bytes - 1] = 0;
             if (int32_t rc = copy_logits(L, logits_host, batch)) return rc;
         } else if (ctx->host_poll) {
-            // Watch the pinned words the last copy node writes; after 50 ms without them
+            // Watch the pinned words the sampling kernel writes; after 50 ms without them
             // (an error, a very long step) fall back to the stream synchronize below.
             const auto t0 = std::chrono::steady_clock::now();
             for (long spin = 0; !seen; spin++) {
