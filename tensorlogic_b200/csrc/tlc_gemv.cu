@@ -28,8 +28,8 @@
 // weights, and crowd out the ring.  Each warp keeps its share of K of all rows in registers for the whole
 // launch instead, a K longer than a CTA's registers hold is shared out over a thread-block cluster,
 // and the RMSNorm is done once by a kernel of its own (frag_rows_kernel) and not by every CTA.  Measured on one
-// B200, before -> now: Q4_0 4096 x 4096, 8 rows 10.1 -> 7.1 us; norm + 7168 x 8192 at 8 / 16 rows 31.2 -> 18.0 /
-// 43.8 -> 24 us; norm + 2560 x 2048 at 5 / 16 rows 9.5 -> 6.4 / 19.3 -> 8.1 us; 28672 x 8192 at 8 rows 42.8 -> 35.9 us.
+// B200, before -> now: Q4_0 4096 x 4096, 8 rows 10.1 -> 7.4 us; norm + 7168 x 8192 at 8 / 16 rows 31.2 -> 16.8 /
+// 43.8 -> 21.9 us; norm + 2560 x 2048 at 5 / 16 rows 9.5 -> 6.9 / 19.3 -> 8.2 us; 28672 x 8192 at 8 rows 42.8 -> 33.2 us.
 #include <cuda_fp16.h>
 
 #include <cstring>
